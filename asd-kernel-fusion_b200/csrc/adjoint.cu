@@ -164,80 +164,6 @@ __global__ void __launch_bounds__(TPB) vjp_gather_kernel(
     if (S) block_add(part, bacc);  // uniform over the grid
 }
 
-// Column sums over sites for each k: Fpart[chunk][k] = sum_i ph_i A[i][k].
-__global__ void __launch_bounds__(128) fsum_kernel(const double *__restrict__ A, long M, int K,
-                                                   const double2 *__restrict__ ph, long rows,
-                                                   double2 *__restrict__ Fpart) {
-    const int k = blockIdx.x * 128 + threadIdx.x;
-    if (k >= K) return;
-    const long i0 = (long)blockIdx.y * rows, i1 = min(M, i0 + rows);
-    double re = 0.0, im = 0.0;
-    for (long i = i0; i < i1; ++i) {
-        const double x = A[i * K + k];
-        const double2 p = ph[i];
-        re += p.x * x;
-        im += p.y * x;
-    }
-    Fpart[(long)blockIdx.y * K + k] = make_double2(re, im);
-}
-
-// G_k = sum over chunks; Z_c = (1/nfile) sum_f G_(f,c).  One block.
-__global__ void gz_kernel(const double2 *__restrict__ Fpart, int nchunks, int K, int nfile,
-                          double2 *__restrict__ G, double2 *__restrict__ Z) {
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        double re = 0.0, im = 0.0;
-        for (int c = 0; c < nchunks; ++c) {
-            re += Fpart[(long)c * K + k].x;
-            im += Fpart[(long)c * K + k].y;
-        }
-        G[k] = make_double2(re, im);
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double re = 0.0, im = 0.0;
-        for (int f = 0; f < nfile; ++f) {
-            re += G[3 * f + threadIdx.x].x;
-            im += G[3 * f + threadIdx.x].y;
-        }
-        Z[threadIdx.x] = make_double2(re / nfile, im / nfile);
-    }
-}
-
-// S = (1/(M nfile)) sum_k F_k (G_k - Z_c(k)), F from the chunk partials.  One
-// block of 256 threads, fixed order.
-__global__ void __launch_bounds__(256) sqt_value_kernel(const double2 *__restrict__ Fpart,
-                                                        int nchunks, int K, int nfile, long M,
-                                                        const double2 *__restrict__ G,
-                                                        const double2 *__restrict__ Z,
-                                                        double2 *__restrict__ out) {
-    __shared__ double sre[256], sim[256];
-    double re = 0.0, im = 0.0;
-    for (int k = threadIdx.x; k < K; k += 256) {
-        double fr = 0.0, fi = 0.0;
-        for (int c = 0; c < nchunks; ++c) {
-            fr += Fpart[(long)c * K + k].x;
-            fi += Fpart[(long)c * K + k].y;
-        }
-        const double gr = G[k].x - Z[k % 3].x, gi = G[k].y - Z[k % 3].y;
-        re += fr * gr - fi * gi;
-        im += fr * gi + fi * gr;
-    }
-    sre[threadIdx.x] = re;
-    sim[threadIdx.x] = im;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            sre[threadIdx.x] += sre[threadIdx.x + w];
-            sim[threadIdx.x] += sim[threadIdx.x + w];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const double s = 1.0 / ((double)M * nfile);
-        *out = make_double2(sre[0] * s, sim[0] * s);
-    }
-}
-
 // lam[i][k] += Re(coef u_i (G_k - Z_c(k))), coef = dL/dS* in the sense
 // dL = Re(coef' dS) with coef' folded with 1/(M nfile) by the caller.
 __global__ void __launch_bounds__(256) loss_grad_kernel(double *__restrict__ lam, long M, int K,
@@ -308,40 +234,6 @@ cudaError_t launch_vjp_gather(const LLGArgs &a, const double *P_in, double *loc,
                               cudaStream_t st) {
     vjp_gather_kernel<<<adjoint_blocks(a), TPB, 0, st>>>(a, P_in, loc, lam_v, lam_y_in, lam_y_out,
                                                          cv, cs, S, P_out, bacc);
-    return cudaGetLastError();
-}
-
-// Rows per chunk of the site sums: 256, halved (down to 16) until the grid
-// of (K / 128) x chunks has at least four blocks per SM of a B200, so that
-// small lattices (64 x 64 x 100: 48 blocks of 256 rows) still fill the GPU;
-// doubled where the chunks would exceed the grid's y extent (N = 4096).
-int fsum_rows(long M, int K) {
-    constexpr long kMinBlocks = 4 * 148;
-    const long kb = (K + 127) / 128;
-    int rows = 256;
-    while (rows > 16 && kb * ((M + rows - 1) / rows) < kMinBlocks) rows >>= 1;
-    while ((M + rows - 1) / rows > 65535) rows <<= 1;  // the grid's y extent
-    return rows;
-}
-
-int fsum_chunks(long M, int K) { return (int)((M + fsum_rows(M, K) - 1) / fsum_rows(M, K)); }
-
-cudaError_t launch_fsum(const double *A, long M, int K, const double2 *ph, double2 *Fpart,
-                        cudaStream_t st) {
-    dim3 grid((unsigned)((K + 127) / 128), (unsigned)fsum_chunks(M, K));
-    fsum_kernel<<<grid, 128, 0, st>>>(A, M, K, ph, fsum_rows(M, K), Fpart);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gz(const double2 *Fpart, long M, int K, int nfile, double2 *G, double2 *Z,
-                      cudaStream_t st) {
-    gz_kernel<<<1, 256, 0, st>>>(Fpart, fsum_chunks(M, K), K, nfile, G, Z);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_sqt_value(const double2 *Fpart, long M, int K, int nfile, const double2 *G,
-                             const double2 *Z, double2 *out, cudaStream_t st) {
-    sqt_value_kernel<<<1, 256, 0, st>>>(Fpart, fsum_chunks(M, K), K, nfile, M, G, Z, out);
     return cudaGetLastError();
 }
 

@@ -118,22 +118,39 @@ inline int split_esize(int kind) { return kind == 1 ? 4 : 2; }
 // 2^-15 * spin_len are normal numbers.  1 for the other kinds.
 double split_scale(int kind, double spin_len);
 
-// ------------------------------------------ FP64 tensor-core GEMM S(q,t)
-// (dmma_sqt.cu) C = alpha A B^T over site-major [M][K] FP64 operands, never
-// stored: per 128 x 128 tile either the S(q,t) partial (part != nullptr and
-// tdiag == nullptr) or the q-grid diagonal partials (tdiag != nullptr).
+// -------------------------------------- FP64 S(q,t) at one q (phase_sum.cu)
+// Work space of the phase sums: phase_work_bytes(M, K) bytes, carved up by
+// phase_work.  Its last 16 bytes hold the count of finished blocks: zero before
+// the first launch, left zero by every launch.
+struct PhaseWork {
+    double2 *Fpart;   // [chunks][K] column sums per chunk of sites
+    double2 *part;    // one partial per 32 columns
+    unsigned *count;
+};
+size_t phase_work_bytes(long M, int K);
+PhaseWork phase_work(void *p, long M, int K);
+// G[k] = sum_j w_j B[j][k] (k < K) and Z[c] = (1/nfile) sum_f G[3 f + c].
+cudaError_t launch_phase_origin(const double *B, long M, int K, int nfile, const double2 *wphase,
+                                const PhaseWork &w, double2 *G, double2 *Z, cudaStream_t st);
+// out[0..1] = scale * sum_k (sum_i u_i A[i][k]) (G[k] - Z[k % 3]); Z == nullptr:
+// without the connected part's Z.
+cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *uphase,
+                             const PhaseWork &w, const double2 *G, const double2 *Z, double scale,
+                             double *out, cudaStream_t st);
+
+// ------------------------------------------------- FP64 tensor-core GEMM
+// (dmma_sqt.cu) C = alpha A B^T over site-major [M][K] FP64 operands.  Per
+// 128 x 128 tile either sum |C_ij - m_i . z_j| (part != nullptr), the q-grid
+// diagonal partials (tdiag != nullptr), neither storing C, or C itself.
 struct DmmaSqtArgs {
     const double *A, *B;  // [M][K], the state at t and the origin
     long M;
     int K;
     double alpha;
-    int outer;            // subtract m_i . z_j (0: a shard's partial GEMM value)
-    const double *mrow, *zcol;       // [M][3] replica means at t and 0
-    const double2 *uphase, *wphase;  // [M]
-    double2 *part;        // one partial per tile, dmma_sqt_tiles(M) of them
+    const double *mrow, *zcol;  // [M][3] replica means at t and 0
+    double2 *part;        // one partial (in .x) per tile, dmma_sqt_tiles(M) of them
     int lat_n = 0;        // q grid: lattice side
-    double *tdiag = nullptr;  // q grid: [tiles][dmma_sqt_tile() * 2 - 1][2]
-    int abs_sum = 0;      // sum |alpha C_ij - m_i . z_j| instead (no phase)
+    double *tdiag = nullptr;  // q grid: [tiles][2 * kDmmaTile - 1][2]
     // Plain product (the cblas_dgemm drop-in): with C set, B has MB rows and
     // the kernel stores C[i + j ldc] = alpha sum_k A_ik B_jk (+ beta C[..] when
     // beta != 0; C is not read when beta == 0) for i < M, j < MB.
@@ -180,14 +197,6 @@ cudaError_t launch_vjp_gather(const LLGArgs &a, const double *P_in, double *loc,
                               const double *lam_v, const double *lam_y_in, double *lam_y_out,
                               double cv, double cs, const double *S, double *P_out, double *bacc,
                               cudaStream_t st);
-int fsum_rows(long M, int K);
-int fsum_chunks(long M, int K);
-cudaError_t launch_fsum(const double *A, long M, int K, const double2 *ph, double2 *Fpart,
-                        cudaStream_t st);
-cudaError_t launch_gz(const double2 *Fpart, long M, int K, int nfile, double2 *G, double2 *Z,
-                      cudaStream_t st);
-cudaError_t launch_sqt_value(const double2 *Fpart, long M, int K, int nfile, const double2 *G,
-                             const double2 *Z, double2 *out, cudaStream_t st);
 cudaError_t launch_loss_grad(double *lam, long M, int K, const double2 *u, const double2 *G,
                              const double2 *Z, double cre, double cim, cudaStream_t st);
 cudaError_t launch_param_reduce(const double *bacc, int nblocks, double *grad, cudaStream_t st);

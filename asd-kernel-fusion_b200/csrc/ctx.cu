@@ -74,6 +74,11 @@ struct asd_ctx {
     double a_scale[4] = {}, b_scale[4] = {};
     double2 *part = nullptr;
     long part_cap = 0;
+    // FP64 phase sums (allocated on the first FP64 S(q,t) or loss): work space,
+    // the origin's column sums G [K] and Z [3], and the origin version they
+    // were formed from
+    double2 *phase_ws = nullptr, *phase_G = nullptr;
+    long g_version = -1;
     double *d_out = nullptr;
     double *h_out = nullptr;  // pinned
     unsigned *status = nullptr;
@@ -328,6 +333,7 @@ int refresh_origin(asd_ctx *c) {
     c->last_launches += 1;
     c->origin_version = c->state_version;
     for (int k = 1; k <= 3; ++k) c->b_version[k] = -1;
+    c->g_version = -1;
     return ASD_OK;
 }
 
@@ -392,35 +398,59 @@ double gemm_alpha(const asd_ctx *c, bool shard) {
     return 1.0 / (double)((shard && c->nfile_total > 0) ? c->nfile_total : c->p.nfile);
 }
 
-// The plain FP64 path: the FP64 tensor-core GEMM with the fused epilogue,
-// one partial per tile, then the fixed-order final sum.
-DmmaSqtArgs dmma_args(const asd_ctx *c, bool shard) {
+// The FP64 GEMM over the state and the origin (the terms' magnitude, the q
+// grid); the replica means must be up to date.
+DmmaSqtArgs dmma_args(const asd_ctx *c) {
     DmmaSqtArgs g{};
     g.A = c->y;
     g.B = c->origin;
     g.M = c->M;
     g.K = c->K;
-    g.alpha = gemm_alpha(c, shard);
-    g.outer = shard ? 0 : 1;
+    g.alpha = 1.0 / (double)c->p.nfile;
     g.mrow = c->mean_t;
     g.zcol = c->mean_0;
-    g.uphase = c->uphase;
-    g.wphase = c->wphase;
     return g;
 }
 
+PhaseWork phase_ws(const asd_ctx *c) { return phase_work(c->phase_ws, c->M, c->K); }
+
+// The work space of the phase sums, and the origin's column sums up to date
+// (formed once per origin and q).
+int ensure_phase_origin(asd_ctx *c) {
+    int rc;
+    if (!c->phase_ws) {
+        const size_t n = phase_work_bytes(c->M, c->K);
+        if ((rc = dalloc(&c->phase_ws, n)) != ASD_OK) return rc;
+        const cudaError_t e = cudaMemsetAsync(phase_ws(c).count, 0, sizeof(double2), c->stream);
+        if (e != cudaSuccess) {  // unusable without its zero count
+            cudaFree(c->phase_ws);
+            c->phase_ws = nullptr;
+            return cuda_fail(e, "cudaMemsetAsync");
+        }
+    }
+    if (!c->phase_G && (rc = dalloc(&c->phase_G, ((size_t)c->K + 3) * sizeof(double2))) != ASD_OK)
+        return rc;
+    if (c->g_version == c->origin_version) return ASD_OK;
+    ASD_CUDA_TRY(launch_phase_origin(c->origin, c->M, c->K, c->p.nfile, c->wphase, phase_ws(c),
+                                     c->phase_G, c->phase_G + c->K, c->stream));
+    c->g_version = c->origin_version;
+    c->last_launches += 2;
+    return ASD_OK;
+}
+
+// The FP64 mode: column sums of the state, their products with the origin's.
+// A shard leaves out the connected part, which only the ensemble's means give.
 int sqt_plain(asd_ctx *c, double *d_out, bool shard) {
-    const long tiles = dmma_sqt_tiles(c->M);
-    if (tiles > 0x7fffffffL) return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 GEMM");
-    int rc = ensure_part(c, tiles);
+    // N > 2435 stays refused, as the header says
+    if (dmma_sqt_tiles(c->M) > 0x7fffffffL)
+        return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 mode");
+    int rc = ensure_phase_origin(c);
     if (rc != ASD_OK) return rc;
-    DmmaSqtArgs g = dmma_args(c, shard);
-    g.part = c->part;
     cudaEvent_t t0 = time_begin(c, c->stream);
-    rc = launch_dmma_sqt(g, c->stream);
+    ASD_CUDA_TRY(launch_phase_sum(c->y, c->M, c->K, c->uphase, phase_ws(c), c->phase_G,
+                                  shard ? nullptr : c->phase_G + c->K,
+                                  gemm_alpha(c, shard) / (double)c->M, d_out, c->stream));
     time_end(c, 1, 1, c->stream, t0);
-    if (rc != ASD_OK) return rc;
-    ASD_CUDA_TRY(launch_finalize(c->part, (int)tiles, 1.0 / (double)c->M, d_out, c->stream));
     c->last_launches += 2;
     return ASD_OK;
 }
@@ -508,12 +538,12 @@ int sqt_async(asd_ctx *c, int mode, double *d_out, bool shard = false) {
         return fail(ASD_ERR_STATE, "set the spins and the origin before S(q,t)");
     if (mode < 0 || mode > 3) return fail(ASD_ERR_INVALID, "unknown S(q,t) mode %d", mode);
     if (!(c->modes & (1u << mode))) return fail(ASD_ERR_STATE, "mode %d not enabled at create", mode);
+    if (mode == ASD_SQT_FP64) return sqt_plain(c, d_out, shard);
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
                                   c->stream));
     c->rows_ready = true;
     c->last_launches += 1;
     switch (mode) {
-        case ASD_SQT_FP64: return sqt_plain(c, d_out, shard);
         case ASD_SQT_TF32X3: return sqt_split(c, 1, d_out, shard);
         case ASD_SQT_BF16X3: return sqt_split(c, 2, d_out, shard);
         case ASD_SQT_FP16X3: return sqt_split(c, 3, d_out, shard);
@@ -570,8 +600,7 @@ int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
         for (long i = 0; i < need; ++i)
             if ((rc = dalloc(&c->adj_bufs[i], sb)) != ASD_OK) return rc;
         const int nb = adjoint_blocks(c->a);
-        const size_t small = (size_t)nb * 6 * sizeof(double) +
-                             ((size_t)fsum_chunks(M, K) * K + 2 * K + 8 + 2) * sizeof(double2);
+        const size_t small = (size_t)(nb + 1) * 6 * sizeof(double);
         if ((rc = dalloc(&c->adj_bufs[need], small)) != ASD_OK) return rc;
         if ((rc = dalloc(&c->adj_bufs[need + 1], (size_t)(E + 8) * sizeof(double2))) != ASD_OK)
             return rc;
@@ -594,7 +623,7 @@ struct AdjBufs {
     double **ck, **seg;
     double **stg;  // with a kept segment: stg[4 (j - 1) + q] = s2, s3, s4, acc of step j
     double *bacc, *dgrad;
-    double2 *Fpart, *G, *Z, *Sv;
+    double2 *Sv;
     int nb;
 };
 
@@ -608,10 +637,7 @@ AdjBufs adj_bufs(asd_ctx *c, int nck, int ckpt) {
     b.stg = b.seg + ckpt + 1;
     b.nb = adjoint_blocks(c->a);
     b.bacc = B[c->adj_states];
-    b.Fpart = reinterpret_cast<double2 *>(b.bacc + (size_t)b.nb * 6);
-    b.G = b.Fpart + (size_t)fsum_chunks(c->M, c->K) * c->K;
-    b.Z = b.G + c->K;
-    b.dgrad = reinterpret_cast<double *>(b.Z + 4);
+    b.dgrad = b.bacc + (size_t)b.nb * 6;
     b.Sv = reinterpret_cast<double2 *>(B[c->adj_states + 1]);
     return b;
 }
@@ -635,10 +661,8 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
     cudaStream_t st = c->stream;
     c->last_launches = 0;
     c->tape_valid = false;
-    // G_k and Z_c of the origin
-    ASD_CUDA_TRY(launch_fsum(c->origin, M, K, c->wphase, b.Fpart, st));
-    ASD_CUDA_TRY(launch_gz(b.Fpart, M, K, c->p.nfile, b.G, b.Z, st));
-    c->last_launches += 2;
+    if ((rc = ensure_phase_origin(c)) != ASD_OK) return rc;
+    const double sqt_scale = 1.0 / ((double)M * c->p.nfile);
     // forward: checkpoints and S(q,t) at every stride-th step
     ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[0], c->origin, sb, cudaMemcpyDeviceToDevice, st));
     double *cur = b.seg[0], *nxt = b.seg[1];
@@ -660,8 +684,9 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
         if (n % ckpt == 0 && n / ckpt < nck)
             ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[n / ckpt], cur, sb, cudaMemcpyDeviceToDevice, st));
         if (n % stride == 0 && n / stride <= E) {
-            ASD_CUDA_TRY(launch_fsum(cur, M, K, c->uphase, b.Fpart, st));
-            ASD_CUDA_TRY(launch_sqt_value(b.Fpart, M, K, c->p.nfile, b.G, b.Z, b.Sv + (n / stride - 1), st));
+            ASD_CUDA_TRY(launch_phase_sum(cur, M, K, c->uphase, phase_ws(c), c->phase_G,
+                                          c->phase_G + K, sqt_scale,
+                                          reinterpret_cast<double *>(b.Sv + (n / stride - 1)), st));
             c->last_launches += 2;
         }
     }
@@ -740,7 +765,8 @@ int loss_backward(asd_ctx *c, const double *target, double *grad, double *dtarge
             const int j = n - base;
             if (n % stride == 0 && n / stride <= E) {
                 const double2 cf = coef[n / stride - 1];
-                ASD_CUDA_TRY(launch_loss_grad(b.lam, M, K, c->uphase, b.G, b.Z, cf.x, cf.y, st));
+                ASD_CUDA_TRY(launch_loss_grad(b.lam, M, K, c->uphase, c->phase_G,
+                                              c->phase_G + K, cf.x, cf.y, st));
                 c->last_launches += 1;
             }
             // y_{n-1} = seg[j-1]: its stage states (kept from the segment's
@@ -830,7 +856,7 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
         rc = ensure_grid_work(c, (size_t)(nm * nm) * nd2,
                               (size_t)qgrid_keys((int)nm, (int)nm, kDmmaTile, kDmmaTile) * nd2);
         if (rc != ASD_OK) return rc;
-        DmmaSqtArgs g = dmma_args(c, false);
+        DmmaSqtArgs g = dmma_args(c);
         g.lat_n = N;
         g.tdiag = c->grid_tdiag;
         if ((rc = launch_dmma_sqt(g, c->stream)) != ASD_OK) return rc;
@@ -1125,7 +1151,8 @@ void destroy(asd_ctx *c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     void *ptrs[] = {c->y, c->ys_a, c->ys_b, c->acc, c->origin, c->mean_t, c->mean_0, c->uphase,
-                    c->wphase, c->row4, c->col4, c->row1, c->col1, c->grid_tdiag, c->grid_ds, c->part, c->d_out,
+                    c->wphase, c->row4, c->col4, c->row1, c->col1, c->grid_tdiag, c->grid_ds, c->part,
+                    c->phase_ws, c->phase_G, c->d_out,
                     c->status, c->grid_g, c->grid_t, c->grid_out};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -1471,10 +1498,12 @@ int asd_ctx_sqt_magnitude(asd_ctx *c, double *out) {
     if (tiles > 0x7fffffffL) return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 GEMM");
     int rc = ensure_part(c, tiles);
     if (rc != ASD_OK) return rc;
-    DmmaSqtArgs g = dmma_args(c, false);
+    DmmaSqtArgs g = dmma_args(c);
     g.part = c->part;
-    g.abs_sum = 1;
-    if ((rc = launch_dmma_sqt(g, c->stream)) != ASD_OK) return rc;
+    cudaEvent_t t0 = time_begin(c, c->stream);
+    rc = launch_dmma_sqt(g, c->stream);
+    time_end(c, 1, 1, c->stream, t0);
+    if (rc != ASD_OK) return rc;
     ASD_CUDA_TRY(launch_finalize(c->part, (int)tiles, 1.0 / (double)c->M, c->d_out, c->stream));
     c->last_launches = 3;
     ASD_CUDA_TRY(cudaMemcpyAsync(c->h_out, c->d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1726,6 +1755,7 @@ int asd_ctx_debug_poison(asd_ctx *c) {
         {c->grid_tdiag, c->grid_tdiag_n * sizeof(double)},
         {c->grid_ds, c->grid_ds_n * sizeof(double)},
         {c->part, (size_t)c->part_cap * sizeof(double2)},
+        {c->phase_ws, phase_work_bytes(c->M, c->K) - sizeof(double2)},  // not the count
         {c->d_out, 2 * sizeof(double)},
         {c->grid_g, (size_t)c->M * sizeof(double)},
         {c->grid_t, (size_t)c->M * sizeof(double2)},

@@ -1,15 +1,12 @@
-// dmma_sqt.cu -- the plain FP64 S(q,t) path: one FP64 tensor-core GEMM
-// (mma.sync m16n8k8 .f64, dmma.cuh) whose epilogue applies the connected-part
-// subtraction, the phase and the reduction, so that no C matrix exists.
+// dmma_sqt.cu -- the FP64 tensor-core GEMM (mma.sync m16n8k8 .f64, dmma.cuh)
+// over the whole N^2 x N^2 correlation, for what needs its elements: the
+// magnitude of the terms S(q,t) sums, the q grid, and the cblas_dgemm drop-in.
 //
-// The reference's plain path is cblas_dgemm of the whole (N^2 x N^2)
-// correlation matrix followed by three sweeps over it: the outer-product
-// subtraction, the phase product and the sum (gemm/llg_sqt_mkl.c:378-423).
-// Here C_ij = alpha * sum_k A_ik B_jk stays in registers: the phase factorises
-// as u_i w_j and the outer term is m_i . z_j, so the epilogue needs only
-// per-row and per-column vectors, and each CTA leaves one complex partial:
-//   part[tile] = sum_{i,j in tile} u_i w_j (alpha C_ij - m_i . z_j)
-// (or, for the error scale of S(q,t), sum_{i,j in tile} |alpha C_ij - m_i . z_j|).
+// The reference's plain path is cblas_dgemm of the whole correlation matrix
+// followed by three sweeps over it (gemm/llg_sqt_mkl.c:378-423).  Here C_ij =
+// alpha * sum_k A_ik B_jk stays in registers and the outer term m_i . z_j comes
+// from per-row and per-column vectors; each CTA leaves one partial:
+//   part[tile] = sum_{i,j in tile} |alpha C_ij - m_i . z_j|
 // The q-grid epilogue instead leaves, per tile, the sums of
 // alpha C_ij - m_i . z_j along each diagonal i - j of the tile, split by
 // whether the lattice column of j wraps around (qgrid.cu bins them by
@@ -44,7 +41,7 @@ constexpr int STAGE_DOUBLES = (BM + BN) * BK;  // 8192 doubles = 64 KB
 constexpr int PIPE_BYTES = STAGES * STAGE_DOUBLES * 8;
 constexpr int TSTRIDE = BN + 1;  // q grid: epilogue tile row stride (doubles)
 constexpr int GRID_SMEM = BM * TSTRIDE * 8;
-constexpr int EPI_PHASE = 0, EPI_GRID = 1, EPI_STORE = 2;
+constexpr int EPI_ABS = 0, EPI_GRID = 1, EPI_STORE = 2;
 constexpr int KCH = BK / 2;  // 16-byte chunks per shared-memory row
 constexpr int LOG_KCH = 4;
 static_assert(KCH == (1 << LOG_KCH), "chunks per row");
@@ -114,11 +111,10 @@ __device__ __forceinline__ void load_tile(double *dst, const double *__restrict_
 template <int VEC, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
     dmma_sqt_kernel(const double *__restrict__ A, const double *__restrict__ B, long M, int K,
-                    int num_m, int num_n, double alpha, int outer,
-                    const double *__restrict__ mrow, const double *__restrict__ zcol,
-                    const double2 *__restrict__ uphase, const double2 *__restrict__ wphase,
-                    double2 *__restrict__ part, int lat_n, double *__restrict__ tdiag,
-                    int abs_sum, long MB, double *__restrict__ Cst, long ldc, double beta) {
+                    int num_m, int num_n, double alpha, const double *__restrict__ mrow,
+                    const double *__restrict__ zcol, double2 *__restrict__ part, int lat_n,
+                    double *__restrict__ tdiag, long MB, double *__restrict__ Cst, long ldc,
+                    double beta) {
     extern __shared__ __align__(16) double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -207,64 +203,35 @@ __global__ void __launch_bounds__(THREADS, 1)
                         *cp = (beta != 0.0) ? v + beta * *cp : v;
                     }
             }
-    } else if (EPI == EPI_PHASE) {
-        // sum over the thread's 8 rows x 8 columns of u_i w_j (alpha C_ij - m_i . z_j)
-        double tot_re = 0.0, tot_im = 0.0;
+    } else if (EPI == EPI_ABS) {
+        // sum over the thread's 8 rows x 8 columns of |alpha C_ij - m_i . z_j|
+        double tot = 0.0;
 #pragma unroll
         for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const long i = m0 + wm * 64 + mt * 16 + g + 8 * h;
                 if (i >= M) continue;
-                double mx = 0.0, my = 0.0, mz = 0.0;
-                if (outer) {
-                    mx = mrow[3 * i];
-                    my = mrow[3 * i + 1];
-                    mz = mrow[3 * i + 2];
-                }
-                double sre = 0.0, sim = 0.0;
+                const double mx = mrow[3 * i], my = mrow[3 * i + 1], mz = mrow[3 * i + 2];
 #pragma unroll
                 for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const long j = n0 + wn * 32 + nt * 8 + 2 * t + e;
                         if (j >= M) continue;
-                        double v = alpha * acc[mt][nt][2 * h + e];
-                        if (outer) v -= mx * zcol[3 * j] + my * zcol[3 * j + 1] + mz * zcol[3 * j + 2];
-                        if (abs_sum) {
-                            sre += fabs(v);
-                        } else {
-                            const double2 w = wphase[j];
-                            sre += w.x * v;
-                            sim += w.y * v;
-                        }
+                        tot += fabs(alpha * acc[mt][nt][2 * h + e] -
+                                    (mx * zcol[3 * j] + my * zcol[3 * j + 1] + mz * zcol[3 * j + 2]));
                     }
-                if (abs_sum) {
-                    tot_re += sre;
-                } else {
-                    const double2 u = uphase[i];
-                    tot_re += u.x * sre - u.y * sim;
-                    tot_im += u.x * sim + u.y * sre;
-                }
             }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            tot_re += __shfl_xor_sync(0xffffffffu, tot_re, o);
-            tot_im += __shfl_xor_sync(0xffffffffu, tot_im, o);
-        }
-        __shared__ double red[2][THREADS / 32];
-        if (lane == 0) {
-            red[0][warp] = tot_re;
-            red[1][warp] = tot_im;
-        }
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        __shared__ double red[THREADS / 32];
+        if (lane == 0) red[warp] = tot;
         __syncthreads();
         if (threadIdx.x == 0) {
-            double re = 0.0, im = 0.0;
-            for (int w = 0; w < THREADS / 32; ++w) {
-                re += red[0][w];
-                im += red[1][w];
-            }
-            part[blockIdx.x] = make_double2(re, im);
+            double sum = 0.0;
+            for (int w = 0; w < THREADS / 32; ++w) sum += red[w];
+            part[blockIdx.x] = make_double2(sum, 0.0);
         }
     } else {
         // The tile's connected values v_ij into shared memory (zero outside
@@ -280,7 +247,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int r = wm * 64 + mt * 16 + g + 8 * h;
                 const long i = m0 + r;
                 double mx = 0.0, my = 0.0, mz = 0.0;
-                if (outer && i < M) {
+                if (i < M) {
                     mx = mrow[3 * i];
                     my = mrow[3 * i + 1];
                     mz = mrow[3 * i + 2];
@@ -294,8 +261,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         double v = 0.0;
                         if (i < M && j < M) {
                             v = alpha * acc[mt][nt][2 * h + e];
-                            if (outer)
-                                v -= mx * zcol[3 * j] + my * zcol[3 * j + 1] + mz * zcol[3 * j + 2];
+                            v -= mx * zcol[3 * j] + my * zcol[3 * j + 1] + mz * zcol[3 * j + 2];
                         }
                         T[r * TSTRIDE + c] = v;
                     }
@@ -395,9 +361,8 @@ int launch_dmma_sqt(const DmmaSqtArgs &p, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         kern<<<(unsigned)(nm * nn), THREADS, smem, st>>>(p.A, p.B, p.M, p.K, num_m, num_n, p.alpha,
-                                                          p.outer, p.mrow, p.zcol, p.uphase,
-                                                          p.wphase, p.part, p.lat_n, p.tdiag,
-                                                          p.abs_sum, MB, p.C, p.ldc, p.beta);
+                                                          p.mrow, p.zcol, p.part, p.lat_n, p.tdiag,
+                                                          MB, p.C, p.ldc, p.beta);
         return cudaGetLastError();
     };
     cudaError_t e;
@@ -406,7 +371,7 @@ int launch_dmma_sqt(const DmmaSqtArgs &p, cudaStream_t st) {
     else if (grid)
         e = vec2 ? go(dmma_sqt_kernel<2, EPI_GRID>) : go(dmma_sqt_kernel<1, EPI_GRID>);
     else
-        e = vec2 ? go(dmma_sqt_kernel<2, EPI_PHASE>) : go(dmma_sqt_kernel<1, EPI_PHASE>);
+        e = vec2 ? go(dmma_sqt_kernel<2, EPI_ABS>) : go(dmma_sqt_kernel<1, EPI_ABS>);
     if (e != cudaSuccess) return cuda_fail(e, "dmma_sqt launch");
     return ASD_OK;
 }

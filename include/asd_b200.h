@@ -57,9 +57,9 @@ extern "C" {
 
 /* Arithmetic of the S(q,t) correlation GEMM. */
 typedef enum {
-    ASD_SQT_FP64 = 0,   /* the plain path: FP64 tensor-core GEMM (mma.sync .f64) with
-                           the phase, connected-part and reduction epilogue fused;
-                           one block per 128 x 128 tile, so up to N = 2435
+    ASD_SQT_FP64 = 0,   /* FP64 throughout: the product summed over the sites first
+                           (F_k = sum_i u_i A_ik, G_k = sum_j w_j B_jk), so one read
+                           of the state instead of a GEMM; up to N = 2435
                            (ASD_ERR_UNSUPPORTED beyond) */
     ASD_SQT_TF32X3 = 1, /* tcgen05 kind::tf32, hi*hi + hi*lo + lo*hi, FP32 accumulate   */
     ASD_SQT_BF16X3 = 2, /* tcgen05 kind::f16 (bf16), hi*hi + hi*lo + lo*hi, FP32 accum. */
@@ -280,8 +280,9 @@ int asd_ctx_last_launches(const asd_ctx *ctx);
 
 /* Diagnostic: with on != 0, later calls record CUDA events on the stream each
  * kernel is launched on, around every RK4 step (the one-launch step kernel, or
- * the four stage kernels of one step) and every S(q,t) GEMM kernel (the
- * tcgen05 split GEMM or the FP64 GEMM); nothing is recorded while a stream is
+ * the four stage kernels of one step) and every S(q,t) evaluation's main pass
+ * (the tcgen05 split GEMM, the FP64 GEMM, or the FP64 mode's phase sums,
+ * counted as one); nothing is recorded while a stream is
  * being captured.  No counterpart in the reference; the benchmark uses it. */
 int asd_ctx_time_kernels(asd_ctx *ctx, int on);
 /* Waits for the events recorded since the last read and returns the summed
