@@ -138,10 +138,20 @@ cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *upha
                              const PhaseWork &w, const double2 *G, const double2 *Z, double scale,
                              double *out, cudaStream_t st);
 
+// ------------------------------------- FP64 S(q,t) on the q grid (qfft.cu)
+// out[2 (a N + b)] = scale * sum_k A~_k conj(B~_k) at q = 2 pi (a, b) / N, the
+// transforms of A - m and B - z (m, z [M][3]); work: qfft_work_bytes, its first
+// N complex values written once by launch_qfft_twiddles; scratch: three buffers
+// of M K doubles.  Returns the number of launches or a negative error.
+size_t qfft_work_bytes(int lat_n, int K);
+cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st);
+int launch_qfft(const double *A, const double *B, int lat_n, int K, const double *m,
+                const double *z, double scale, void *work, double *const scratch[3], double *out,
+                cudaStream_t st);
+
 // ------------------------------------------------- FP64 tensor-core GEMM
 // (dmma_sqt.cu) C = alpha A B^T over site-major [M][K] FP64 operands.  Per
-// 128 x 128 tile either sum |C_ij - m_i . z_j| (part != nullptr), the q-grid
-// diagonal partials (tdiag != nullptr), neither storing C, or C itself.
+// 128 x 128 tile either sum |C_ij - m_i . z_j| (part != nullptr) or C itself.
 struct DmmaSqtArgs {
     const double *A, *B;  // [M][K], the state at t and the origin
     long M;
@@ -149,8 +159,6 @@ struct DmmaSqtArgs {
     double alpha;
     const double *mrow, *zcol;  // [M][3] replica means at t and 0
     double2 *part;        // one partial (in .x) per tile, dmma_sqt_tiles(M) of them
-    int lat_n = 0;        // q grid: lattice side
-    double *tdiag = nullptr;  // q grid: [tiles][2 * kDmmaTile - 1][2]
     // Plain product (the cblas_dgemm drop-in): with C set, B has MB rows and
     // the kernel stores C[i + j ldc] = alpha sum_k A_ik B_jk (+ beta C[..] when
     // beta != 0; C is not read when beta == 0) for i < M, j < MB.
@@ -159,7 +167,6 @@ struct DmmaSqtArgs {
     long ldc = 0;
     double beta = 0.0;
 };
-constexpr int kDmmaTile = 128;  // tile rows = tile columns
 long dmma_sqt_tiles(long M);
 int launch_dmma_sqt(const DmmaSqtArgs &p, cudaStream_t st);
 // Device transpose of a dense [rows][cols] FP64 matrix into [cols][rows].

@@ -86,7 +86,8 @@ struct asd_ctx {
     bool has_state = false, has_origin = false;
     int last_launches = 0;
     int chunk_k = -1;  // < 0: per mode, 512 for TF32x3, 1024 for BF16x3 and FP16x3
-    double *grid_g = nullptr;     // q grid: N*N displacement bins (FP64)
+    double2 *grid_fft = nullptr;  // q grid, FP64: twiddles, sums over k
+    double *grid_g = nullptr;     // q grid, split modes: N*N displacement bins (FP64)
     double2 *grid_t = nullptr;    // q grid: DFT intermediate
     double *grid_out = nullptr;   // q grid: device result for the host-buffer form
     double *grid_tdiag = nullptr; // q grid: per-tile diagonal partials
@@ -398,8 +399,8 @@ double gemm_alpha(const asd_ctx *c, bool shard) {
     return 1.0 / (double)((shard && c->nfile_total > 0) ? c->nfile_total : c->p.nfile);
 }
 
-// The FP64 GEMM over the state and the origin (the terms' magnitude, the q
-// grid); the replica means must be up to date.
+// The FP64 GEMM over the state and the origin (the terms' magnitude); the
+// replica means must be up to date.
 DmmaSqtArgs dmma_args(const asd_ctx *c) {
     DmmaSqtArgs g{};
     g.A = c->y;
@@ -841,6 +842,31 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
         return fail(ASD_ERR_UNSUPPORTED, "q-grid S(q,t): mode %d not supported", mode);
     if (!(c->modes & (1u << mode))) return fail(ASD_ERR_STATE, "mode %d not enabled at create", mode);
     int rc;
+    if (mode == ASD_SQT_FP64) {
+        // N > 2435 stays refused, as the header says
+        if (dmma_sqt_tiles(M) > 0x7fffffffL)
+            return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 mode");
+        if (!c->grid_fft) {
+            if ((rc = dalloc(&c->grid_fft, qfft_work_bytes(N, c->K))) != ASD_OK) return rc;
+            const cudaError_t e = launch_qfft_twiddles(N, c->grid_fft, c->stream);
+            if (e != cudaSuccess) {  // unusable without its twiddles
+                cudaFree(c->grid_fft);
+                c->grid_fft = nullptr;
+                return cuda_fail(e, "launch_qfft_twiddles");
+            }
+            c->last_launches += 1;
+        }
+        ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4,
+                                      c->row1, c->stream));
+        c->rows_ready = true;
+        c->last_launches += 1;
+        double *const scratch[3] = {c->ys_a, c->ys_b, c->acc};  // RK4 state only within a step
+        rc = launch_qfft(c->y, c->origin, N, c->K, c->mean_t, c->mean_0,
+                         1.0 / ((double)M * c->p.nfile), c->grid_fft, scratch, d_out, c->stream);
+        if (rc < 0) return rc;
+        c->last_launches += rc;
+        return ASD_OK;
+    }
     // each checked on its own: after a failed allocation of grid_t, grid_g
     // is already there and the next call must still allocate grid_t
     if (!c->grid_g && (rc = dalloc(&c->grid_g, (size_t)M * sizeof(double))) != ASD_OK) return rc;
@@ -849,23 +875,6 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
                                   c->stream));
     c->rows_ready = true;
     c->last_launches += 1;
-    if (mode == ASD_SQT_FP64) {
-        const long nm = (M + kDmmaTile - 1) / kDmmaTile;
-        if (nm * nm > 0x7fffffffL) return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 GEMM");
-        const size_t nd2 = 2 * (2 * kDmmaTile - 1);
-        rc = ensure_grid_work(c, (size_t)(nm * nm) * nd2,
-                              (size_t)qgrid_keys((int)nm, (int)nm, kDmmaTile, kDmmaTile) * nd2);
-        if (rc != ASD_OK) return rc;
-        DmmaSqtArgs g = dmma_args(c);
-        g.lat_n = N;
-        g.tdiag = c->grid_tdiag;
-        if ((rc = launch_dmma_sqt(g, c->stream)) != ASD_OK) return rc;
-        ASD_CUDA_TRY(launch_qgrid_bins(c->grid_tdiag, (int)nm, (int)nm, kDmmaTile, kDmmaTile, N,
-                                       c->grid_ds, c->grid_g, c->stream));
-        ASD_CUDA_TRY(launch_grid_dft(c->grid_g, N, 1.0 / (double)M, c->grid_t, d_out, c->stream));
-        c->last_launches += 5;
-        return ASD_OK;
-    }
     const int kind = mode_kind(mode);
     if ((rc = ensure_split(c, kind)) != ASD_OK) return rc;
     const int bm = umma_tile_rows(), bn = umma_tile_cols();
@@ -1152,7 +1161,7 @@ void destroy(asd_ctx *c) {
     cudaStreamSynchronize(c->stream);
     void *ptrs[] = {c->y, c->ys_a, c->ys_b, c->acc, c->origin, c->mean_t, c->mean_0, c->uphase,
                     c->wphase, c->row4, c->col4, c->row1, c->col1, c->grid_tdiag, c->grid_ds, c->part,
-                    c->phase_ws, c->phase_G, c->d_out,
+                    c->phase_ws, c->phase_G, c->grid_fft, c->d_out,
                     c->status, c->grid_g, c->grid_t, c->grid_out};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -1756,6 +1765,8 @@ int asd_ctx_debug_poison(asd_ctx *c) {
         {c->grid_ds, c->grid_ds_n * sizeof(double)},
         {c->part, (size_t)c->part_cap * sizeof(double2)},
         {c->phase_ws, phase_work_bytes(c->M, c->K) - sizeof(double2)},  // not the count
+        {c->grid_fft ? c->grid_fft + c->p.N : nullptr,  // not the twiddles
+         qfft_work_bytes(c->p.N, c->K) - (size_t)c->p.N * sizeof(double2)},
         {c->d_out, 2 * sizeof(double)},
         {c->grid_g, (size_t)c->M * sizeof(double)},
         {c->grid_t, (size_t)c->M * sizeof(double2)},

@@ -1,16 +1,13 @@
 // dmma_sqt.cu -- the FP64 tensor-core GEMM (mma.sync m16n8k8 .f64, dmma.cuh)
 // over the whole N^2 x N^2 correlation, for what needs its elements: the
-// magnitude of the terms S(q,t) sums, the q grid, and the cblas_dgemm drop-in.
+// magnitude of the terms S(q,t) sums, and the cblas_dgemm drop-in.
 //
 // The reference's plain path is cblas_dgemm of the whole correlation matrix
 // followed by three sweeps over it (gemm/llg_sqt_mkl.c:378-423).  Here C_ij =
 // alpha * sum_k A_ik B_jk stays in registers and the outer term m_i . z_j comes
 // from per-row and per-column vectors; each CTA leaves one partial:
 //   part[tile] = sum_{i,j in tile} |alpha C_ij - m_i . z_j|
-// The q-grid epilogue instead leaves, per tile, the sums of
-// alpha C_ij - m_i . z_j along each diagonal i - j of the tile, split by
-// whether the lattice column of j wraps around (qgrid.cu bins them by
-// displacement).  Every sum runs in a fixed order: results repeat bit for bit.
+// Every sum runs in a fixed order: results repeat bit for bit.
 //
 // The same main loop with a store epilogue is the plain product behind the
 // cblas_dgemm drop-in (C = alpha A B^T + beta C, A [M][K], B [MB][K]).
@@ -39,9 +36,7 @@ constexpr int GROUP_M = 16;  // row tiles per raster group (A bands stay in L2)
 constexpr int TILE_DOUBLES = BM * BK;          // one operand tile of one stage
 constexpr int STAGE_DOUBLES = (BM + BN) * BK;  // 8192 doubles = 64 KB
 constexpr int PIPE_BYTES = STAGES * STAGE_DOUBLES * 8;
-constexpr int TSTRIDE = BN + 1;  // q grid: epilogue tile row stride (doubles)
-constexpr int GRID_SMEM = BM * TSTRIDE * 8;
-constexpr int EPI_ABS = 0, EPI_GRID = 1, EPI_STORE = 2;
+constexpr int EPI_ABS = 0, EPI_STORE = 1;
 constexpr int KCH = BK / 2;  // 16-byte chunks per shared-memory row
 constexpr int LOG_KCH = 4;
 static_assert(KCH == (1 << LOG_KCH), "chunks per row");
@@ -112,9 +107,8 @@ template <int VEC, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
     dmma_sqt_kernel(const double *__restrict__ A, const double *__restrict__ B, long M, int K,
                     int num_m, int num_n, double alpha, const double *__restrict__ mrow,
-                    const double *__restrict__ zcol, double2 *__restrict__ part, int lat_n,
-                    double *__restrict__ tdiag, long MB, double *__restrict__ Cst, long ldc,
-                    double beta) {
+                    const double *__restrict__ zcol, double2 *__restrict__ part, long MB,
+                    double *__restrict__ Cst, long ldc, double beta) {
     extern __shared__ __align__(16) double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -203,7 +197,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         *cp = (beta != 0.0) ? v + beta * *cp : v;
                     }
             }
-    } else if (EPI == EPI_ABS) {
+    } else {
         // sum over the thread's 8 rows x 8 columns of |alpha C_ij - m_i . z_j|
         double tot = 0.0;
 #pragma unroll
@@ -232,62 +226,6 @@ __global__ void __launch_bounds__(THREADS, 1)
             double sum = 0.0;
             for (int w = 0; w < THREADS / 32; ++w) sum += red[w];
             part[blockIdx.x] = make_double2(sum, 0.0);
-        }
-    } else {
-        // The tile's connected values v_ij into shared memory (zero outside
-        // the lattice), then one thread per diagonal d = r - c sums them in
-        // row order, split by class: 0 when the lattice column of j is at
-        // most that of i (no wrap), 1 otherwise.
-        __syncthreads();  // every warp is done reading the pipeline stages
-        double *T = smem;
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = wm * 64 + mt * 16 + g + 8 * h;
-                const long i = m0 + r;
-                double mx = 0.0, my = 0.0, mz = 0.0;
-                if (i < M) {
-                    mx = mrow[3 * i];
-                    my = mrow[3 * i + 1];
-                    mz = mrow[3 * i + 2];
-                }
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = wn * 32 + nt * 8 + 2 * t + e;
-                        const long j = n0 + c;
-                        double v = 0.0;
-                        if (i < M && j < M) {
-                            v = alpha * acc[mt][nt][2 * h + e];
-                            v -= mx * zcol[3 * j] + my * zcol[3 * j + 1] + mz * zcol[3 * j + 2];
-                        }
-                        T[r * TSTRIDE + c] = v;
-                    }
-            }
-        __syncthreads();
-        constexpr int ND = BM + BN - 1;
-        const long tslot = (long)mb * num_n + nb;
-        for (int dd = threadIdx.x; dd < ND; dd += THREADS) {
-            const int d = dd - (BN - 1);  // r - c
-            const int r0 = d > 0 ? d : 0, r1 = (BM - 1 < BN - 1 + d) ? BM - 1 : BN - 1 + d;
-            // a = (i - j) mod N, the column displacement; class 0 iff col(i) >= a
-            const long delta = m0 - n0 + d;
-            long a = delta % lat_n;
-            if (a < 0) a += lat_n;
-            int xi = (int)((m0 + r0) % lat_n);
-            double s0 = 0.0, s1 = 0.0;
-            for (int r = r0; r <= r1; ++r) {
-                const double v = T[r * TSTRIDE + (r - d)];
-                if (xi >= a)
-                    s0 += v;
-                else
-                    s1 += v;
-                if (++xi == lat_n) xi = 0;
-            }
-            tdiag[(tslot * ND + dd) * 2] = s0;
-            tdiag[(tslot * ND + dd) * 2 + 1] = s1;
         }
     }
 }
@@ -342,34 +280,26 @@ long dmma_sqt_tiles(long M) {
     return nm * nm;
 }
 
-int dmma_sqt_diagonals() { return BM + BN - 1; }
-
 int launch_dmma_sqt(const DmmaSqtArgs &p, cudaStream_t st) {
     const bool store = (p.C != nullptr);
     const long MB = store ? p.MB : p.M;
     if (p.M <= 0 || MB <= 0 || p.K <= 0) return fail(ASD_ERR_INVALID, "empty GEMM");
-    if (store && (p.tdiag || p.ldc < p.M)) return fail(ASD_ERR_INVALID, "store: bad ldc or q grid");
+    if (store && p.ldc < p.M) return fail(ASD_ERR_INVALID, "store: bad ldc");
     const long nm = (p.M + BM - 1) / BM, nn = (MB + BN - 1) / BN;
     if (nm * nn > 0x7fffffffL) return fail(ASD_ERR_UNSUPPORTED, "too many tiles");
     const int num_m = (int)nm, num_n = (int)nn;
-    const bool grid = (p.tdiag != nullptr);
-    if (grid && (p.lat_n < 1 || (long)p.lat_n * p.lat_n != p.M))
-        return fail(ASD_ERR_INVALID, "q grid needs M = N*N");
     const bool vec2 = (p.K % 2 == 0) && (((uintptr_t)p.A | (uintptr_t)p.B) & 15) == 0;
-    const int smem = (grid && GRID_SMEM > PIPE_BYTES) ? GRID_SMEM : PIPE_BYTES;
+    const int smem = PIPE_BYTES;
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         kern<<<(unsigned)(nm * nn), THREADS, smem, st>>>(p.A, p.B, p.M, p.K, num_m, num_n, p.alpha,
-                                                          p.mrow, p.zcol, p.part, p.lat_n, p.tdiag,
-                                                          MB, p.C, p.ldc, p.beta);
+                                                          p.mrow, p.zcol, p.part, MB, p.C, p.ldc, p.beta);
         return cudaGetLastError();
     };
     cudaError_t e;
     if (store)
         e = vec2 ? go(dmma_sqt_kernel<2, EPI_STORE>) : go(dmma_sqt_kernel<1, EPI_STORE>);
-    else if (grid)
-        e = vec2 ? go(dmma_sqt_kernel<2, EPI_GRID>) : go(dmma_sqt_kernel<1, EPI_GRID>);
     else
         e = vec2 ? go(dmma_sqt_kernel<2, EPI_ABS>) : go(dmma_sqt_kernel<1, EPI_ABS>);
     if (e != cudaSuccess) return cuda_fail(e, "dmma_sqt launch");

@@ -144,14 +144,15 @@ int asd_ctx_sqt_magnitude(asd_ctx *ctx, double *out);
 
 /* S(q,t) for every q = 2*pi*(a, b)/N of the N x N grid, into d_out[2*(a*N+b)]
  * (real) and d_out[2*(a*N+b)+1] (imaginary), a device buffer of 2*N*N
- * doubles; asynchronous.  The same correlation GEMM (any asd_sqt_mode),
- * with an epilogue that sums every connected C_ij - m_i . z_j along the
- * diagonals i - j of each tile; the diagonal sums are binned by displacement
- * r_i - r_j (mod N) and a 2-D DFT of the N*N bins gives S at every q.
- * d_out[2*(vx*N+vy)] equals asd_ctx_sqt's value up to rounding.  Any N; work
- * space on the first call: 8 * (128 + BN - 1) * 2 bytes per GEMM tile (BN =
- * 128 in FP64, 256 in the split modes; 1.1 GB / 0.8 GB at N = 256).  Every
- * sum runs in a fixed order, so results repeat bit for bit.
+ * doubles; asynchronous.  In FP64 the 2-D transforms of the spins at t and at
+ * the origin, multiplied and summed over the replicas.  In the split modes the
+ * correlation GEMM with an epilogue that sums every connected C_ij - m_i . z_j
+ * along the diagonals i - j of each tile; the diagonal sums are binned by
+ * displacement r_i - r_j (mod N) and a 2-D DFT of the N*N bins gives S at every
+ * q.  d_out[2*(vx*N+vy)] equals asd_ctx_sqt's value up to rounding.  Any N
+ * (FP64: up to 2435); work space on the first call: a few MB in FP64, 8 * 383 * 2
+ * bytes per GEMM tile of 128 x 256 in the split modes (0.8 GB at N = 256).
+ * Every sum runs in a fixed order, so results repeat bit for bit.
  * No counterpart in the reference (its programs evaluate one q). */
 int asd_ctx_sqt_grid_async(asd_ctx *ctx, asd_sqt_mode mode, double *d_out);
 /* Same into host memory (2*N*N doubles); synchronous. */
