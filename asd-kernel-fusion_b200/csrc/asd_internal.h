@@ -60,6 +60,13 @@ cudaError_t launch_llg_stage(int stage, const LLGArgs &a, const double *y, const
 // (distinct buffers), replicas [a.f0, a.f0 + a.nc) only.
 cudaError_t launch_llg_step_fused(const LLGArgs &a, const double *y, double *yout,
                                   cudaStream_t st);
+// nsteps (>= 1) RK4 steps in one launch, each replica's lattice resident on one
+// SM or on a cluster of up to 8: y -> yout (may be the same buffer), replicas
+// [a.f0, a.f0 + a.nc); scratch: nc * 3 * M doubles.  llg_resident_wins:
+// the lattice side allows it and it is the fastest of the three ways to step.
+cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout, double *scratch,
+                                int nsteps, cudaStream_t st);
+bool llg_resident_wins(const LLGArgs &a, int nsteps);
 // True if the streamed one-launch step has enough work for this lattice and
 // replica range to fill the GPU (at least 8 rows per resident CTA).
 bool llg_fused_fills(const LLGArgs &a);

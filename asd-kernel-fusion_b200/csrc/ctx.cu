@@ -10,6 +10,7 @@
 //   q-grid work          per-tile diagonal partials (on the first q grid)
 // The AoS <-> site-major transposes stage through ys_b.
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -358,14 +359,23 @@ int set_spins_common(asd_ctx *c, const double *aos, bool host, int as_origin) {
     return ASD_OK;
 }
 
-// The LLG kernel for replicas [a.f0, a.f0 + a.nc): the one-launch step or
-// the four stage kernels (ASD_LLG_AUTO: the former where it fills the GPU).
+// The LLG kernel for one step of replicas [a.f0, a.f0 + a.nc) out of place: the
+// one-launch step or the four stage kernels (ASD_LLG_AUTO: the former where it
+// fills the GPU; steps in place may also run resident, llg_resident_wins).
 bool use_fused(const asd_ctx *c, const LLGArgs &a) {
     return c->llg_kernel == ASD_LLG_FUSED_STEP ||
            (c->llg_kernel == ASD_LLG_AUTO && llg_fused_fills(a));
 }
 
 int run_steps(asd_ctx *c, int nsteps) {
+    if (nsteps > 0 && c->llg_kernel == ASD_LLG_AUTO && llg_resident_wins(c->a, nsteps)) {
+        cudaEvent_t t0 = time_begin(c, c->stream);
+        ASD_CUDA_TRY(launch_llg_resident(c->a, c->y, c->y, c->ys_b, nsteps, c->stream));
+        time_end(c, 0, nsteps, c->stream, t0);
+        c->last_launches += 1;
+        c->state_version += nsteps;
+        return ASD_OK;
+    }
     if (use_fused(c, c->a)) {
         for (int s = 0; s < nsteps; ++s) {
             cudaEvent_t t0 = time_begin(c, c->stream);
@@ -668,20 +678,29 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
     ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[0], c->origin, sb, cudaMemcpyDeviceToDevice, st));
     double *cur = b.seg[0], *nxt = b.seg[1];
     ASD_CUDA_TRY(cudaMemcpyAsync(cur, c->origin, sb, cudaMemcpyDeviceToDevice, st));
-    // Only states are kept on the way forward: one launch per step where
-    // that fills the GPU.
+    // Only states are kept on the way forward, and only at the multiples of
+    // ckpt and stride: the steps up to the next one in one launch where the
+    // lattices stay resident, else one launch a step where that fills the GPU.
     const bool fwd_fused = use_fused(c, c->a);
-    for (int n = 1; n <= nsteps; ++n) {
-        if (fwd_fused) {
-            ASD_CUDA_TRY(launch_llg_step_fused(c->a, cur, nxt, st));
+    for (int n = 0; n < nsteps;) {
+        const int run = std::min(nsteps, std::min((n / ckpt + 1) * ckpt, (n / stride + 1) * stride)) - n;
+        if (c->llg_kernel == ASD_LLG_AUTO && llg_resident_wins(c->a, run)) {
+            ASD_CUDA_TRY(launch_llg_resident(c->a, cur, cur, b.s2, run, st));
             c->last_launches += 1;
+            n += run;
         } else {
-            if ((rc = step_into(c, cur, b.s2, b.s3, b.s4, b.acc, nxt)) != ASD_OK) return rc;
-            c->last_launches += 4;
+            if (fwd_fused) {
+                ASD_CUDA_TRY(launch_llg_step_fused(c->a, cur, nxt, st));
+                c->last_launches += 1;
+            } else {
+                if ((rc = step_into(c, cur, b.s2, b.s3, b.s4, b.acc, nxt)) != ASD_OK) return rc;
+                c->last_launches += 4;
+            }
+            double *t = cur;
+            cur = nxt;
+            nxt = t;
+            n += 1;
         }
-        double *t = cur;
-        cur = nxt;
-        nxt = t;
         if (n % ckpt == 0 && n / ckpt < nck)
             ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[n / ckpt], cur, sb, cudaMemcpyDeviceToDevice, st));
         if (n % stride == 0 && n / stride <= E) {

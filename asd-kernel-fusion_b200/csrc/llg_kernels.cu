@@ -6,6 +6,9 @@
 // an FMA.  With alpha = J2 = h = 0 the trajectory is therefore bit-identical
 // to the reference's euler / runge_kutta / renormalisation built with
 // -ffp-contract=off (llg_sqt_baseline.c:29-142, :298-309).
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -450,6 +453,195 @@ cudaError_t launch_stream(const LLGArgs &a, const double *y, double *yout, cudaS
     }
 }
 
+// ------------------------------------------------- resident steps
+// Any number of RK4 steps in one launch, one replica's whole lattice held on
+// chip: a thread-block cluster of S CTAs (S = 1: a CTA) per replica, its rows
+// split over the CTAs.  A CTA keeps the stage input and the stage output of its
+// rows in shared memory (rows of 3 x W doubles, one halo row above and below,
+// the two swapped after every stage); a thread owns up to RP consecutive rows of
+// one column, whose running RK4 combination stays in registers and whose base
+// values y lie in a planar scratch in L2, read and written by that thread alone.
+// Walking down its column a thread reuses the two rows above from registers: 9
+// shared loads per site and stage instead of 15 (21 instead of 27 with J2), all
+// at compile-time offsets.  The first and last row of a CTA are also stored into
+// the neighbouring CTAs' halo rows (distributed shared memory, or the same
+// CTA's when S = 1), so one barrier ends a stage.  No redundant halo
+// arithmetic, no traffic between steps.
+//
+// Up to 32 columns: CTAs of 256 threads with at most 4 rows each, three to an SM
+// (85 registers); above, 512 threads with at most 8 rows, one to an SM (128).
+namespace resident {
+__host__ __device__ constexpr int threads(int W) { return W <= 32 ? 256 : 512; }
+__host__ __device__ constexpr int rows_per_thread(int W) { return W <= 32 ? 4 : 8; }
+__host__ __device__ constexpr int ctas_per_sm(int W) { return W <= 32 ? 3 : 1; }
+}  // namespace resident
+
+struct ResGeom {
+    int s;       // CTAs per replica
+    int rows;    // rows of the largest CTA
+    int groups;  // row groups: threads / N
+};
+
+template <int W, bool J2, bool H, bool DAMP, bool UNIT, bool CL>
+__global__ void __launch_bounds__(resident::threads(W), resident::ctas_per_sm(W))
+    llg_resident_kernel(LLGArgs a, ResGeom g, const double *y, double *yout, double *scratch,
+                        int nsteps) {
+    namespace cg = cooperative_groups;
+    constexpr int RP = resident::rows_per_thread(W), WARPS = resident::threads(W) / 32;
+    constexpr int RS = 3 * W;  // doubles per row
+    extern __shared__ double rsm[];
+    const int N = a.N, rank = CL ? (int)(blockIdx.x % g.s) : 0;
+    const int lf = CL ? (int)(blockIdx.x / g.s) : (int)blockIdx.x;
+    const int r0 = (int)((long)rank * N / g.s), nr = (int)((long)(rank + 1) * N / g.s) - r0;
+    const int bs = (g.rows + 2) * RS;  // doubles per buffer
+    const long K = 3L * a.nfile, off = 3L * (a.f0 + lf);
+    double *ysc = scratch + (long)lf * 3 * a.M;  // [3][M]: this replica's y
+
+    // every CTA's rows and halo rows of the initial state, a warp per row:
+    // consecutive lanes take the components of a site, then the next site
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int l = warp; l < nr + 2; l += WARPS) {
+        int row = r0 - 1 + l;
+        row = row < 0 ? row + N : (row >= N ? row - N : row);
+        const double *src = y + (long)row * N * K + off;
+        for (int x = lane; x < 3 * N; x += 32)
+            cp_async8(rsm + l * RS + (x % 3) * W + x / 3, src + (long)(x / 3) * K + x % 3);
+    }
+    cp_async_commit();
+    double *up_cta = rsm, *dn_cta = rsm;  // shared memory of the CTAs above and below
+    int nr_up = nr;
+    if (CL) {
+        cg::cluster_group cluster = cg::this_cluster();
+        const int ru = rank == 0 ? g.s - 1 : rank - 1, rd = rank + 1 == g.s ? 0 : rank + 1;
+        up_cta = cluster.map_shared_rank(rsm, ru);
+        dn_cta = cluster.map_shared_rank(rsm, rd);
+        nr_up = (int)((long)(ru + 1) * N / g.s) - (int)((long)ru * N / g.s);
+    }
+    auto barrier = [&] {
+        if (CL) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    const int grp = threadIdx.x / N, col = threadIdx.x - grp * N;
+    const int rp = (nr + g.groups - 1) / g.groups;      // <= RP
+    const int first = grp * rp;                         // this thread's rows of the CTA
+    const int cnt = grp < g.groups ? min(rp, nr - first) : 0;
+    const int dl = col == 0 ? N - 1 : -1, dr = col == N - 1 ? 1 - N : 1;
+    const int at0 = (first + 1) * RS + col;
+    const long site0 = (long)(r0 + first) * N + col;
+    // halo copies of the CTA's first and last row (only their owners use them)
+    const bool owns_top = cnt > 0 && first == 0, owns_bot = cnt > 0 && first + cnt == nr;
+    double *const halo_up = up_cta + (nr_up + 1) * RS + col, *const halo_dn = dn_cta + col;
+    cp_async_wait_all();
+    barrier();
+
+    double acc[RP][3];
+    // One stage, buffer `in` to buffer `out`; body(r, s, k) gives the output of
+    // the thread's row r from its value s and k = dt f.
+    auto walk = [&](int in, int out, auto body) {
+        const double *const p = rsm + in * bs + at0, *const pl = p + dl, *const pr = p + dr;
+        double *const o = rsm + out * bs + at0;
+        const int ob = out * bs;
+        auto at = [](const double *q) { return V3{q[0], q[W], q[2 * W]}; };
+        V3 up, mid;
+        if (cnt > 0) {
+            up = at(p - RS);
+            mid = at(p);
+        }
+#pragma unroll
+        for (int r = 0; r < RP; ++r) {
+            if (r < cnt) {
+                const int q = r * RS;
+                V3 nb[4], n2[4];
+                nb[0] = at(p + q + RS);
+                nb[1] = up;
+                nb[2] = at(pl + q);
+                nb[3] = at(pr + q);
+                if (J2) {
+                    n2[0] = at(pr + q + RS);
+                    n2[1] = at(pl + q + RS);
+                    n2[2] = at(pr + q - RS);
+                    n2[3] = at(pl + q - RS);
+                }
+                const V3 d = llg_rhs_vals<J2, H, DAMP, UNIT>(mid, nb, n2, a);
+                const V3 v = body(r, mid, V3{dm(d.x, a.dt), dm(d.y, a.dt), dm(d.z, a.dt)});
+                o[q] = v.x;
+                o[q + W] = v.y;
+                o[q + 2 * W] = v.z;
+                if (r == 0 && owns_top) {
+                    halo_up[ob] = v.x;
+                    halo_up[ob + W] = v.y;
+                    halo_up[ob + 2 * W] = v.z;
+                }
+                if (owns_bot && r == cnt - 1) {
+                    halo_dn[ob] = v.x;
+                    halo_dn[ob + W] = v.y;
+                    halo_dn[ob + 2 * W] = v.z;
+                }
+                up = mid;
+                mid = nb[0];
+            }
+        }
+    };
+    for (int step = 0; step < nsteps; ++step) {
+        // Stages 1 to 3: out = y + ck k; acc = y + k/6, then acc + k/3.  One copy
+        // of the code: the divisors and their reciprocals (div6, div3) and the
+        // factors 1/2 and 1 are uniform variables, the roundings the same.
+#pragma unroll 1
+        for (int st = 1; st <= 3; ++st) {
+            const double ck = st == 3 ? 1.0 : 0.5, dd = st == 1 ? 6.0 : 3.0;
+            const double inv = st == 1 ? 1.0 / 6.0 : 1.0 / 3.0;
+            double *yp = ysc + site0;
+            walk((st - 1) & 1, st & 1, [&](int r, const V3 &s, const V3 &k) {
+                V3 yb = s;
+                if (st > 1) {
+                    yb = V3{yp[0], yp[a.M], yp[2 * a.M]};
+                } else if (step == 0) {  // later steps: written by stage 4
+                    yp[0] = s.x;
+                    yp[a.M] = s.y;
+                    yp[2 * a.M] = s.z;
+                }
+                yp += N;
+                auto div = [&](double x) {
+                    const double q = __dmul_rn(x, inv);
+                    const double t = __fma_rn(q, dd, -x);
+                    return __fma_rn(-t, inv, q);
+                };
+                const double bx = st == 1 ? yb.x : acc[r][0], by = st == 1 ? yb.y : acc[r][1],
+                             bz = st == 1 ? yb.z : acc[r][2];
+                acc[r][0] = da(bx, div(k.x));
+                acc[r][1] = da(by, div(k.y));
+                acc[r][2] = da(bz, div(k.z));
+                return V3{da(yb.x, dm(k.x, ck)), da(yb.y, dm(k.y, ck)), da(yb.z, dm(k.z, ck))};
+            });
+            barrier();
+        }
+        double *yp = ysc + site0;
+        const bool more = step + 1 < nsteps;
+        walk(1, 0, [&](int r, const V3 &, const V3 &k) {
+            const double o0 = da(acc[r][0], div6(k.x));
+            const double o1 = da(acc[r][1], div6(k.y));
+            const double o2 = da(acc[r][2], div6(k.z));
+            const double nrm = __dsqrt_rn(da(da(dm(o0, o0), dm(o1, o1)), dm(o2, o2)));
+            const V3 v{dq(dm(a.spin_len, o0), nrm), dq(dm(a.spin_len, o1), nrm),
+                       dq(dm(a.spin_len, o2), nrm)};
+            if (more) {
+                yp[0] = v.x;
+                yp[a.M] = v.y;
+                yp[2 * a.M] = v.z;
+                yp += N;
+            }
+            return v;
+        });
+        barrier();  // also: no CTA leaves while another may store into its halo rows
+    }
+    for (int l = warp; l < nr; l += WARPS) {
+        double *dst = yout + (long)(r0 + l) * N * K + off;
+        const double *src = rsm + (l + 1) * RS;
+        for (int x = lane; x < 3 * N; x += 32)
+            dst[(long)(x / 3) * K + x % 3] = src[(x % 3) * W + x / 3];
+    }
+}
+
 // Tiled transpose between [nfile][M][3] and [M][nfile][3] through shared
 // memory: 32 sites x 32 replicas x 3 doubles per block.
 template <bool TO_SITEMAJOR>
@@ -576,6 +768,120 @@ cudaError_t launch_llg_stage(int stage, const LLGArgs &a, const double *y, const
         case 4: return launch_stage_t<4>(a, y, ys_in, acc, ys_out, st);
     }
     return cudaErrorInvalidValue;
+}
+
+// The geometry of the resident steps for lattice side N: rows of W doubles a
+// component, the fewest CTAs per replica (1, 2, 4, 8) whose threads cover the
+// rows and whose two buffers fit shared memory; false if none does.
+static bool resident_geom(int N, ResGeom &g, int &w, size_t &smem) {
+    w = N <= 32 ? 32 : N <= 64 ? 64 : 128;
+    if (N > w) return false;
+    g.groups = resident::threads(w) / N;
+    for (g.s = 1; g.s <= 8 && g.s <= N; g.s *= 2) {
+        g.rows = (N + g.s - 1) / g.s;
+        smem = (size_t)2 * 3 * (g.rows + 2) * w * sizeof(double);
+        if ((g.rows + g.groups - 1) / g.groups <= resident::rows_per_thread(w) && smem <= 227 * 1024) return true;
+    }
+    return false;
+}
+
+template <int W, bool J2, bool H, bool DAMP, bool UNIT>
+static cudaError_t launch_resident_t(const LLGArgs &a, const ResGeom &g, size_t smem,
+                                     const double *y, double *yout, double *scratch, int nsteps,
+                                     cudaStream_t st) {
+    constexpr bool CL = W > 64;  // up to 64 columns one CTA holds a lattice
+    auto k = llg_resident_kernel<W, J2, H, DAMP, UNIT, CL>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((long)a.nc * g.s));
+    cfg.blockDim = dim3(resident::threads(W));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)g.s;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CL ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, a, g, y, yout, scratch, nsteps);
+}
+
+template <int W>
+static cudaError_t launch_resident_w(const LLGArgs &a, const ResGeom &g, size_t smem,
+                                     const double *y, double *yout, double *scratch, int nsteps,
+                                     cudaStream_t st) {
+    const bool unit = a.J1 == 1.0 || a.J1 == -1.0;
+    const int sel = (a.use_j2 ? 4 : 0) | (a.use_h ? 2 : 0) | (a.use_damp ? 1 : 0);
+#define ASD_RES_CASE(S, J, Hh, D)                                                                 \
+    case S:                                                                                       \
+        return unit ? launch_resident_t<W, J, Hh, D, true>(a, g, smem, y, yout, scratch, nsteps,  \
+                                                           st)                                    \
+                    : launch_resident_t<W, J, Hh, D, false>(a, g, smem, y, yout, scratch, nsteps, \
+                                                            st);
+    switch (sel) {
+        ASD_RES_CASE(0, false, false, false)
+        ASD_RES_CASE(1, false, false, true)
+        ASD_RES_CASE(2, false, true, false)
+        ASD_RES_CASE(3, false, true, true)
+        ASD_RES_CASE(4, true, false, false)
+        ASD_RES_CASE(5, true, false, true)
+        ASD_RES_CASE(6, true, true, false)
+        ASD_RES_CASE(7, true, true, true)
+    }
+#undef ASD_RES_CASE
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout, double *scratch,
+                                int nsteps, cudaStream_t st) {
+    ResGeom g;
+    int w = 0;
+    size_t smem = 0;
+    if (nsteps < 1 || a.f0 < 0 || a.nc < 1 || a.f0 + a.nc > a.nfile ||
+        !resident_geom(a.N, g, w, smem))
+        return cudaErrorInvalidValue;
+    return w == 32   ? launch_resident_w<32>(a, g, smem, y, yout, scratch, nsteps, st)
+           : w == 64 ? launch_resident_w<64>(a, g, smem, y, yout, scratch, nsteps, st)
+                     : launch_resident_w<128>(a, g, smem, y, yout, scratch, nsteps, st);
+}
+
+// The three ways to step, compared by what each was measured to take on B200 (in
+// us a step; the lines below are within 10 % of the measurements that matter,
+// those near the crossings).  w = site-replicas, n = sites of a CTA:
+//   stage kernels   16 + 0.065e-3 w (0.073 with J2): four launches, then HBM / L2
+//   one-launch      the larger of 48 and 10 + 0.055e-3 w (0.068)
+//   resident        4 a launch, and per round of resident CTAs, q to an SM:
+//                   2.3 + 3.7e-3 q n a step (4.7 with J2; clusters 6.3 + 3.9e-3 n),
+//                   and 0.8 + 2.6e-3 q n once to load and store the lattice
+// Measured, stage kernels / one-launch / resident 1 step / resident 10 steps:
+//   32x32x50    16.4 /  39 / 13.7 /  7.0     64x64x8    16.4 / 47 / 31.5 / 18.5
+//   32x32x200   29.0 /  37 / 18.9 / 10.3     64x64x100  43.6 / 49 / 35.3 / 18.9
+//   32x32x1000  76.1 /  71 / 52.0 / 31.8     12x12x1000 24.6 / 50 / 18.9 / 10.1
+//   64x64x400   121 / 105 / 109 / 57.8       128x128x500 548 / 388 / 604 / 333
+//   51x51x70    29.4 /  49 / 25.1 / 13.6
+bool llg_resident_wins(const LLGArgs &a, int nsteps) {
+    ResGeom g;
+    int w = 0;
+    size_t smem = 0;
+    if (!resident_geom(a.N, g, w, smem)) return false;
+    const double work = (double)a.M * a.nc, n = (double)g.rows * a.N;
+    const double stages = 16.0 + (a.use_j2 ? 0.073e-3 : 0.065e-3) * work;
+    const double fused = std::max(48.0, 10.0 + (a.use_j2 ? 0.068e-3 : 0.055e-3) * work);
+    const bool cl = g.s > 1;
+    // CTAs an SM has to take in all, and at once (clusters of 4 fill about 140
+    // of the 148 SMs)
+    const long total = (long)a.nc * g.s, per_sm = (total + (cl ? 139 : 147)) / (cl ? 140 : 148);
+    const double base = cl ? 6.3 : 2.3, site = (cl ? 3.9e-3 : 3.7e-3) * (a.use_j2 ? 1.27 : 1.0);
+    double res = 4.0;
+    for (long left = per_sm; left > 0;) {
+        const long q = std::min<long>(left, resident::ctas_per_sm(w));
+        const long rounds = left / q;
+        res += rounds * (nsteps * (base + site * q * n) + 0.8 + 2.6e-3 * q * n);
+        left -= rounds * q;
+    }
+    return res < 0.95 * nsteps * (llg_fused_fills(a) ? fused : stages);
 }
 
 bool llg_fused_fills(const LLGArgs &a) {

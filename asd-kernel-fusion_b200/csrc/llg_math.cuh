@@ -41,19 +41,28 @@ struct V3 {
 // dS/dt from the centre spin s and its neighbours' values nb (nearest, in the
 // reference's order) and n2 (diagonal; read only when J2).  The exchange field
 // starts at 0 and accumulates t*J1 per neighbour (llg_sqt_baseline.c:52,
-// :73-75); tau = H x S (v3d_cross, v3d.h:48-53).  Extensions, each skipped
+// :73-75).  With UNIT, for |J1| = 1, the four neighbours are added first and J1
+// applied once: the products t*J1 are exact, rounding to nearest is symmetric
+// in the sign, and neither form gives -0 (the sums start from +0, and the FMA
+// adds +0), so the bits are the same for 5 operations instead of 8 a component.
+// tau = H x S (v3d_cross, v3d.h:48-53).  Extensions, each skipped
 // when zero: J2 over the diagonal neighbours, the Zeeman field, and Gilbert
 // damping g * (tau + alpha * (S x tau)).  Every kernel that evaluates the
 // right-hand side goes through this function, so all share one operation order.
-template <bool J2, bool H, bool DAMP>
+template <bool J2, bool H, bool DAMP, bool UNIT = false>
 __device__ __forceinline__ V3 llg_rhs_vals(const V3 &s, const V3 (&nb)[4], const V3 (&n2)[4],
                                            const LLGArgs &a) {
     double ex = 0.0, ey = 0.0, ez = 0.0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        ex = da(ex, dm(nb[j].x, a.J1));
-        ey = da(ey, dm(nb[j].y, a.J1));
-        ez = da(ez, dm(nb[j].z, a.J1));
+        ex = da(ex, UNIT ? nb[j].x : dm(nb[j].x, a.J1));
+        ey = da(ey, UNIT ? nb[j].y : dm(nb[j].y, a.J1));
+        ez = da(ez, UNIT ? nb[j].z : dm(nb[j].z, a.J1));
+    }
+    if (UNIT) {
+        ex = __fma_rn(ex, a.J1, 0.0);
+        ey = __fma_rn(ey, a.J1, 0.0);
+        ez = __fma_rn(ez, a.J1, 0.0);
     }
     if (J2) {
 #pragma unroll

@@ -259,11 +259,13 @@ int asd_ctx_shard_sqt_finish(asd_ctx *ctx, const double *d_part, const double *d
                                 memory by column band (48 B of DRAM traffic per
                                 site-step; FP64-bound; 1.35x the stages at
                                 128x128x500, 1.6x at 256x256x1000 on B200)  */
-#define ASD_LLG_AUTO 2       /* default: the one-launch step when the lattice
-                                and replicas give it at least 8 rows of work
-                                per resident CTA (e.g. 128x128x500, or its
-                                64-replica chunks), else the stage kernels
-                                (e.g. 64x64x100)                             */
+#define ASD_LLG_AUTO 2       /* default: the fastest of three for the lattice,
+                                replicas and steps of the call: the stage
+                                kernels, the one-launch step, or the resident
+                                steps (each replica's lattice held on one SM, or
+                                a cluster of SMs, for all steps of an
+                                asd_ctx_step; up to N = 128: 64x64x100
+                                43.6 -> 18.9 us a step on B200)              */
 int asd_ctx_set_llg_kernel(asd_ctx *ctx, int kernel);
 
 /* K elements accumulated per TMEM chunk by the split S(q,t) modes (rounded
@@ -288,7 +290,8 @@ int asd_ctx_last_launches(const asd_ctx *ctx);
 int asd_ctx_time_kernels(asd_ctx *ctx, int on);
 /* Waits for the events recorded since the last read and returns the summed
  * duration in ms and the number of kernel launches of `which` (0 = RK4 step
- * kernels, 1 = S(q,t) GEMM), then forgets them. */
+ * kernels, 1 = S(q,t) GEMM; a launch of several resident RK4 steps counts once
+ * per step), then forgets them. */
 int asd_ctx_kernel_time(asd_ctx *ctx, int which, double *ms, int *launches);
 
 /* Status word set by device code (bounded waits that gave up, etc.);
