@@ -189,9 +189,10 @@ cudaError_t launch_scale_f64(double *c, long m, long n, long ldc, double beta, c
 long qgrid_keys(int num_m, int num_n, int bm, int bn);
 cudaError_t launch_qgrid_bins(const double *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
                               double *ds, double *G, cudaStream_t st);
-// out[2*(a*N+b)+{0,1}] = scale * sum_d G[d] e^{-2 pi i (a dr + b dc)/N}; tmp holds N*N double2.
-cudaError_t launch_grid_dft(const double *G, int lat_n, double scale, double2 *tmp, double *out,
-                            cudaStream_t st);
+// out[2*(a*N+b)+{0,1}] = scale * sum_d G[d] e^{-2 pi i (a dr + b dc)/N} (qfft.cu); tw: N twiddles
+// (launch_qfft_twiddles), T: N*N of work space.
+cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const double2 *tw, double2 *T,
+                            double *out, cudaStream_t st);
 
 // out[0..1] = (sum of nparts partials) * scale, deterministic order.
 cudaError_t launch_finalize(const double2 *part, int nparts, double scale, double *out,

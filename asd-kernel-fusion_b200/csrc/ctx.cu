@@ -89,7 +89,7 @@ struct asd_ctx {
     int chunk_k = -1;  // < 0: per mode, 512 for TF32x3, 1024 for BF16x3 and FP16x3
     double2 *grid_fft = nullptr;  // q grid, FP64: twiddles, sums over k
     double *grid_g = nullptr;     // q grid, split modes: N*N displacement bins (FP64)
-    double2 *grid_t = nullptr;    // q grid: DFT intermediate
+    double2 *grid_t = nullptr;    // q grid, split modes: DFT intermediate, then N twiddles
     double *grid_out = nullptr;   // q grid: device result for the host-buffer form
     double *grid_tdiag = nullptr; // q grid: per-tile diagonal partials
     size_t grid_tdiag_n = 0;
@@ -889,7 +889,16 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
     // each checked on its own: after a failed allocation of grid_t, grid_g
     // is already there and the next call must still allocate grid_t
     if (!c->grid_g && (rc = dalloc(&c->grid_g, (size_t)M * sizeof(double))) != ASD_OK) return rc;
-    if (!c->grid_t && (rc = dalloc(&c->grid_t, (size_t)M * sizeof(double2))) != ASD_OK) return rc;
+    if (!c->grid_t) {
+        if ((rc = dalloc(&c->grid_t, (size_t)(M + N) * sizeof(double2))) != ASD_OK) return rc;
+        const cudaError_t e = launch_qfft_twiddles(N, c->grid_t + M, c->stream);
+        if (e != cudaSuccess) {  // unusable without its twiddles
+            cudaFree(c->grid_t);
+            c->grid_t = nullptr;
+            return cuda_fail(e, "launch_qfft_twiddles");
+        }
+        c->last_launches += 1;
+    }
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
                                   c->stream));
     c->rows_ready = true;
@@ -909,8 +918,9 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
     ASD_CUDA_TRY(launch_qgrid_bins(c->grid_tdiag, num_m, num_n, bm, bn, N, c->grid_ds, c->grid_g,
                                    c->stream));
     c->last_launches += 3;
-    ASD_CUDA_TRY(launch_grid_dft(c->grid_g, N, 1.0 / (double)M, c->grid_t, d_out, c->stream));
-    c->last_launches += 1;
+    ASD_CUDA_TRY(launch_bins_dft(c->grid_g, N, 1.0 / (double)M, c->grid_t + M, c->grid_t, d_out,
+                                 c->stream));
+    c->last_launches += 2;
     return ASD_OK;
 }
 

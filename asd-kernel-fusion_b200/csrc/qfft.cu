@@ -25,7 +25,8 @@
 // whatever the stride along the lattice: no bank conflicts for any radix.
 // Stockham stages of radix 8, 4, 2, 3, 5 in registers; any other prime factor p
 // as p-term sums from the twiddle table, so every N works.  Fixed order of
-// summation everywhere: the grid repeats bit for bit.
+// summation everywhere: the grid repeats bit for bit.  The split modes' N x N
+// displacement bins take the same transform (bins_dft_kernel).
 //
 // Bound by shared-memory traffic (each stage reads and writes 16 bytes a point)
 // and, below about 64 x 64, by launch latency.  Measured on B200 against the FP64
@@ -307,6 +308,38 @@ __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict
     }
 }
 
+// One dimension of the 2-D transform of the displacement bins (split modes):
+// a block transforms KC lines.  REAL: lines are rows of G [n][n], the result
+// goes transposed to T [frequency][line]; else lines are rows of T, the result
+// to out, scaled.
+template <bool REAL>
+__global__ void __launch_bounds__(MAX_THREADS) bins_dft_kernel(FftPlan p,
+                                                               const double *__restrict__ G,
+                                                               const double2 *__restrict__ T,
+                                                               const double2 *__restrict__ tw,
+                                                               double scale,
+                                                               double2 *__restrict__ out) {
+    extern __shared__ __align__(16) double2 fsm[];
+    const int n = p.n, kc = 1 << p.lk;
+    double2 *b0 = fsm, *b1 = fsm + (n << p.lk), *stw = b1 + (n << p.lk);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) stw[j] = tw[j];
+    const int l0 = blockIdx.x * kc;
+    for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x) {
+        const int line = l0 + (idx & (kc - 1));
+        const long e = (long)line * n + (idx >> p.lk);
+        double2 v = make_double2(0.0, 0.0);
+        if (line < n) v = REAL ? make_double2(G[e], 0.0) : T[e];
+        b0[idx] = v;
+    }
+    __syncthreads();
+    const double2 *f = transform(b0, b1, stw, p);
+    for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x) {
+        const int line = l0 + (idx & (kc - 1));
+        if (line < n)
+            out[(long)(idx >> p.lk) * n + line] = make_double2(f[idx].x * scale, f[idx].y * scale);
+    }
+}
+
 FftPlan make_plan(int n, int K) {
     FftPlan p{};
     p.n = n;
@@ -402,6 +435,25 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
         part, lat_n, g.slices, scale, reinterpret_cast<double2 *>(out));
     ASD_CUDA_TRY(cudaGetLastError());
     return launches + 1;
+}
+
+cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const double2 *tw, double2 *T,
+                            double *out, cudaStream_t st) {
+    const FftPlan p = make_plan(lat_n, 16);
+    const int kc = 1 << p.lk, blocks = (lat_n + kc - 1) / kc, threads = threads_for(p);
+    const size_t smem = rows_smem(p);
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(bins_dft_kernel<true>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess ||
+        (e = cudaFuncSetAttribute(bins_dft_kernel<false>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess)
+        return e;
+    bins_dft_kernel<true><<<blocks, threads, smem, st>>>(p, G, nullptr, tw, 1.0, T);
+    bins_dft_kernel<false><<<blocks, threads, smem, st>>>(p, nullptr, T, tw, scale,
+                                                          reinterpret_cast<double2 *>(out));
+    return cudaGetLastError();
 }
 
 }  // namespace asd

@@ -42,11 +42,12 @@ __global__ void qgrid_keys_kernel(const double *__restrict__ tdiag, int num_m, i
     // tiles: mb = kp (mod R), 0 <= mb < num_m, 0 <= nb = (mb - kp) / R < num_n
     long mb = kp >= 0 ? kp : ((kp % R) + R) % R;
     const long mb_end = kp + (long)R * num_n;  // nb < num_n
+    // consecutive tiles of a key lie a constant distance apart
+    const double *t = tdiag + (mb * num_n + (mb - kp) / R) * nd * 2 + rem;
+    const long step = ((long)R * num_n + 1) * nd * 2, end = num_m < mb_end ? num_m : mb_end;
     double s = 0.0;
-    for (; mb < num_m && mb < mb_end; mb += R) {
-        const long nb = (mb - kp) / R;
-        s += tdiag[(mb * num_n + nb) * nd * 2 + rem];
-    }
+#pragma unroll 8
+    for (; mb < end; mb += R, t += step) s += *t;
     ds[idx] = s;
 }
 

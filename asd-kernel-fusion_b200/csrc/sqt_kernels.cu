@@ -198,42 +198,6 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const double *__restrict
 }
 
 
-// Separable 2-D DFT of the displacement histogram: T[dr][b] = sum_dc G[dr][dc]
-// e^{-2 pi i b dc / N}, then S[a][b] = scale * sum_dr T[dr][b] e^{-2 pi i a dr / N}.
-__global__ void grid_dft_rows_kernel(const double *__restrict__ G, int N,
-                                     double2 *__restrict__ T) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N * N) return;
-    const int dr = t / N, b = t % N;
-    double re = 0.0, im = 0.0;
-    for (int dc = 0; dc < N; ++dc) {
-        double sn, cs;
-        sincospi(2.0 * (double)((b * dc) % N) / (double)N, &sn, &cs);
-        const double g = G[dr * N + dc];
-        re += g * cs;
-        im -= g * sn;
-    }
-    T[t] = make_double2(re, im);
-}
-
-__global__ void grid_dft_cols_kernel(const double2 *__restrict__ T, int N, double scale,
-                                     double *__restrict__ out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= N * N) return;
-    const int a = t / N, b = t % N;
-    double re = 0.0, im = 0.0;
-    for (int dr = 0; dr < N; ++dr) {
-        double sn, cs;
-        sincospi(2.0 * (double)((a * dr) % N) / (double)N, &sn, &cs);
-        const double2 v = T[dr * N + b];
-        // (v.x + i v.y) (cs - i sn)
-        re += v.x * cs + v.y * sn;
-        im += v.y * cs - v.x * sn;
-    }
-    out[2 * t] = re * scale;
-    out[2 * t + 1] = im * scale;
-}
-
 // Single block, fixed summation order: thread t sums t, t+256, ... then a
 // shared-memory tree.
 __global__ void __launch_bounds__(256) finalize_kernel(const double2 *__restrict__ part,
@@ -310,17 +274,6 @@ cudaError_t launch_split(int kind, const double *state, long M, int K, int Kp, v
 double split_scale(int kind, double spin_len) {
     if (kind != 3 || !(spin_len > 0.0) || !(spin_len < 1e300)) return 1.0;
     return ldexp(1.0, 12 - ilogb(spin_len));
-}
-
-
-
-
-cudaError_t launch_grid_dft(const double *G, int lat_n, double scale, double2 *tmp, double *out,
-                            cudaStream_t st) {
-    const int n = lat_n * lat_n;
-    grid_dft_rows_kernel<<<(n + 127) / 128, 128, 0, st>>>(G, lat_n, tmp);
-    grid_dft_cols_kernel<<<(n + 127) / 128, 128, 0, st>>>(tmp, lat_n, scale, out);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_finalize(const double2 *part, int nparts, double scale, double *out,
