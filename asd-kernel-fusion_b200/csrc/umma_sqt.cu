@@ -16,12 +16,10 @@
 // Roles (one CTA per SM, persistent over 128 x 256 tiles):
 //   warp 0      TMA producer (one thread): 4 tiles per k block (Ah, Al, Bh, Bl)
 //   warp 1      MMA issuer (one thread): 3 x 4 tcgen05.mma per k block
-//   warps 2..   epilogue: TMEM -> registers, phase/outer/reduction.  Eight
+//   warps 2..9  epilogue: TMEM -> registers, phase/outer/reduction.  Eight
 //               warps (two per TMEM lane quarter, each taking half of the
-//               tile's columns) for the phase epilogue, so that its pass over
-//               an accumulation chunk stays shorter than the chunk's MMAs even
-//               for small chunks; four for the q-grid epilogue, whose
-//               per-warp transposition buffers fill the shared memory.
+//               tile's columns), so that the pass over an accumulation chunk
+//               stays shorter than the chunk's MMAs even for small chunks.
 // TMEM holds two 128 x 256 FP32 accumulators (all 512 columns), so the
 // epilogue of one tile overlaps the MMAs of the next.
 #include <cuda.h>
@@ -37,22 +35,23 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BN = 256;
-// Epilogue warps of each epilogue kind (EPI_GRID: 4, the others 8) and the
-// CTA's threads: the TMA and MMA warps plus those.
-__host__ __device__ constexpr int epi_warps(int epi) { return epi == 2 ? 4 : 8; }
-__host__ __device__ constexpr int cta_threads(int epi) { return 64 + 32 * epi_warps(epi); }
-constexpr int MAX_EPI_WARPS = 8;
+// Epilogue warps, and the CTA's threads: the TMA and MMA warps plus those.
+constexpr int EW = 8;
+constexpr int CTA_THREADS = 64 + 32 * EW;
 constexpr int TMEM_COLS = 512;
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 // Row tiles per raster group.  Measured on B200 at 128x128x500 and
 // 256x256x1000: groups of 16 keep the DRAM traffic lowest (the group's A
 // bands, 24-48 MB, stay in L2 while B streams past once per group).
 constexpr int GROUP_M = 16;
-// q grid: per warp, a 32 x 32 transposition buffer (FP32) while a tile is
-// binned, then the warp's tile-diagonal partials (9 x 32 x 2 FP64) when it is
-// combined; the two uses alternate, so they share one region.
-constexpr int GRID_DIAG_M = 9;  // diagonals per lane and warp: 32 m + lane, 9 values of m
-constexpr int GRID_SCRATCH_BYTES = 4 * GRID_DIAG_M * 32 * 2 * 8;  // >= 4 * 32 * 32 * 4
+// q grid: per warp, a transposition buffer for half a block (32 rows x 16
+// columns FP32, row stride 17) while a tile is binned, then the warp's
+// tile-diagonal partials (5 x 32 x 2 FP64) when it is combined; the two uses
+// alternate, so they share one region.
+constexpr int GRID_DIAG_M = 5;  // diagonals per lane and warp: 32 m + lane, 5 values of m
+constexpr int GRID_XPOSE = 32 * 17;
+constexpr int GRID_SCRATCH_BYTES = EW * GRID_DIAG_M * 32 * 2 * 8;
+static_assert(GRID_SCRATCH_BYTES >= EW * GRID_XPOSE * 4, "the transposition buffers fit");
 constexpr int GRID_ND = BM + BN - 1;  // diagonals r - c of a 128 x 256 tile
 
 // Pipeline geometry: 128 bytes of K per operand row per stage (the 128-byte
@@ -80,7 +79,7 @@ struct SmemTail {
     uint64_t ebar;  // epilogue warps' barrier
     uint32_t tmem_base;
     int abort_flag;
-    double red[2][MAX_EPI_WARPS];
+    double red[2][EW];
 };
 
 constexpr int smem_bytes() {
@@ -142,54 +141,42 @@ __device__ __forceinline__ uint32_t grid_below_mask(int x0, int thr, int N) {
     return m;
 }
 
-// val added to exactly one of the four sums, chosen by (b, c): predicated
-// adds, so no lane branches and each sum sees its values in step order.
+// val added to the sums whose mask has the step's bit set (one of the four):
+// predicated adds, so no lane branches and each sum sees its values in step
+// order.
 __device__ __forceinline__ void grid_add4(float &pa0, float &pa1, float &pb0, float &pb1,
-                                          float val, uint32_t b, uint32_t c) {
-    asm("{\n\t.reg .pred pb, q0, q1, q2, q3;\n\t"
-        "setp.ne.u32 pb, %5, 0;\n\t"
-        "setp.eq.and.u32 q0, %6, 0, !pb;\n\t"
-        "setp.ne.and.u32 q1, %6, 0, !pb;\n\t"
-        "setp.eq.and.u32 q2, %6, 0, pb;\n\t"
-        "setp.ne.and.u32 q3, %6, 0, pb;\n\t"
+                                          float val, uint32_t a0, uint32_t a1, uint32_t b0,
+                                          uint32_t b1) {
+    asm("{\n\t.reg .pred q0, q1, q2, q3;\n\t"
+        "setp.ne.u32 q0, %5, 0;\n\t"
+        "setp.ne.u32 q1, %6, 0;\n\t"
+        "setp.ne.u32 q2, %7, 0;\n\t"
+        "setp.ne.u32 q3, %8, 0;\n\t"
         "@q0 add.rn.f32 %0, %0, %4;\n\t"
         "@q1 add.rn.f32 %1, %1, %4;\n\t"
         "@q2 add.rn.f32 %2, %2, %4;\n\t"
         "@q3 add.rn.f32 %3, %3, %4;\n\t}"
         : "+f"(pa0), "+f"(pa1), "+f"(pb0), "+f"(pb1)
-        : "f"(val), "r"(b), "r"(c));
+        : "f"(val), "r"(a0), "r"(a1), "r"(b0), "r"(b1));
 }
 
 // q grid: one 32 x 32 block (column group c) of a warp's accumulator rows.
 // Lane l holds v[jj] = acc(row 32 q + l, column 32 c + jj).  The block's
 // diagonals are lambda = l - jj in [-31, 31]; lane L owns lambda = L (tile
-// diagonal 32 (q - c) + L, register gd[8 - c]) and lambda = L - 32 (tile
-// diagonal 32 (q - c - 1) + L, gd[7 - c]).  Lane l writes v[jj] to row
-// (l - jj) mod 32, column l of the warp's buffer; lane L then reads its row,
-// from column L onwards (conflict-free both ways): step s reads column
-// l = (L + s) mod 32, which is on lambda = L - 32 iff s >= 32 - L.  The class
-// of a step (class 0 iff the row's lattice column x >= a, a = (i - j) mod N
-// of the diagonal) comes from two 32-bit masks formed once per block, so a
-// step is a shared load and one predicated add to one of four sums.
+// diagonal 32 (q - c) + L, sums ga) and lambda = L - 32 (tile diagonal
+// 32 (q - c - 1) + L, sums gb).  In two halves of 16 columns: lane l writes
+// v[jj] to row (l - jj) mod 32, place jj mod 16 of the warp's buffer (rows of
+// 17: conflict-free); lane L then reads its row, so step s = jj is the element of
+// lattice row (L + s) mod 32, on lambda = L - 32 iff s >= 32 - L.  The class of a
+// step (class 0 iff the row's lattice column x >= a, a = (i - j) mod N of the
+// diagonal) and the diagonal choose one of four sums through four 32-bit masks
+// formed once per block, so a step is a shared load at a fixed offset and one
+// predicated add.
 __device__ __forceinline__ void grid_block(const uint32_t (&v)[32], int c, int lane,
                                            const float4 &r4, const float4 *z_tab, float alpha,
                                            bool last, int x_row, int a_first, int N, float *xp,
-                                           double (&gd)[9][2]) {
+                                           double (&ga)[2], double (&gb)[2]) {
     const float4 *zq = z_tab + c * 32;
-    const int wbase = lane * 33;  // row (lane - jj) mod 32, column lane: (wbase - 32 jj) mod 1024
-#pragma unroll
-    for (int jj = 0; jj < 32; ++jj) {
-        float val = alpha * __uint_as_float(v[jj]);
-        if (last) {
-            const float4 z = zq[jj];
-            float o = r4.x * z.x;
-            o = fmaf(r4.y, z.y, o);
-            o = fmaf(r4.z, z.z, o);
-            val -= o;
-        }
-        xp[(wbase - 32 * jj) & 1023] = val;
-    }
-    __syncwarp();
     // diagonal lambda = L of block c: i - j shifted by -32 c from block 0
     int aa = (a_first - ((32 * c) % N)) % N;
     if (aa < 0) aa += N;
@@ -200,22 +187,39 @@ __device__ __forceinline__ void grid_block(const uint32_t (&v)[32], int c, int l
     // rotated right by L so that bit s is the row read at step s
     const uint32_t lowL = (1u << lane) - 1u;
     const uint32_t cm = (grid_below_mask(x0, aa, N) & ~lowL) | (grid_below_mask(x0, ab, N) & lowL);
-    uint32_t cbits = __funnelshift_r(cm, cm, lane);
-    uint32_t bbits = __funnelshift_r(lowL, lowL, lane);  // steps on lambda = L - 32
-    const float *row = xp + lane * 32;
+    const uint32_t cbits = __funnelshift_r(cm, cm, lane);
+    const uint32_t bbits = __funnelshift_r(lowL, lowL, lane);  // steps on lambda = L - 32
+    const uint32_t ma0 = ~bbits & ~cbits, ma1 = ~bbits & cbits, mb0 = bbits & ~cbits,
+                   mb1 = bbits & cbits;
+    float *const wlo = xp + lane * 17, *const whi = wlo + 32 * 17;  // rows l - jj, l - jj + 32
+    const float *const row = xp + lane * 17;
     float pa0 = 0.f, pa1 = 0.f, pb0 = 0.f, pb1 = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < 32; ++s) {
-        const float val = row[(lane + s) & 31];
-        grid_add4(pa0, pa1, pb0, pb1, val, bbits & 1u, cbits & 1u);
-        bbits >>= 1;
-        cbits >>= 1;
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+#pragma unroll
+        for (int jj = h; jj < h + 16; ++jj) {
+            float val = alpha * __uint_as_float(v[jj]);
+            if (last) {
+                const float4 z = zq[jj];
+                float o = r4.x * z.x;
+                o = fmaf(r4.y, z.y, o);
+                o = fmaf(r4.z, z.z, o);
+                val -= o;
+            }
+            float *const w = jj > lane ? whi : wlo;
+            w[(jj - h) - 17 * jj] = val;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int s = h; s < h + 16; ++s)
+            grid_add4(pa0, pa1, pb0, pb1, row[s - h], ma0 & (1u << s), ma1 & (1u << s),
+                      mb0 & (1u << s), mb1 & (1u << s));
+        __syncwarp();  // the buffer is free for the next half
     }
-    __syncwarp();  // the buffer is free for the next block
-    gd[8 - c][0] += (double)pa0;
-    gd[8 - c][1] += (double)pa1;
-    gd[7 - c][0] += (double)pb0;  // zero in lane 0, which has no lambda = -32
-    gd[7 - c][1] += (double)pb1;
+    ga[0] += (double)pa0;
+    ga[1] += (double)pa1;
+    gb[0] += (double)pb0;  // zero in lane 0, which has no lambda = -32
+    gb[1] += (double)pb1;
 }
 
 // KIND: 1 = TF32x3, 2 = BF16x3, 3 = FP16x3.  EPI selects the epilogue:
@@ -226,17 +230,15 @@ __device__ __forceinline__ void grid_block(const uint32_t (&v)[32], int c, int l
 //              the lattice column of j wraps (class 0: col(j) <= col(i)),
 //              into tdiag[mb][nb][d + BN - 1][class] (qgrid.cu bins them).
 //              Each epilogue lane owns the diagonals d = 32 m + lane of its
-//              warp's 32 rows: a 32 x 32 block of the accumulator goes
-//              through shared memory transposed along its diagonals (lane l
-//              writes its value of column jj to row (l - jj) mod 32), each
-//              lane sums its two diagonals of the block in a fixed order
-//              (FP32, at most 32 terms) into FP64 registers, and the four
-//              warps' registers are combined per tile in warp order.  No
-//              atomics: the bins repeat bit for bit.
+//              warp's 32 rows and 128 columns: a 32 x 32 block of the
+//              accumulator goes through shared memory transposed along its
+//              diagonals, each lane sums its two diagonals of the block in a
+//              fixed order (FP32, at most 32 terms) into FP64 registers, and
+//              the eight warps' registers are combined per tile in warp order.
+//              No atomics: the bins repeat bit for bit.
 constexpr int EPI_PHASE = 0, EPI_STORE = 1, EPI_GRID = 2;
-static_assert(epi_warps(EPI_GRID) == 4 && epi_warps(EPI_PHASE) == MAX_EPI_WARPS, "warp counts");
 template <int KIND, int EPI>
-__global__ void __launch_bounds__(cta_threads(EPI), 1)
+__global__ void __launch_bounds__(CTA_THREADS, 1)
     umma_sqt_kernel(const __grid_constant__ CUtensorMap tm_ah,
                     const __grid_constant__ CUtensorMap tm_al,
                     const __grid_constant__ CUtensorMap tm_bh,
@@ -248,7 +250,6 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
                     int lat_n, double *__restrict__ tdiag, int group_m) {
     using G = Geo;
     constexpr bool STORE = (EPI == EPI_STORE);
-    constexpr int EW = epi_warps(EPI);         // epilogue warps
     constexpr int NHALF = EW / 4;              // warps per TMEM lane quarter
     constexpr int GPH = BN / 32 / NHALF;       // 32-column groups per warp
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -417,9 +418,9 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
             if (i >= WAIT_LIMIT && status) atomicOr(status, (unsigned)kStatusTimeout);
         }
     } else {
-        // Epilogue warps 2.. own TMEM lane quarters (warp % 4) * 32; with
-        // eight, warps 2..5 take the column groups [0, 4) and warps 6..9
-        // the groups [4, 8) of every chunk.
+        // Epilogue warps 2..9 own TMEM lane quarters (warp % 4) * 32; warps
+        // 2..5 take the column groups [0, 4) and warps 6..9 the groups [4, 8)
+        // of every chunk.
         const int quarter = warp & 3;
         const int rloc = quarter * 32 + lane;
         const int etid = threadIdx.x - 64;  // 0 .. 32 EW - 1 among the epilogue threads
@@ -429,8 +430,8 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
         double tot_re = 0.0, tot_im = 0.0;
         int tcount = 0;
         uint32_t ephase = 0;
-        float *xpose = reinterpret_cast<float *>(gscr) + quarter * 32 * 32;  // [32][32]
-        double *wdiag = reinterpret_cast<double *>(gscr);                       // [4][9][32][2]
+        float *xpose = reinterpret_cast<float *>(gscr) + (warp - 2) * GRID_XPOSE;
+        double *wdiag = reinterpret_cast<double *>(gscr);  // [EW][5][32][2]
         for (long tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcount) {
             int mb, nb;
             tile_coords(tile, num_m, num_n, group_m, mb, nb);
@@ -459,9 +460,9 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
             const float ui = STORE ? 0.f : row1[i];
             double s_re = 0.0, s_im = 0.0;
             bool ok = true;
-            // q grid: this lane's diagonals d = 32 (quarter - 8 + mm) + lane of
-            // the tile, both classes; the column of its own row's site;
-            // the columns a = (i - j) mod N of its first block's two diagonals.
+            // q grid: this lane's diagonals d = 32 (quarter - c_first - 4 + mm)
+            // + lane of the tile, both classes; the column of its own row's
+            // site; the columns a = (i - j) mod N of block 0's two diagonals.
             double gd[GRID_DIAG_M][2];
             int x_row = 0, a_first = 0;
             if (EPI == EPI_GRID) {
@@ -487,11 +488,11 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
                 // Per 32-column group, in FP32: a = sum_j w_j acc_ij and, in the
                 // last chunk only, o = sum_j w_j (m_i . z_j); the row sum
                 // s_i = alpha * a - o is carried in FP64.  (The q grid unrolls
-                // the groups: its per-lane diagonal registers are indexed by c.)
-                constexpr int CU = (EPI == EPI_GRID) ? BN / 32 : 1;
+                // the groups: its per-lane diagonal registers are indexed by cc.)
+                constexpr int CU = (EPI == EPI_GRID) ? GPH : 1;
 #pragma unroll CU
                 for (int cc = 0; cc < GPH; ++cc) {
-                    const int c = (EPI == EPI_GRID) ? cc : c_first + cc;  // a constant for the grid
+                    const int c = c_first + cc;
                     uint32_t v[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                            (uint32_t)(abuf * BN + c * 32);
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
                     }
                     if (EPI == EPI_GRID) {
                         grid_block(v, c, lane, r4, z_tab, alpha, last, x_row, a_first, lat_n,
-                                   xpose, gd);
+                                   xpose, gd[GPH - cc], gd[GPH - 1 - cc]);
                         continue;
                     }
                     const float4 *wq = reinterpret_cast<const float4 *>(w_tab + c * 32);
@@ -549,13 +550,13 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
             }
             if (!ok) break;
             if (EPI == EPI_GRID) {
-                // the four warps' diagonals -> tdiag[tile], in warp order; the
+                // the warps' diagonals -> tdiag[tile], in warp order; the
                 // shared region served as transposition buffers until now
                 if (!epilogue_sync(&tail->ebar, ephase, abort_flag)) {
                     raise_abort(tail, status);
                     break;
                 }
-                double *wq = wdiag + quarter * (GRID_DIAG_M * 32 * 2);
+                double *wq = wdiag + (warp - 2) * (GRID_DIAG_M * 32 * 2);
 #pragma unroll
                 for (int mm = 0; mm < GRID_DIAG_M; ++mm) {
                     wq[(mm * 32 + lane) * 2] = gd[mm][0];
@@ -571,8 +572,9 @@ __global__ void __launch_bounds__(cta_threads(EPI), 1)
                     const int L = (d + 256) & 31, m = (d - L) / 32;
                     double sum = 0.0;
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const int mm = m - w + 8;
+                    for (int w = 0; w < EW; ++w) {
+                        // warp 2 + w: quarter (2 + w) % 4, column half w / 4
+                        const int mm = m - ((2 + w) & 3) + (w / 4) * GPH + GPH;
                         if (mm >= 0 && mm < GRID_DIAG_M)
                             sum += wdiag[((w * GRID_DIAG_M + mm) * 32 + L) * 2 + cls];
                     }
@@ -704,7 +706,7 @@ int launch_umma_sqt(const UmmaSqtArgs &a, cudaStream_t st) {
         cudaError_t r =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (r != cudaSuccess) return r;
-        kern<<<grid, cta_threads(epi), smem, st>>>(tah, tal, tbh, tbl, num_m, num_n, kb_begin, kb_end,
+        kern<<<grid, CTA_THREADS, smem, st>>>(tah, tal, tbh, tbl, num_m, num_n, kb_begin, kb_end,
                                               kpc, a.outer, a.row4, a.row1, a.col4, a.col1,
                                               a.alpha, a.part, a.status, a.dbg_c, a.dbg_ldc,
                                               a.lat_n, a.tdiag, GROUP_M);
