@@ -16,13 +16,15 @@
 // in the context's RK4 scratch (no memory of their own):
 //   qfft_rows_kernel  a block takes one lattice row of KC columns, transforms
 //                     along it in shared memory, writes X[r][b][columns]
-//   qfft_cols_kernel  a block takes the lattice columns b and N - b of KC
-//                     columns k, transforms both, forms the product above for
-//                     every a and adds it to its slice's sums over k
+//   qfft_cols_kernel  a block takes the lattice columns b and N - b of up to
+//                     KC columns k, transforms both side by side, forms the
+//                     product above for every a and adds it to its slice's
+//                     sums over k
 //   qfft_sum_kernel   sums the slices, scales, writes q and -q (conjugates)
-// Both passes hold KC = 8 columns k side by side (16 bytes each), so that eight
-// neighbouring threads touch one 128-byte line in global and in shared memory
-// whatever the stride along the lattice: no bank conflicts for any radix.
+// Both passes hold eight or more lines side by side (16 bytes each), so that
+// eight neighbouring threads touch one 128-byte line in shared memory (and, KC
+// = 8, in global memory) whatever the stride along the lattice: no bank
+// conflicts for any radix.
 // Stockham stages of radix 8, 4, 2, 3, 5 in registers; any other prime factor p
 // as p-term sums from the twiddle table, so every N works.  Fixed order of
 // summation everywhere: the grid repeats bit for bit.  The split modes' N x N
@@ -31,7 +33,7 @@
 // Bound by shared-memory traffic (each stage reads and writes 16 bytes a point)
 // and, below about 64 x 64, by launch latency.  Measured on B200 against the FP64
 // tensor-core GEMM with diagonal sums that served this before: 256x256x1000 831
-// -> 7.03 ms, 128x128x500 26.9 -> 0.725 ms, 32x32x200 0.145 -> 0.041 ms.
+// -> 6.61 ms, 128x128x500 26.9 -> 0.80 ms, 32x32x200 0.145 -> 0.031 ms.
 #include "asd_internal.h"
 
 namespace asd {
@@ -39,12 +41,14 @@ namespace {
 
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_THREADS = 256;
+constexpr int MAX_SHARED_TW = 2048;  // column pass: longer twiddle tables stay in L2
 
 struct FftPlan {
     int n;
     int stages;
     int radix[MAX_STAGES];
-    int lk;  // log2 of the columns k held side by side
+    int lk;   // log2 of the columns k held side by side, KC
+    int lkc;  // the same in the column pass (of each of its two lines)
 };
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
@@ -161,16 +165,16 @@ __device__ __forceinline__ void stage_any(const double2 *in, double2 *out, const
 // Transforms `a` (n points x 2^lk columns); b is the other buffer.  Returns the
 // one that holds the result; every thread is past its last write.
 __device__ __forceinline__ double2 *transform(double2 *a, double2 *b, const double2 *tw,
-                                              const FftPlan &p) {
+                                              const FftPlan &p, int lk) {
     int Ns = 1;
     for (int s = 0; s < p.stages; ++s) {
         const int r = p.radix[s];
-        if (r == 8) stage<8>(a, b, tw, p.n, Ns, p.lk);
-        else if (r == 4) stage<4>(a, b, tw, p.n, Ns, p.lk);
-        else if (r == 2) stage<2>(a, b, tw, p.n, Ns, p.lk);
-        else if (r == 3) stage<3>(a, b, tw, p.n, Ns, p.lk);
-        else if (r == 5) stage<5>(a, b, tw, p.n, Ns, p.lk);
-        else stage_any(a, b, tw, p.n, r, Ns, p.lk);
+        if (r == 8) stage<8>(a, b, tw, p.n, Ns, lk);
+        else if (r == 4) stage<4>(a, b, tw, p.n, Ns, lk);
+        else if (r == 2) stage<2>(a, b, tw, p.n, Ns, lk);
+        else if (r == 3) stage<3>(a, b, tw, p.n, Ns, lk);
+        else if (r == 5) stage<5>(a, b, tw, p.n, Ns, lk);
+        else stage_any(a, b, tw, p.n, r, Ns, lk);
         Ns *= r;
         double2 *t = a;
         a = b;
@@ -193,10 +197,11 @@ __global__ void qfft_twiddle_kernel(int n, double2 *__restrict__ tw) {
 struct Chunk {
     double2 *buf[3];
     int blocks, per;
-    __device__ __forceinline__ double2 *at(int kb, int lk, int &width) const {
-        const int q = kb / per, first = q * per;
+    // column k of the chunk
+    __device__ __forceinline__ double2 *at(int k, int lk, int &width) const {
+        const int q = (k >> lk) / per, first = q * per;
         width = min(per, blocks - first) << lk;
-        return buf[q] + ((kb - first) << lk);
+        return buf[q] + (k - (first << lk));
     }
 };
 
@@ -222,9 +227,9 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
         b0[idx] = v;
     }
     __syncthreads();
-    const double2 *f = transform(b0, b1, stw, p);
+    const double2 *f = transform(b0, b1, stw, p, p.lk);
     int kw;
-    double2 *o = X.at(blockIdx.x, p.lk, kw);
+    double2 *o = X.at(kl, p.lk, kw);
     o += r * n * kw;
     for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x)
         o[(long)(idx >> p.lk) * kw + (idx & (kc - 1))] = f[idx];
@@ -235,38 +240,33 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
 __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
     FftPlan p, Chunk X, const double2 *__restrict__ tw, int add, double2 *__restrict__ part) {
     extern __shared__ __align__(16) double2 fsm[];
-    const int n = p.n, kc = 1 << p.lk, len = n << p.lk;
-    double2 *b0 = fsm, *b1 = b0 + len, *b2 = b1 + len, *stw = b2 + len, *sum = stw + n;
+    const int n = p.n, kc = 1 << p.lkc, lt = p.lkc + 1, len = n << p.lkc;
+    double2 *b0 = fsm, *b1 = b0 + (n << lt), *sum = b1 + (n << lt), *stw = sum + n;
     const int b = blockIdx.x, mb = (b == 0) ? 0 : n - b;
+    const bool copy_tw = n <= MAX_SHARED_TW;
     for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        stw[j] = tw[j];
+        if (copy_tw) stw[j] = tw[j];
         sum[j] = make_double2(0.0, 0.0);
     }
-    for (int kb = blockIdx.y; kb < X.blocks; kb += gridDim.y) {
+    const int nkb = X.blocks << (p.lk - p.lkc);
+    for (int kb = blockIdx.y; kb < nkb; kb += gridDim.y) {
         int kw;
-        const double2 *x = X.at(kb, p.lk, kw);
-        auto load = [&](double2 *dst, int col) {
-            const double2 *src = x + (long)col * kw;
-            for (int idx = threadIdx.x; idx < len; idx += blockDim.x)
-                dst[idx] = src[(long)(idx >> p.lk) * n * kw + (idx & (kc - 1))];
-        };
+        const double2 *x = X.at(kb << p.lkc, p.lk, kw);
         __syncthreads();  // the previous block's products are formed
-        load(b0, b);
-        __syncthreads();
-        const double2 *Z = transform(b0, b1, stw, p), *W = Z;
-        if (mb != b) {
-            double2 *other = (Z == b0) ? b1 : b0;
-            load(b2, mb);
-            __syncthreads();
-            W = transform(b2, other, stw, p);
+        // line b in columns 0 .. kc - 1, line n - b in kc .. 2 kc - 1
+        for (int idx = threadIdx.x; idx < (n << lt); idx += blockDim.x) {
+            const int r = idx >> lt, j = idx & (2 * kc - 1);
+            b0[idx] = x[((long)r * n + (j < kc ? b : mb)) * kw + (j & (kc - 1))];
         }
+        __syncthreads();
+        const double2 *Z = transform(b0, b1, copy_tw ? stw : tw, p, lt);
         // whole warps: len is a multiple of kc, lanes of one a stay together
         for (int i0 = 0; i0 < len; i0 += blockDim.x) {
-            const int idx = i0 + threadIdx.x, a = idx >> p.lk;
+            const int idx = i0 + threadIdx.x, a = idx >> p.lkc, k = idx & (kc - 1);
             double re = 0.0, im = 0.0;
             if (idx < len) {
                 const int ma = (a == 0) ? 0 : n - a;
-                const double2 zv = Z[idx], w = W[(ma << p.lk) + (idx & (kc - 1))];
+                const double2 zv = Z[(a << lt) + k], w = Z[(ma << lt) + kc + k];
                 re = 0.5 * (zv.x * w.y + zv.y * w.x);
                 im = 0.25 * ((zv.x - w.x) * (zv.x + w.x) + (zv.y - w.y) * (zv.y + w.y));
             }
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
                 re += __shfl_xor_sync(0xffffffffu, re, o);
                 im += __shfl_xor_sync(0xffffffffu, im, o);
             }
-            if (idx < len && (idx & (kc - 1)) == 0) {
+            if (idx < len && k == 0) {
                 sum[a].x += re;
                 sum[a].y += im;
             }
@@ -289,16 +289,25 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
     }
 }
 
+// 16 frequencies a block, eight threads each: thread s adds slices s, s + 8, ...
 __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict__ part, int n,
                                                        int slices, double scale,
                                                        double2 *__restrict__ out) {
-    const long t = (long)blockIdx.x * 128 + threadIdx.x;
+    __shared__ double2 red[8][16];
+    const int tl = threadIdx.x & 15, sl = threadIdx.x >> 4;
+    const long t = (long)blockIdx.x * 16 + tl;
     const long half = (long)n * (n / 2 + 1);
-    if (t >= half) return;
-    const int b = (int)(t / n), a = (int)(t - (long)b * n);
     double2 s = make_double2(0.0, 0.0);
+    if (t < half) {
 #pragma unroll 4
-    for (int q = 0; q < slices; ++q) s = cadd(s, part[q * half + t]);
+        for (int q = sl; q < slices; q += 8) s = cadd(s, part[q * half + t]);
+    }
+    red[sl][tl] = s;
+    __syncthreads();
+    if (sl != 0 || t >= half) return;
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s = cadd(s, red[q][tl]);
+    const int b = (int)(t / n), a = (int)(t - (long)b * n);
     s.x *= scale;
     s.y *= scale;
     out[(long)a * n + b] = s;
@@ -332,7 +341,7 @@ __global__ void __launch_bounds__(MAX_THREADS) bins_dft_kernel(FftPlan p,
         b0[idx] = v;
     }
     __syncthreads();
-    const double2 *f = transform(b0, b1, stw, p);
+    const double2 *f = transform(b0, b1, stw, p, p.lk);
     for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x) {
         const int line = l0 + (idx & (kc - 1));
         if (line < n)
@@ -356,20 +365,25 @@ FftPlan make_plan(int n, int K) {
     take(3);
     take(5);
     for (int r = 7; m > 1; r += 2) take(r);
-    // Columns side by side: 8, less where three buffers of a line do not fit
-    // an SM or a scratch buffer (K doubles a site) holds no block of them.
+    // Columns side by side: 8, less where the two buffers do not leave room for
+    // a second block on the SM or a scratch buffer (K doubles a site) holds no
+    // block of them; in the column pass two lines lie side by side.
+    auto fits = [&](int lines) { return (size_t)2 * n * lines * sizeof(double2) <= 104 * 1024; };
     p.lk = 3;
-    while (p.lk > 0 && ((size_t)3 * (n << p.lk) * sizeof(double2) > 160 * 1024 || (2 << p.lk) > K))
-        --p.lk;
+    while (p.lk > 0 && (!fits(1 << p.lk) || (2 << p.lk) > K)) --p.lk;
+    p.lkc = p.lk;
+    while (p.lkc > 0 && !fits(2 << p.lkc)) --p.lkc;
     return p;
 }
 
 size_t rows_smem(const FftPlan &p) { return ((size_t)2 * (p.n << p.lk) + p.n) * sizeof(double2); }
-size_t cols_smem(const FftPlan &p) { return ((size_t)3 * (p.n << p.lk) + 2 * p.n) * sizeof(double2); }
+size_t cols_smem(const FftPlan &p) {
+    return ((size_t)4 * (p.n << p.lkc) + (p.n <= MAX_SHARED_TW ? 2 : 1) * p.n) * sizeof(double2);
+}
 
 // Threads of a block: one per four points, whole warps, 64 to 256.
-int threads_for(const FftPlan &p) {
-    const int t = ((p.n << p.lk) / 4 + 31) / 32 * 32;
+int threads_for(int points) {
+    const int t = (points / 4 + 31) / 32 * 32;
     return t < 64 ? 64 : (t > MAX_THREADS ? MAX_THREADS : t);
 }
 
@@ -387,9 +401,9 @@ Geometry geometry(const FftPlan &p, int K) {
     if (b < 1) b = 1;
     if (b > 3L * g.per) b = 3L * g.per;
     g.blocks = b < all ? (int)b : all;
-    const int lines = p.n / 2 + 1;
+    const int lines = p.n / 2 + 1, nkb = g.blocks << (p.lk - p.lkc);
     g.slices = (8 * 148 + lines - 1) / lines;  // about eight blocks per SM
-    if (g.slices > g.blocks) g.slices = g.blocks;
+    if (g.slices > nkb) g.slices = nkb;
     return g;
 }
 
@@ -411,7 +425,8 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
     const FftPlan p = make_plan(lat_n, K);
     const Geometry g = geometry(p, K);
     double2 *tw = static_cast<double2 *>(work), *part = tw + lat_n;
-    const int threads = threads_for(p), kc = 1 << p.lk, all = (K + kc - 1) / kc;
+    const int rows_t = threads_for(p.n << p.lk), cols_t = threads_for(p.n << (p.lkc + 1));
+    const int kc = 1 << p.lk, all = (K + kc - 1) / kc;
     ASD_CUDA_TRY(cudaFuncSetAttribute(qfft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)rows_smem(p)));
     ASD_CUDA_TRY(cudaFuncSetAttribute(qfft_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -422,16 +437,16 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
         for (int q = 0; q < 3; ++q) X.buf[q] = reinterpret_cast<double2 *>(scratch[q]);
         X.blocks = all - b0 < g.blocks ? all - b0 : g.blocks;
         X.per = g.per;
-        qfft_rows_kernel<<<dim3((unsigned)X.blocks, (unsigned)lat_n), threads, rows_smem(p), st>>>(
+        qfft_rows_kernel<<<dim3((unsigned)X.blocks, (unsigned)lat_n), rows_t, rows_smem(p), st>>>(
             p, A, B, K, b0 * kc, X, m, z, tw);
         // a last, shorter chunk still visits every slice (with no block it adds zero)
-        qfft_cols_kernel<<<dim3((unsigned)(lat_n / 2 + 1), (unsigned)g.slices), threads,
+        qfft_cols_kernel<<<dim3((unsigned)(lat_n / 2 + 1), (unsigned)g.slices), cols_t,
                            cols_smem(p), st>>>(p, X, tw, b0 > 0, part);
         ASD_CUDA_TRY(cudaGetLastError());
         launches += 2;
     }
     const long half = (long)lat_n * (lat_n / 2 + 1);
-    qfft_sum_kernel<<<(unsigned)((half + 127) / 128), 128, 0, st>>>(
+    qfft_sum_kernel<<<(unsigned)((half + 15) / 16), 128, 0, st>>>(
         part, lat_n, g.slices, scale, reinterpret_cast<double2 *>(out));
     ASD_CUDA_TRY(cudaGetLastError());
     return launches + 1;
@@ -440,7 +455,7 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
 cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const double2 *tw, double2 *T,
                             double *out, cudaStream_t st) {
     const FftPlan p = make_plan(lat_n, 16);
-    const int kc = 1 << p.lk, blocks = (lat_n + kc - 1) / kc, threads = threads_for(p);
+    const int kc = 1 << p.lk, blocks = (lat_n + kc - 1) / kc, threads = threads_for(p.n << p.lk);
     const size_t smem = rows_smem(p);
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(bins_dft_kernel<true>,

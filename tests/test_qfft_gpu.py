@@ -24,7 +24,8 @@ def numpy_grid(N, nf, st, s0):
 
 @pytest.mark.parametrize("N,nfile", [(3, 2), (4, 5), (5, 3), (7, 8), (8, 11), (13, 3), (16, 86),
                                      (30, 4), (49, 2), (51, 7), (64, 9), (67, 3), (96, 5), (121, 2),
-                                     (125, 3), (128, 40), (256, 3), (600, 2), (601, 2), (1024, 2)])
+                                     (125, 3), (128, 40), (256, 3), (600, 2), (601, 2), (1024, 2),
+                                     (2432, 1)])
 def test_fp64_grid_over_the_transform_paths(N, nfile):
     s0 = asd.random_spins(N, nfile, seed=11 * N + nfile)
     with asd.Context(asd.Params.make(N, nfile, J1=1.0, alpha=0.1, dt=0.01), modes=["fp64"]) as ctx:
