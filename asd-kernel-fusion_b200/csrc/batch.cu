@@ -62,6 +62,20 @@ struct F3 {
     float x, y, z;
 };
 
+// fdiv_const of the three components with one range test for all of them.
+__device__ __forceinline__ F3 fdiv3_const(const F3 &v, float d, float c) {
+    const float ax = fabsf(v.x), ay = fabsf(v.y), az = fabsf(v.z);
+    const float lo = fminf(ax, fminf(ay, az)), hi = fmaxf(ax, fmaxf(ay, az));
+    if (!(lo >= 0x1p-100f && hi <= 0x1p100f))
+        return F3{__fdiv_rn(v.x, d), __fdiv_rn(v.y, d), __fdiv_rn(v.z, d)};
+    auto one = [&](float x) {
+        const float q = __fmul_rn(x, c);
+        const float t = __fmaf_rn(q, d, -x);
+        return __fmaf_rn(-t, c, q);
+    };
+    return F3{one(v.x), one(v.y), one(v.z)};
+}
+
 // Reads that follow a grid barrier must not hit stale L1 lines: L2 only.
 __device__ __forceinline__ F3 ld3(const float *p, long M, long i) {
     return F3{__ldcg(p + i), __ldcg(p + M + i), __ldcg(p + 2 * M + i)};
@@ -70,16 +84,23 @@ __device__ __forceinline__ F3 ld3(const float *p, long M, long i) {
 // dS/dt from the centre s and the neighbours nb (nearest, in the reference's
 // order (row+1), (row-1), (col-1), (col+1)) and n2 (diagonals (+1,+1),
 // (+1,-1), (-1,+1), (-1,-1); read only with J2), FP32, explicitly rounded.
-// Both batch kernels go through this function: one operation order.
-template <bool J2, bool H, bool DAMP>
+// Both batch kernels go through this function: one operation order.  UNIT, for
+// |J1| = 1: J1 applied once to the sum of the neighbours, the same bits (as
+// llg_rhs_vals in llg_math.cuh).
+template <bool J2, bool H, bool DAMP, bool UNIT = false>
 __device__ __forceinline__ F3 rhs32_vals_t(const F3 &s, const F3 (&nb)[4], const F3 (&n2)[4],
                                            const BatchLattice &L) {
     float ex = 0.f, ey = 0.f, ez = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        ex = fa(ex, fm(nb[j].x, L.J1));
-        ey = fa(ey, fm(nb[j].y, L.J1));
-        ez = fa(ez, fm(nb[j].z, L.J1));
+        ex = fa(ex, UNIT ? nb[j].x : fm(nb[j].x, L.J1));
+        ey = fa(ey, UNIT ? nb[j].y : fm(nb[j].y, L.J1));
+        ez = fa(ez, UNIT ? nb[j].z : fm(nb[j].z, L.J1));
+    }
+    if (UNIT) {
+        ex = __fmaf_rn(ex, L.J1, 0.f);
+        ey = __fmaf_rn(ey, L.J1, 0.f);
+        ez = __fmaf_rn(ez, L.J1, 0.f);
     }
     if (J2) {
 #pragma unroll
@@ -243,18 +264,25 @@ __global__ void __launch_bounds__(256, 4) batch_kernel(const BatchLattice *__res
 // The lattices live in shared memory for the whole run.  Each lattice
 // belongs to one thread-block cluster; its rows are split over the
 // cluster's CTAs (a CTA may hold rows of several lattices, one segment per
-// lattice).  A CTA keeps, as float planes (x, y, z), two stage buffers over
-// its segments' rows plus one halo row above and below each segment (the
-// stencil's inputs, ping-ponged by the four stages: y -> ys1 -> ys2 -> ys3
-// -> y_new), and per site the RK4 base value and the running combination.
-// After every stage the cluster synchronises (a hardware cluster barrier,
-// the same control flow in every CTA) and each CTA copies its segments' two
-// halo rows from the owning CTAs' shared memory (distributed shared memory),
-// then synchronises its own threads.  Threads walk each segment row by row
-// (thread t takes column t % N of rows t / N, t / N + T / N, ...), so a
-// lattice's parameters and a site's column and wrap offsets are uniform or
-// fixed per segment.  No grid-wide barrier and no global-memory traffic
-// between the first load and the final store.
+// lattice).  A CTA keeps two stage buffers over its segments' rows plus one
+// halo row above and below each segment (the stencil's inputs, ping-ponged by
+// the four stages: y -> ys1 -> ys2 -> ys3 -> y_new), and per site the RK4 base
+// value and the running combination; a slot's three components lie together,
+// so a neighbour is one address with three fixed offsets, free of bank
+// conflicts.  A thread owns a strip of consecutive rows of one column of a
+// segment and walks down it with the two rows above in registers (9 shared
+// loads a site and stage instead of 15; 21 instead of 27 with J2).  The
+// segment's first and last row are also stored into the halo rows of the CTAs
+// above and below (distributed shared memory), so one cluster barrier (a
+// hardware barrier, the same control flow in every CTA) ends a stage.  No
+// grid-wide barrier and no global-memory traffic between the first load and the
+// final store.
+//
+// Bound by instruction issue.  Measured on B200, 48 lattices of 48^2..160^2
+// (534 784 sites), autotuned: 28.0 us a step with halo rows fetched after a
+// cluster barrier and a CTA barrier a stage, sites walked row by row and the
+// exchange multiplied per neighbour; 18.8 us as it is (strips unrolled by 2; by 1
+// 19.6, by 3 19.2 with spills).
 struct CSeg {
     int lat;       // lattice
     int N;         // its side
@@ -272,7 +300,7 @@ struct CCta {
 constexpr int CL_THREADS = 896;
 
 __host__ __device__ constexpr size_t cluster_smem_floats(int buf, int sites) {
-    return (size_t)6 * buf + (size_t)6 * sites;  // 2 x 3 planes, y base and combination
+    return (size_t)6 * buf + (size_t)6 * sites;  // two stage buffers, y base and combination
 }
 
 __global__ void __launch_bounds__(CL_THREADS, 1)
@@ -283,128 +311,148 @@ __global__ void __launch_bounds__(CL_THREADS, 1)
     extern __shared__ float cfs[];
     const CCta me = ctas[blockIdx.x];
     const int T = blockDim.x, tid = threadIdx.x, ns = me.nsites;
-    // plane c of stage buffer b: cfs + (3 b + c) * buf; y base [3][ns]; combination [3][ns]
-    auto plane = [&](int b, int c) { return cfs + (3 * b + c) * me.buf; };
+    // stage buffer b: cfs + 3 b buf, slot s at 3 s; y base and combination: 3 a site
     float *const yb = cfs + 6 * (size_t)me.buf;
     float *const ac = yb + 3 * (size_t)ns;
+    const bool alone = cluster.num_blocks() == 1;
+    auto barrier = [&] {
+        if (alone) __syncthreads();
+        else cluster.sync();
+    };
 
+    // every segment's rows and its two halo rows of the initial state
     for (int k = me.seg0; k < me.seg0 + me.nseg; ++k) {
         const CSeg sg = segs[k];
         const long M = (long)sg.N * sg.N;
         const float *Y = y + lats[sg.lat].off;
-        for (int e = tid; e < sg.rows * sg.N; e += T) {
-            const int row = e / sg.N, col = e - row * sg.N;
-            const long i = (long)(sg.r0 + row) * sg.N + col;
-            const int slot = sg.base + (row + 1) * sg.N + col, q = sg.core0 + e;
+        for (int e = tid; e < (sg.rows + 2) * sg.N; e += T) {
+            const int l = e / sg.N, col = e - l * sg.N;
+            int row = sg.r0 - 1 + l;
+            row = row < 0 ? row + sg.N : (row >= sg.N ? row - sg.N : row);
+            const long i = (long)row * sg.N + col;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float v = Y[c * M + i];
-                yb[c * ns + q] = v;
-                plane(0, c)[slot] = v;
+                cfs[3 * (sg.base + e) + c] = v;
+                if (l >= 1 && l <= sg.rows) yb[3 * (sg.core0 + e - sg.N) + c] = v;
             }
         }
     }
-    // halo rows of stage buffer b from the owning CTAs
-    auto halo = [&](int b) {
-        cluster.sync();
-        for (int k = me.seg0; k < me.seg0 + me.nseg; ++k) {
-            const CSeg sg = segs[k];
-            const float *rt = cluster.map_shared_rank(cfs, sg.top_rank) + sg.top_off;
-            const float *rb = cluster.map_shared_rank(cfs, sg.bot_rank) + sg.bot_off;
-            for (int col = tid; col < sg.N; col += T) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    plane(b, c)[sg.base + col] = rt[(3 * b + c) * sg.top_buf + col];
-                    plane(b, c)[sg.base + (sg.rows + 1) * sg.N + col] =
-                        rb[(3 * b + c) * sg.bot_buf + col];
-                }
-            }
-        }
-        __syncthreads();
-    };
-    halo(0);
+    barrier();  // also: every CTA of the cluster has started before one stores into it
 
     auto stage = [&](auto sc) {
         constexpr int S = decltype(sc)::value;
-        const float *ix = plane((S - 1) & 1, 0), *iy = plane((S - 1) & 1, 1),
-                    *iz = plane((S - 1) & 1, 2);
-        float *ox = plane(S & 1, 0), *oy = plane(S & 1, 1), *oz = plane(S & 1, 2);
+        const float *const in = cfs + (size_t)((S - 1) & 1) * 3 * me.buf;
+        float *const out = cfs + (size_t)(S & 1) * 3 * me.buf;
         for (int k = me.seg0; k < me.seg0 + me.nseg; ++k) {
             const CSeg sg = segs[k];
             const BatchLattice L = lats[sg.lat];
-            const int N = sg.N, rpp = T / N, r1 = tid / N, col = tid - r1 * N;
-            if (r1 >= rpp) continue;  // the last T % N threads
-            const int dl = (col == 0) ? N - 1 : -1, dr = (col == N - 1) ? 1 - N : 1;
-            // the segment's rows with the lattice's model terms fixed at compile time
-            auto rows_t = [&](auto j2c, auto hc, auto dc) {
+            const int N = sg.N, groups = T / N, grp = tid / N, col = tid - grp * N;
+            const int strip = (sg.rows + groups - 1) / groups, first = grp * strip;
+            const int cnt = min(strip, sg.rows - first);
+            if (grp >= groups || cnt <= 0) continue;
+            const int N3 = 3 * N, dl = col == 0 ? N3 - 3 : -3, dr = col == N - 1 ? 3 - N3 : 3;
+            const int slot = 3 * (sg.base + (first + 1) * N + col);
+            const float *p = in + slot;
+            float *o = out + slot;
+            const int site = 3 * (sg.core0 + first * N + col);
+            float *b = yb + site, *a = ac + site;
+            // the halo rows of the neighbouring CTAs: below the last row of the
+            // CTA above, above the first row of the CTA below
+            float *up_halo = nullptr, *dn_halo = nullptr;
+            if (first == 0)
+                up_halo = cluster.map_shared_rank(cfs, sg.top_rank) +
+                          (size_t)(S & 1) * 3 * sg.top_buf + 3 * (sg.top_off + N + col);
+            if (first + cnt == sg.rows)
+                dn_halo = cluster.map_shared_rank(cfs, sg.bot_rank) +
+                          (size_t)(S & 1) * 3 * sg.bot_buf + 3 * (sg.bot_off - N + col);
+            // the strip with the lattice's model terms fixed at compile time
+            auto strip_t = [&](auto j2c, auto hc, auto dc, auto uc) {
                 constexpr bool J2 = decltype(j2c)::value, H = decltype(hc)::value,
-                               DAMP = decltype(dc)::value;
-                for (int row = r1; row < sg.rows; row += rpp) {
-                    const int c = sg.base + (row + 1) * N + col, q = sg.core0 + row * N + col;
-                    auto at = [&](int o) { return F3{ix[o], iy[o], iz[o]}; };
+                               DAMP = decltype(dc)::value, UNIT = decltype(uc)::value;
+                auto at = [](const float *q) { return F3{q[0], q[1], q[2]}; };
+                F3 up = at(p - N3), mid = at(p);
+#pragma unroll 2
+                for (int r = 0; r < cnt; ++r) {
                     F3 nb[4], n2[4];
-                    nb[0] = at(c + N);
-                    nb[1] = at(c - N);
-                    nb[2] = at(c + dl);
-                    nb[3] = at(c + dr);
+                    nb[0] = at(p + N3);
+                    nb[1] = up;
+                    nb[2] = at(p + dl);
+                    nb[3] = at(p + dr);
                     if (J2) {
-                        n2[0] = at(c + N + dr);
-                        n2[1] = at(c + N + dl);
-                        n2[2] = at(c - N + dr);
-                        n2[3] = at(c - N + dl);
+                        n2[0] = at(p + N3 + dr);
+                        n2[1] = at(p + N3 + dl);
+                        n2[2] = at(p - N3 + dr);
+                        n2[3] = at(p - N3 + dl);
                     }
-                    const F3 d = rhs32_vals_t<J2, H, DAMP>(at(c), nb, n2, L);
-                    const float k0 = fm(d.x, L.dt), k1 = fm(d.y, L.dt), k2 = fm(d.z, L.dt);
+                    const F3 d = rhs32_vals_t<J2, H, DAMP, UNIT>(mid, nb, n2, L);
+                    const F3 kk{fm(d.x, L.dt), fm(d.y, L.dt), fm(d.z, L.dt)};
+                    F3 v;
                     if (S == 4) {
-                        const double o0 = (double)fa(ac[q], fd6(k0));
-                        const double o1 = (double)fa(ac[ns + q], fd6(k1));
-                        const double o2 = (double)fa(ac[2 * ns + q], fd6(k2));
+                        const F3 q = fdiv3_const(kk, 6.f, 1.f / 6.f);
+                        const double o0 = (double)fa(a[0], q.x), o1 = (double)fa(a[1], q.y),
+                                     o2 = (double)fa(a[2], q.z);
                         const double nrm = __dsqrt_rn(__dadd_rn(
                             __dadd_rn(__dmul_rn(o0, o0), __dmul_rn(o1, o1)), __dmul_rn(o2, o2)));
-                        const float n0 = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o0), nrm));
-                        const float n1 = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o1), nrm));
-                        const float n2v =
-                            __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o2), nrm));
-                        yb[q] = ox[c] = n0;
-                        yb[ns + q] = oy[c] = n1;
-                        yb[2 * ns + q] = oz[c] = n2v;
+                        v.x = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o0), nrm));
+                        v.y = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o1), nrm));
+                        v.z = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o2), nrm));
+                        b[0] = v.x;
+                        b[1] = v.y;
+                        b[2] = v.z;
                     } else {
-                        const float bx = yb[q], by = yb[ns + q], bz = yb[2 * ns + q];
-                        if (S == 3) {
-                            ox[c] = fa(bx, k0);
-                            oy[c] = fa(by, k1);
-                            oz[c] = fa(bz, k2);
-                        } else {
-                            ox[c] = fa(bx, fm(k0, 0.5f));
-                            oy[c] = fa(by, fm(k1, 0.5f));
-                            oz[c] = fa(bz, fm(k2, 0.5f));
-                        }
-                        if (S == 1) {
-                            ac[q] = fa(bx, fd6(k0));
-                            ac[ns + q] = fa(by, fd6(k1));
-                            ac[2 * ns + q] = fa(bz, fd6(k2));
-                        } else {
-                            ac[q] = fa(ac[q], fd3(k0));
-                            ac[ns + q] = fa(ac[ns + q], fd3(k1));
-                            ac[2 * ns + q] = fa(ac[2 * ns + q], fd3(k2));
-                        }
+                        const F3 base = S == 1 ? mid : at(b);
+                        const F3 q = S == 1 ? fdiv3_const(kk, 6.f, 1.f / 6.f)
+                                            : fdiv3_const(kk, 3.f, 1.f / 3.f);
+                        const F3 from = S == 1 ? base : at(a);
+                        a[0] = fa(from.x, q.x);
+                        a[1] = fa(from.y, q.y);
+                        a[2] = fa(from.z, q.z);
+                        v = S == 3 ? F3{fa(base.x, kk.x), fa(base.y, kk.y), fa(base.z, kk.z)}
+                                   : F3{fa(base.x, fm(kk.x, 0.5f)), fa(base.y, fm(kk.y, 0.5f)),
+                                        fa(base.z, fm(kk.z, 0.5f))};
                     }
+                    o[0] = v.x;
+                    o[1] = v.y;
+                    o[2] = v.z;
+                    if (r == 0 && up_halo) {
+                        up_halo[0] = v.x;
+                        up_halo[1] = v.y;
+                        up_halo[2] = v.z;
+                    }
+                    if (r == cnt - 1 && dn_halo) {
+                        dn_halo[0] = v.x;
+                        dn_halo[1] = v.y;
+                        dn_halo[2] = v.z;
+                    }
+                    up = mid;
+                    mid = nb[0];
+                    p += N3;
+                    o += N3;
+                    b += N3;
+                    a += N3;
                 }
             };
             using TT = std::true_type;
             using FF = std::false_type;
+            auto unit_t = [&](auto j2c, auto hc, auto dc) {
+                if (L.J1 == 1.f || L.J1 == -1.f) strip_t(j2c, hc, dc, TT{});
+                else strip_t(j2c, hc, dc, FF{});
+            };
             switch ((L.use_j2 ? 4 : 0) | (L.use_h ? 2 : 0) | (L.use_damp ? 1 : 0)) {
-                case 0: rows_t(FF{}, FF{}, FF{}); break;
-                case 1: rows_t(FF{}, FF{}, TT{}); break;
-                case 2: rows_t(FF{}, TT{}, FF{}); break;
-                case 3: rows_t(FF{}, TT{}, TT{}); break;
-                case 4: rows_t(TT{}, FF{}, FF{}); break;
-                case 5: rows_t(TT{}, FF{}, TT{}); break;
-                case 6: rows_t(TT{}, TT{}, FF{}); break;
-                default: rows_t(TT{}, TT{}, TT{}); break;
+                case 0: unit_t(FF{}, FF{}, FF{}); break;
+                case 1: unit_t(FF{}, FF{}, TT{}); break;
+                case 2: unit_t(FF{}, TT{}, FF{}); break;
+                case 3: unit_t(FF{}, TT{}, TT{}); break;
+                case 4: unit_t(TT{}, FF{}, FF{}); break;
+                case 5: unit_t(TT{}, FF{}, TT{}); break;
+                case 6: unit_t(TT{}, TT{}, FF{}); break;
+                default: unit_t(TT{}, TT{}, TT{}); break;
             }
         }
-        halo(S & 1);
+        // also, after the last stage: no CTA exits while another may store into
+        // its halo rows
+        barrier();
     };
     for (int step = 0; step < nsteps; ++step) {
         stage(std::integral_constant<int, 1>{});
@@ -412,9 +460,6 @@ __global__ void __launch_bounds__(CL_THREADS, 1)
         stage(std::integral_constant<int, 3>{});
         stage(std::integral_constant<int, 4>{});
     }
-    // No CTA may exit while another CTA of its cluster can still read its
-    // shared memory (the last halo copy).
-    cluster.sync();
     for (int k = me.seg0; k < me.seg0 + me.nseg; ++k) {
         const CSeg sg = segs[k];
         const long M = (long)sg.N * sg.N;
@@ -423,10 +468,25 @@ __global__ void __launch_bounds__(CL_THREADS, 1)
             const int row = e / sg.N, col = e - row * sg.N;
             const long i = (long)(sg.r0 + row) * sg.N + col;
             const int q = sg.core0 + e;
-            Y[i] = yb[q];
-            Y[M + i] = yb[ns + q];
-            Y[2 * M + i] = yb[2 * ns + q];
+            Y[i] = yb[3 * q];
+            Y[M + i] = yb[3 * q + 1];
+            Y[2 * M + i] = yb[3 * q + 2];
         }
+    }
+}
+
+// One lattice between the caller's layout float[M][3] and the planes [3][M].
+template <bool TO_PLANES>
+__global__ void __launch_bounds__(256) layout_kernel(const float *__restrict__ in, long M,
+                                                     float *__restrict__ out) {
+    const long t = (long)blockIdx.x * 256 + threadIdx.x;
+    if (t >= 3 * M) return;
+    if (TO_PLANES) {
+        const long c = t / M, i = t - c * M;
+        out[t] = in[3 * i + c];
+    } else {
+        const long i = t / 3, c = t - 3 * i;
+        out[t] = in[c * M + i];
     }
 }
 
@@ -838,11 +898,13 @@ int asd_batch_set_spins(asd_batch *b, int lattice, const float *spin_aos) {
     ASD_CUDA_TRY(cudaSetDevice(b->device));
     const BatchLattice &L = b->lat[lattice];
     const long M = (long)L.N * L.N;
-    std::vector<float> soa((size_t)3 * M);
-    for (long i = 0; i < M; ++i)
-        for (int c = 0; c < 3; ++c) soa[c * M + i] = spin_aos[3 * i + c];
-    ASD_CUDA_TRY(cudaMemcpy(b->y + L.off, soa.data(), soa.size() * sizeof(float),
-                            cudaMemcpyHostToDevice));
+    // staged in ysa (stage states only within a run)
+    ASD_CUDA_TRY(cudaMemcpyAsync(b->ysa, spin_aos, (size_t)3 * M * sizeof(float),
+                                 cudaMemcpyHostToDevice, b->stream));
+    layout_kernel<true><<<(unsigned)((3 * M + 255) / 256), 256, 0, b->stream>>>(b->ysa, M,
+                                                                                b->y + L.off);
+    ASD_CUDA_TRY(cudaGetLastError());
+    ASD_CUDA_TRY(cudaStreamSynchronize(b->stream));
     return ASD_OK;
 }
 
@@ -850,14 +912,14 @@ int asd_batch_get_spins(asd_batch *b, int lattice, float *spin_aos) {
     if (!b || !spin_aos || lattice < 0 || lattice >= (int)b->lat.size())
         return fail(ASD_ERR_INVALID, "bad argument");
     ASD_CUDA_TRY(cudaSetDevice(b->device));
-    ASD_CUDA_TRY(cudaStreamSynchronize(b->stream));
     const BatchLattice &L = b->lat[lattice];
     const long M = (long)L.N * L.N;
-    std::vector<float> soa((size_t)3 * M);
-    ASD_CUDA_TRY(cudaMemcpy(soa.data(), b->y + L.off, soa.size() * sizeof(float),
-                            cudaMemcpyDeviceToHost));
-    for (long i = 0; i < M; ++i)
-        for (int c = 0; c < 3; ++c) spin_aos[3 * i + c] = soa[c * M + i];
+    layout_kernel<false><<<(unsigned)((3 * M + 255) / 256), 256, 0, b->stream>>>(b->y + L.off, M,
+                                                                                 b->ysa);
+    ASD_CUDA_TRY(cudaGetLastError());
+    ASD_CUDA_TRY(cudaMemcpyAsync(spin_aos, b->ysa, (size_t)3 * M * sizeof(float),
+                                 cudaMemcpyDeviceToHost, b->stream));
+    ASD_CUDA_TRY(cudaStreamSynchronize(b->stream));
     return ASD_OK;
 }
 
