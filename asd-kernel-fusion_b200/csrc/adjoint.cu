@@ -23,15 +23,8 @@ namespace asd {
 namespace {
 
 #include "llg_math.cuh"
+#include "adjoint_math.cuh"
 
-__device__ __forceinline__ V3 v3(double x, double y, double z) { return V3{x, y, z}; }
-__device__ __forceinline__ V3 vadd(V3 a, V3 b) { return v3(a.x + b.x, a.y + b.y, a.z + b.z); }
-__device__ __forceinline__ V3 vsub(V3 a, V3 b) { return v3(a.x - b.x, a.y - b.y, a.z - b.z); }
-__device__ __forceinline__ V3 vmul(double s, V3 a) { return v3(s * a.x, s * a.y, s * a.z); }
-__device__ __forceinline__ double vdot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ V3 vcross(V3 a, V3 b) {
-    return v3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
 __device__ __forceinline__ V3 vload(const double *p) { return v3(p[0], p[1], p[2]); }
 __device__ __forceinline__ void vstore(double *p, V3 a) {
     p[0] = a.x;
@@ -39,7 +32,6 @@ __device__ __forceinline__ void vstore(double *p, V3 a) {
     p[2] = a.z;
 }
 
-constexpr int NPAR = 6;  // J1, J2, alpha, hx, hy, hz
 constexpr int TPB = 256;
 
 struct Site {
@@ -94,21 +86,10 @@ __device__ __forceinline__ void vjp_local(const LLGArgs &a, const Site &s,
     const V3 sv = vload(S + s.e);
     V3 nn, nnn;
     neighbour_sums(S, s, a.N, nn, nnn);
-    const V3 H = vadd(vadd(vmul(a.J1, nn), vmul(a.J2, nnn)), v3(a.hx, a.hy, a.hz));
-    const V3 tau = vcross(H, sv);
-    const V3 nu = vmul(a.g, vadd(m, vmul(a.alpha, vcross(m, sv))));
-    const V3 p = vcross(sv, nu);
-    const V3 l = vadd(vmul(a.g * a.alpha, vcross(tau, m)), vcross(nu, H));
+    V3 p, l;
+    vjp_vals(a, sv, nn, nnn, m, p, l, part);
     vstore(P + s.e, p);
     vstore(loc + s.e, l);
-    const V3 sxt = vcross(sv, tau);
-    const V3 f = vmul(a.g, vadd(tau, vmul(a.alpha, sxt)));
-    part[0] = vdot(p, nn);
-    part[1] = vdot(p, nnn);
-    part[2] = vdot(m, vadd(vmul(-2.0 * a.alpha * a.g, f), vmul(a.g, sxt)));
-    part[3] = p.x;
-    part[4] = p.y;
-    part[5] = p.z;
 }
 
 // Adjoint of the renormalisation, then the vector-Jacobian product at the

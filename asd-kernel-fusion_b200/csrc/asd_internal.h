@@ -212,6 +212,22 @@ cudaError_t launch_vjp_gather(const LLGArgs &a, const double *P_in, double *loc,
                               const double *lam_v, const double *lam_y_in, double *lam_y_out,
                               double cv, double cs, const double *S, double *P_out, double *bacc,
                               cudaStream_t st);
+// One segment of the resident adjoint (adjoint_resident.cu).
+struct AdjSegment {
+    const double *ck;    // state at step base, site-major
+    int base, len;       // steps base + 1 .. base + len
+    int newest;          // the last segment: lam starts at zero
+    int stride, E;       // S(q,t) at the steps e * stride, e <= E
+    const double2 *coef; // [E] factors of the loss gradient at those steps
+    const double2 *u, *G, *Z;  // phases [M], the origin's sums [K] and [3]
+    double *work, *states;     // work space; lam stays in it between segments
+    double *bacc;        // [adjoint_resident_blocks][6], added to
+};
+// CTAs of the resident adjoint (0: the lattice side does not allow it), and the
+// bytes of its work space and of that plus `states` states of a segment.
+int adjoint_resident_blocks(const LLGArgs &a);
+size_t adjoint_resident_bytes(const LLGArgs &a, int states, size_t *work_bytes);
+cudaError_t launch_adjoint_segment(const LLGArgs &a, const AdjSegment &q, cudaStream_t st);
 cudaError_t launch_loss_grad(double *lam, long M, int K, const double2 *u, const double2 *G,
                              const double2 *Z, double cre, double cim, cudaStream_t st);
 cudaError_t launch_param_reduce(const double *bacc, int nblocks, double *grad, cudaStream_t st);

@@ -98,11 +98,16 @@ struct asd_ctx {
     // adjoint work space (allocated on the first asd_ctx_loss_grad)
     std::vector<double *> adj_bufs;
     long adj_states = 0;
+    size_t adj_small_cap = 0;
+    double *adj_res = nullptr;  // the resident adjoint's work space
+    size_t adj_res_cap = 0;
+    bool adj_resident = false;  // the last loss call's choice
     bool adj_keep = false;  // the work space holds every stage state of a segment
     // the tape of the last loss forward pass: its S(q,t) values and sizes,
     // valid while the parameters and the origin stay those it ran with
     bool tape_valid = false;
     bool tape_keep = false;  // the backward pass keeps a segment's stage states
+    bool tape_resident = false;  // the work space is the resident adjoint's
     int tape_nsteps = 0, tape_stride = 0, tape_ckpt = 0;
     long tape_params = -1, tape_origin = -1;
     std::vector<double2> tape_S;
@@ -573,6 +578,17 @@ int step_into(asd_ctx *c, const double *y_in, double *s2, double *s3, double *s4
     return ASD_OK;
 }
 
+// The backward pass segment by segment in one launch each (adjoint_resident.cu)
+// where the default kernels run and the lattice side allows it (12 to 64): 1.4 to
+// 2.4 times the speed of the kernel-by-kernel adjoint from 16 replicas on (figures
+// in adjoint_resident.cu).  Fewer replicas keep the latter, which spreads a
+// lattice over all SMs.
+bool use_resident_adjoint(const asd_ctx *c) {
+    if (c->llg_kernel != ASD_LLG_AUTO || c->p.nfile < 16) return false;
+    const int blocks = adjoint_resident_blocks(c->a);
+    return blocks > 0;
+}
+
 // Work space of the adjoint: state-sized buffers (stage states, adjoint
 // variables, checkpoints, one recomputed segment) and small reduction buffers.
 // Where the RK4 step runs as four stage kernels and half of the free device
@@ -584,10 +600,26 @@ int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
     const int K = c->K, E = nsteps / stride;
     const size_t sb = (size_t)M * K * sizeof(double);
     const int nck = (nsteps + ckpt - 1) / ckpt;  // checkpoints at 0, ckpt, 2 ckpt, ...
-    long need = 10 + nck + (ckpt + 1);
+    const int seglen = std::min(ckpt, nsteps);
+    bool resident = use_resident_adjoint(c);
+    size_t work_bytes = 0;
+    const size_t resident_bytes =
+        resident ? adjoint_resident_bytes(c->a, seglen, &work_bytes) : 0;
+    if (resident && resident_bytes > c->adj_res_cap) {  // its padded states may need more memory
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+            resident = (double)resident_bytes <= 0.5 * ((double)free_b + (double)c->adj_res_cap);
+        } else {
+            cudaGetLastError();
+            resident = false;
+        }
+    }
+    c->adj_resident = resident;
+    // resident: the segment's states are in its own work space
+    long need = 10 + nck + (resident ? 2 : ckpt + 1);
     const long need_keep = need + 4L * ckpt;
     bool keep = false;
-    if (!use_fused(c, c->a)) {
+    if (!use_fused(c, c->a) && !resident) {
         size_t free_b = 0, total_b = 0;
         if (c->adj_states >= need_keep) {
             keep = true;
@@ -610,20 +642,30 @@ int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
         c->adj_states = 0;
         for (long i = 0; i < need; ++i)
             if ((rc = dalloc(&c->adj_bufs[i], sb)) != ASD_OK) return rc;
-        const int nb = adjoint_blocks(c->a);
+        const int nb = std::max(adjoint_blocks(c->a), adjoint_resident_blocks(c->a));
         const size_t small = (size_t)(nb + 1) * 6 * sizeof(double);
         if ((rc = dalloc(&c->adj_bufs[need], small)) != ASD_OK) return rc;
-        if ((rc = dalloc(&c->adj_bufs[need + 1], (size_t)(E + 8) * sizeof(double2))) != ASD_OK)
-            return rc;
+        c->adj_small_cap = 0;
         c->adj_states = need;
-    } else {
-        // the S(q,t) buffer depends on E
+    }
+    // S(q,t) and the loss gradient's factors per evaluation: grown on demand
+    const size_t small = (size_t)(2 * E + 8) * sizeof(double2);
+    double *&buf = c->adj_bufs[c->adj_states + 1];
+    if (small > c->adj_small_cap) {
         c->tape_valid = false;
-        if (c->adj_bufs[c->adj_states + 1]) cudaFree(c->adj_bufs[c->adj_states + 1]);
-        c->adj_bufs[c->adj_states + 1] = nullptr;
-        if ((rc = dalloc(&c->adj_bufs[c->adj_states + 1], (size_t)(E + 8) * sizeof(double2))) !=
-            ASD_OK)
-            return rc;
+        if (buf) cudaFree(buf);
+        buf = nullptr;
+        c->adj_small_cap = 0;
+        if ((rc = dalloc(&buf, small)) != ASD_OK) return rc;
+        c->adj_small_cap = small;
+    }
+    if (resident && resident_bytes > c->adj_res_cap) {
+        c->tape_valid = false;
+        if (c->adj_res) cudaFree(c->adj_res);
+        c->adj_res = nullptr;
+        c->adj_res_cap = 0;
+        if ((rc = dalloc(&c->adj_res, resident_bytes)) != ASD_OK) return rc;
+        c->adj_res_cap = resident_bytes;
     }
     return ASD_OK;
 }
@@ -634,11 +676,11 @@ struct AdjBufs {
     double **ck, **seg;
     double **stg;  // with a kept segment: stg[4 (j - 1) + q] = s2, s3, s4, acc of step j
     double *bacc, *dgrad;
-    double2 *Sv;
+    double2 *Sv, *coef;  // [E] each
     int nb;
 };
 
-AdjBufs adj_bufs(asd_ctx *c, int nck, int ckpt) {
+AdjBufs adj_bufs(asd_ctx *c, int nck, int ckpt, int E, bool resident) {
     double **B = c->adj_bufs.data();
     AdjBufs b;
     b.s2 = B[0], b.s3 = B[1], b.s4 = B[2], b.acc = B[3], b.lam = B[4], b.lam_v = B[5];
@@ -646,10 +688,11 @@ AdjBufs adj_bufs(asd_ctx *c, int nck, int ckpt) {
     b.ck = B + 10;        // nck checkpoints
     b.seg = B + 10 + nck; // ckpt + 1 recomputed states
     b.stg = b.seg + ckpt + 1;
-    b.nb = adjoint_blocks(c->a);
+    b.nb = resident ? adjoint_resident_blocks(c->a) : adjoint_blocks(c->a);
     b.bacc = B[c->adj_states];
     b.dgrad = b.bacc + (size_t)b.nb * 6;
     b.Sv = reinterpret_cast<double2 *>(B[c->adj_states + 1]);
+    b.coef = b.Sv + E + 4;
     return b;
 }
 
@@ -668,7 +711,7 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
     const int K = c->K, E = nsteps / stride;
     const size_t sb = (size_t)M * K * sizeof(double);
     const int nck = (nsteps + ckpt - 1) / ckpt;
-    AdjBufs b = adj_bufs(c, nck, ckpt);
+    AdjBufs b = adj_bufs(c, nck, ckpt, E, c->adj_resident);
     cudaStream_t st = c->stream;
     c->last_launches = 0;
     c->tape_valid = false;
@@ -727,6 +770,7 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
     if (loss) *loss = L;
     c->tape_valid = true;
     c->tape_keep = c->adj_keep;
+    c->tape_resident = c->adj_resident;
     c->tape_nsteps = nsteps;
     c->tape_stride = stride;
     c->tape_ckpt = ckpt;
@@ -748,7 +792,7 @@ int loss_backward(asd_ctx *c, const double *target, double *grad, double *dtarge
     const int E = nsteps / stride;
     const size_t sb = (size_t)M * K * sizeof(double);
     const int nck = (nsteps + ckpt - 1) / ckpt;
-    AdjBufs b = adj_bufs(c, nck, ckpt);
+    AdjBufs b = adj_bufs(c, nck, ckpt, E, c->tape_resident);
     cudaStream_t st = c->stream;
     int rc;
     c->last_launches = 0;
@@ -766,10 +810,29 @@ int loss_backward(asd_ctx *c, const double *target, double *grad, double *dtarge
     const bool fwd_fused = use_fused(c, c->a);
     const bool keep = c->tape_keep && !fwd_fused;
     // backward through the segments, last first
-    ASD_CUDA_TRY(cudaMemsetAsync(b.lam, 0, sb, st));
+    if (!c->tape_resident) ASD_CUDA_TRY(cudaMemsetAsync(b.lam, 0, sb, st));
     ASD_CUDA_TRY(cudaMemsetAsync(b.bacc, 0, (size_t)b.nb * 6 * sizeof(double), st));
     double **seg = b.seg;
-    for (int cidx = nck - 1; cidx >= 0; --cidx) {
+    if (c->tape_resident) {
+        ASD_CUDA_TRY(cudaMemcpyAsync(b.coef, coef.data(), (size_t)E * sizeof(double2),
+                                     cudaMemcpyHostToDevice, st));
+        size_t work_bytes = 0;
+        adjoint_resident_bytes(c->a, ckpt, &work_bytes);
+        AdjSegment q{};
+        q.stride = stride, q.E = E, q.coef = b.coef;
+        q.u = c->uphase, q.G = c->phase_G, q.Z = c->phase_G + K;
+        q.work = c->adj_res;
+        q.states = c->adj_res + work_bytes / sizeof(double);
+        q.bacc = b.bacc;
+        for (int cidx = nck - 1; cidx >= 0; --cidx) {
+            q.ck = b.ck[cidx];
+            q.base = cidx * ckpt;
+            q.len = std::min(nsteps - q.base, ckpt);
+            q.newest = cidx == nck - 1;
+            ASD_CUDA_TRY(launch_adjoint_segment(c->a, q, st));
+            c->last_launches += 1;
+        }
+    } else for (int cidx = nck - 1; cidx >= 0; --cidx) {
         const int base = cidx * ckpt;
         const int len = (nsteps - base < ckpt) ? nsteps - base : ckpt;
         ASD_CUDA_TRY(cudaMemcpyAsync(seg[0], b.ck[cidx], sb, cudaMemcpyDeviceToDevice, st));
@@ -1190,7 +1253,7 @@ void destroy(asd_ctx *c) {
     cudaStreamSynchronize(c->stream);
     void *ptrs[] = {c->y, c->ys_a, c->ys_b, c->acc, c->origin, c->mean_t, c->mean_0, c->uphase,
                     c->wphase, c->row4, c->col4, c->row1, c->col1, c->grid_tdiag, c->grid_ds, c->part,
-                    c->phase_ws, c->phase_G, c->grid_fft, c->d_out,
+                    c->phase_ws, c->phase_G, c->grid_fft, c->adj_res, c->d_out,
                     c->status, c->grid_g, c->grid_t, c->grid_out};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -1796,6 +1859,7 @@ int asd_ctx_debug_poison(asd_ctx *c) {
         {c->phase_ws, phase_work_bytes(c->M, c->K) - sizeof(double2)},  // not the count
         {c->grid_fft ? c->grid_fft + c->p.N : nullptr,  // not the twiddles
          qfft_work_bytes(c->p.N, c->K) - (size_t)c->p.N * sizeof(double2)},
+        {c->adj_res, c->adj_res_cap},
         {c->d_out, 2 * sizeof(double)},
         {c->grid_g, (size_t)c->M * sizeof(double)},
         {c->grid_t, (size_t)c->M * sizeof(double2)},

@@ -169,9 +169,13 @@ int asd_ctx_sqt_grid(asd_ctx *ctx, asd_sqt_mode mode, double *out);
  * doubles) receives the S(q,t_e) values.  Host buffers; synchronous.  The
  * current state is not changed.  Device work space, allocated on the first
  * call and kept by the context: about (nsteps / checkpoint + checkpoint + 13)
- * spin-state arrays; where the RK4 step runs as four stage kernels (small
- * lattices) and half of the free device memory holds them, 4 * checkpoint
- * more, so that the backward pass reads each segment's stage states instead
+ * spin-state arrays.  For N = 12 to 64 and at least 16 replicas the backward
+ * pass runs a segment per launch, each replica's lattice resident on chip, with a
+ * work space of about (checkpoint + 10) states laid out by thread (up to four
+ * times that for the smallest lattices) in place of the segment's states.
+ * Elsewhere, where the RK4 step runs as four stage kernels (small lattices) and
+ * half of the free device memory holds them, 4 * checkpoint more, so that the
+ * backward pass reads each segment's stage states instead
  * of recomputing them (the results are the same bits either way).  No
  * counterpart in the reference. */
 int asd_ctx_loss_grad(asd_ctx *ctx, int nsteps, int stride, int checkpoint, const double *target,
