@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const V3 from = st == 1 ? yb : pload(ac);
                 pstore(ac, V3{da(from.x, div(k.x)), da(from.y, div(k.y)),
                                        da(from.z, div(k.z))});
-                put(st & 1, r, V3{da(yb.x, dm(k.x, ck)), da(yb.y, dm(k.y, ck)), da(yb.z, dm(k.z, ck))});
+                put(st & 1, r, V3{add_pow2(yb.x, ck, k.x), add_pow2(yb.y, ck, k.y), add_pow2(yb.z, ck, k.z)});
             });
             barrier();
         }

@@ -155,7 +155,11 @@ cudaError_t launch_stage_t(const LLGArgs &a, const double *y, const double *ys, 
 // five rows in flight in registers.  Halo work is (wc + 8) / wc in columns;
 // DRAM traffic: y read once (the halo columns mostly from L2) and y_new
 // written once, 48 bytes per site-step.  Per (site, replica) the arithmetic
-// is the stage kernels' (bit-identical).
+// is the stage kernels' (bit-identical); with |J1| = 1 and the exact half and
+// whole factors as FMAs 42 of 303 FP64 operations go (128x128x500 379 -> 364 us,
+// 256x256x1000 with J2 3545 -> 3452 us).  Keeping y's own column in registers
+// (12 shared loads fewer) spilled 160 bytes at the 96 registers that two CTAs of
+// nine warps leave.
 namespace stream {
 constexpr int SF = 4;                  // replicas per CTA (96 contiguous bytes per site)
 constexpr int WC_MAX = 64;             // core columns per band
@@ -213,7 +217,7 @@ __device__ __forceinline__ void load_in(const double *up, const double *mid, con
     }
 }
 
-template <bool J2, bool H, bool DAMP>
+template <bool J2, bool H, bool DAMP, bool UNIT>
 __global__ void __launch_bounds__(stream::NT_MAX, 2)
     llg_step_stream_kernel(LLGArgs a, StreamGeom g, const double *__restrict__ y,
                            double *__restrict__ yout) {
@@ -296,29 +300,29 @@ __global__ void __launch_bounds__(stream::NT_MAX, 2)
             return in;
         };
         auto st1 = [&](const SIn &in, int r3, double *ac) {  // s1 = y + k/2, acc = y + k/6
-            const V3 d = llg_rhs_vals<J2, H, DAMP>(in.s, in.nb, in.n2, a);
+            const V3 d = llg_rhs_vals<J2, H, DAMP, UNIT>(in.s, in.nb, in.n2, a);
             const double k0 = dm(d.x, dt), k1 = dm(d.y, dt), k2 = dm(d.z, dt);
             double *o = s1 + r3 * rw + me;
-            o[0] = da(in.s.x, half(k0));
-            o[1] = da(in.s.y, half(k1));
-            o[2] = da(in.s.z, half(k2));
+            o[0] = add_pow2(in.s.x, 0.5, k0);
+            o[1] = add_pow2(in.s.y, 0.5, k1);
+            o[2] = add_pow2(in.s.z, 0.5, k2);
             ac[0] = da(in.s.x, div6(k0));
             ac[1] = da(in.s.y, div6(k1));
             ac[2] = da(in.s.z, div6(k2));
         };
         auto st2 = [&](const SIn &in, int r3, double *ac) {  // s2 = y + k/2, acc += k/3
-            const V3 d = llg_rhs_vals<J2, H, DAMP>(in.s, in.nb, in.n2, a);
+            const V3 d = llg_rhs_vals<J2, H, DAMP, UNIT>(in.s, in.nb, in.n2, a);
             const double k0 = dm(d.x, dt), k1 = dm(d.y, dt), k2 = dm(d.z, dt);
             double *o = s2 + r3 * rw + me;
-            o[0] = da(in.yb.x, half(k0));
-            o[1] = da(in.yb.y, half(k1));
-            o[2] = da(in.yb.z, half(k2));
+            o[0] = add_pow2(in.yb.x, 0.5, k0);
+            o[1] = add_pow2(in.yb.y, 0.5, k1);
+            o[2] = add_pow2(in.yb.z, 0.5, k2);
             ac[0] = da(ac[0], div3(k0));
             ac[1] = da(ac[1], div3(k1));
             ac[2] = da(ac[2], div3(k2));
         };
         auto st3 = [&](const SIn &in, int r3, double *ac) {  // s3 = y + k, acc += k/3
-            const V3 d = llg_rhs_vals<J2, H, DAMP>(in.s, in.nb, in.n2, a);
+            const V3 d = llg_rhs_vals<J2, H, DAMP, UNIT>(in.s, in.nb, in.n2, a);
             const double k0 = dm(d.x, dt), k1 = dm(d.y, dt), k2 = dm(d.z, dt);
             double *o = s3 + r3 * rw + me;
             o[0] = da(in.yb.x, k0);
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(stream::NT_MAX, 2)
             ac[2] = da(ac[2], div3(k2));
         };
         auto st4 = [&](const SIn &in, int r, const double *ac) {  // acc + k/6, renormalised
-            const V3 d = llg_rhs_vals<J2, H, DAMP>(in.s, in.nb, in.n2, a);
+            const V3 d = llg_rhs_vals<J2, H, DAMP, UNIT>(in.s, in.nb, in.n2, a);
             const double k0 = dm(d.x, dt), k1 = dm(d.y, dt), k2 = dm(d.z, dt);
             const double o0 = da(ac[0], div6(k0));
             const double o1 = da(ac[1], div6(k1));
@@ -404,10 +408,10 @@ size_t stream_smem_bytes(const StreamGeom &g) {
     return (size_t)stream::ROWS * g.rw * sizeof(double);
 }
 
-template <bool J2, bool H, bool DAMP>
+template <bool J2, bool H, bool DAMP, bool UNIT>
 cudaError_t launch_stream_t(const LLGArgs &a, const double *y, double *yout, cudaStream_t st) {
     using namespace stream;
-    auto k = llg_step_stream_kernel<J2, H, DAMP>;
+    auto k = llg_step_stream_kernel<J2, H, DAMP, UNIT>;
     StreamGeom g;
     g.nb = (a.N + WC_MAX - 1) / WC_MAX;
     g.wc = ((a.N + g.nb - 1) / g.nb + 7) / 8 * 8;  // wt * SF is a whole number of warps
@@ -441,16 +445,23 @@ cudaError_t launch_stream_t(const LLGArgs &a, const double *y, double *yout, cud
 cudaError_t launch_stream(const LLGArgs &a, const double *y, double *yout, cudaStream_t st) {
     if (a.f0 < 0 || a.nc < 1 || a.f0 + a.nc > a.nfile) return cudaErrorInvalidValue;
     const int sel = (a.use_j2 ? 4 : 0) | (a.use_h ? 2 : 0) | (a.use_damp ? 1 : 0);
+    const bool unit = a.J1 == 1.0 || a.J1 == -1.0;
+#define ASD_STREAM_CASE(S, J, Hh, D)                                              \
+    case S:                                                                       \
+        return unit ? launch_stream_t<J, Hh, D, true>(a, y, yout, st)             \
+                    : launch_stream_t<J, Hh, D, false>(a, y, yout, st);
     switch (sel) {
-        case 0: return launch_stream_t<false, false, false>(a, y, yout, st);
-        case 1: return launch_stream_t<false, false, true>(a, y, yout, st);
-        case 2: return launch_stream_t<false, true, false>(a, y, yout, st);
-        case 3: return launch_stream_t<false, true, true>(a, y, yout, st);
-        case 4: return launch_stream_t<true, false, false>(a, y, yout, st);
-        case 5: return launch_stream_t<true, false, true>(a, y, yout, st);
-        case 6: return launch_stream_t<true, true, false>(a, y, yout, st);
-        default: return launch_stream_t<true, true, true>(a, y, yout, st);
+        ASD_STREAM_CASE(0, false, false, false)
+        ASD_STREAM_CASE(1, false, false, true)
+        ASD_STREAM_CASE(2, false, true, false)
+        ASD_STREAM_CASE(3, false, true, true)
+        ASD_STREAM_CASE(4, true, false, false)
+        ASD_STREAM_CASE(5, true, false, true)
+        ASD_STREAM_CASE(6, true, true, false)
+        ASD_STREAM_CASE(7, true, true, true)
     }
+#undef ASD_STREAM_CASE
+    return cudaErrorInvalidValue;
 }
 
 // ------------------------------------------------- resident steps
@@ -611,7 +622,7 @@ __global__ void __launch_bounds__(resident::threads(W), resident::ctas_per_sm(W)
                 acc[r][0] = da(bx, div(k.x));
                 acc[r][1] = da(by, div(k.y));
                 acc[r][2] = da(bz, div(k.z));
-                return V3{da(yb.x, dm(k.x, ck)), da(yb.y, dm(k.y, ck)), da(yb.z, dm(k.z, ck))};
+                return V3{add_pow2(yb.x, ck, k.x), add_pow2(yb.y, ck, k.y), add_pow2(yb.z, ck, k.z)};
             });
             barrier();
         }

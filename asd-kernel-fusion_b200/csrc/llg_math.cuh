@@ -11,6 +11,10 @@ __device__ __forceinline__ double dq(double a, double b) { return __ddiv_rn(a, b
 // of the radix), without a division.
 __device__ __forceinline__ double half(double x) { return __dmul_rn(x, 0.5); }
 
+// y + c x for c a power of two: the product is exact (away from the subnormal
+// range), so one FMA gives the bits of the rounded product and sum.
+__device__ __forceinline__ double add_pow2(double y, double c, double x) { return __fma_rn(x, c, y); }
+
 // x / d for the constants d = 3 and 6, correctly rounded, by Markstein's
 // correction step (P. Markstein, IBM J. Res. Dev. 34(1), 1990): with
 // yinv = RN(1/d), q = RN(x * yinv) is within one ulp of x/d, the remainder
