@@ -81,6 +81,32 @@ __device__ __forceinline__ F3 ld3(const float *p, long M, long i) {
     return F3{__ldcg(p + i), __ldcg(p + M + i), __ldcg(p + 2 * M + i)};
 }
 
+// The renormalised spin RN32(RN64(RN64(l o_c) / RN64(|o|))), |o| the rounded square
+// root of ((o_x^2 + o_y^2) + o_z^2), all in FP64.  (l o_c) rsqrt(|o|^2), with CUDA's
+// rsqrt (within 1 ulp), is within 4 units of 2^-52 of that quotient, so both round
+// to the same float unless one of them lies that close to the middle between two
+// floats: the 29 bits below a float's last one, seen as a number, then differ from
+// 2^28 by less than 8.  There, and outside float's normal range, the divisions
+// themselves.  About 50 instructions a site instead of 140.
+__device__ __forceinline__ F3 renormalise(double o0, double o1, double o2, double l) {
+    const double n2 = __dadd_rn(__dadd_rn(__dmul_rn(o0, o0), __dmul_rn(o1, o1)), __dmul_rn(o2, o2));
+    const double a0 = __dmul_rn(l, o0), a1 = __dmul_rn(l, o1), a2 = __dmul_rn(l, o2);
+    const double y = rsqrt(n2);
+    const double q0 = __dmul_rn(a0, y), q1 = __dmul_rn(a1, y), q2 = __dmul_rn(a2, y);
+    auto clear = [](double q) {
+        const unsigned mid = ((unsigned)__double2loint(q) & 0x1fffffffu) - 0x0ffffff8u;
+        const double m = fabs(q);
+        return mid > 16u && m > 0x1p-120 && m < 0x1p120;
+    };
+    // an exact zero stays one, with its sign
+    if ((clear(q0) || o0 == 0.0) && (clear(q1) || o1 == 0.0) && (clear(q2) || o2 == 0.0) &&
+        n2 > 0x1p-500 && n2 < 0x1p500)
+        return F3{__double2float_rn(q0), __double2float_rn(q1), __double2float_rn(q2)};
+    const double nrm = __dsqrt_rn(n2);
+    return F3{__double2float_rn(__ddiv_rn(a0, nrm)), __double2float_rn(__ddiv_rn(a1, nrm)),
+              __double2float_rn(__ddiv_rn(a2, nrm))};
+}
+
 // dS/dt from the centre s and the neighbours nb (nearest, in the reference's
 // order (row+1), (row-1), (col-1), (col+1)) and n2 (diagonals (+1,+1),
 // (+1,-1), (-1,+1), (-1,-1); read only with J2), FP32, explicitly rounded.
@@ -228,12 +254,10 @@ __global__ void __launch_bounds__(256, 4) batch_kernel(const BatchLattice *__res
                     const double o0 = (double)fa(__ldcg(A + i), fd6(k0));
                     const double o1 = (double)fa(__ldcg(A + M + i), fd6(k1));
                     const double o2 = (double)fa(__ldcg(A + 2 * M + i), fd6(k2));
-                    const double nrm = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(o0, o0),
-                                                                      __dmul_rn(o1, o1)),
-                                                            __dmul_rn(o2, o2)));
-                    O[i] = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o0), nrm));
-                    O[M + i] = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o1), nrm));
-                    O[2 * M + i] = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o2), nrm));
+                    const F3 v = renormalise(o0, o1, o2, L.spin_len);
+                    O[i] = v.x;
+                    O[M + i] = v.y;
+                    O[2 * M + i] = v.z;
                 } else {
                     const F3 yb = ld3(Y, M, i);
                     const F3 kk{k0, k1, k2};
@@ -281,8 +305,9 @@ __global__ void __launch_bounds__(256, 4) batch_kernel(const BatchLattice *__res
 // Bound by instruction issue.  Measured on B200, 48 lattices of 48^2..160^2
 // (534 784 sites), autotuned: 28.0 us a step with halo rows fetched after a
 // cluster barrier and a CTA barrier a stage, sites walked row by row and the
-// exchange multiplied per neighbour; 18.8 us as it is (strips unrolled by 2; by 1
-// 19.6, by 3 19.2 with spills).
+// exchange multiplied per neighbour; 17.9 us as it is (strips unrolled by 2; by 1
+// 4 % slower, by 3 2 % with spills; three divisions and a root in every
+// renormalisation 18.9).
 struct CSeg {
     int lat;       // lattice
     int N;         // its side
@@ -392,11 +417,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1)
                         const F3 q = fdiv3_const(kk, 6.f, 1.f / 6.f);
                         const double o0 = (double)fa(a[0], q.x), o1 = (double)fa(a[1], q.y),
                                      o2 = (double)fa(a[2], q.z);
-                        const double nrm = __dsqrt_rn(__dadd_rn(
-                            __dadd_rn(__dmul_rn(o0, o0), __dmul_rn(o1, o1)), __dmul_rn(o2, o2)));
-                        v.x = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o0), nrm));
-                        v.y = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o1), nrm));
-                        v.z = __double2float_rn(__ddiv_rn(__dmul_rn(L.spin_len, o2), nrm));
+                        v = renormalise(o0, o1, o2, L.spin_len);
                         b[0] = v.x;
                         b[1] = v.y;
                         b[2] = v.z;
