@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(TPB) adj_renorm_vjp_kernel(
     LLGArgs a, const double *__restrict__ s4, const double *__restrict__ acc,
     const double *__restrict__ lam, double *__restrict__ lam_v, double *__restrict__ P,
     double *__restrict__ loc, double *__restrict__ bacc) {
+    pdl_begin();
     double part[NPAR] = {0, 0, 0, 0, 0, 0};
     Site s;
     if (site_of(a, s)) {
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(TPB) vjp_gather_kernel(
     LLGArgs a, const double *__restrict__ P_in, double *loc, const double *__restrict__ lam_v,
     const double *lam_y_in, double *lam_y_out, double cv, double cs,
     const double *__restrict__ S, double *__restrict__ P_out, double *__restrict__ bacc) {
+    pdl_begin();
     double part[NPAR] = {0, 0, 0, 0, 0, 0};
     Site s;
     if (site_of(a, s)) {
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(double *__restrict__ lam
                                                         const double2 *__restrict__ G,
                                                         const double2 *__restrict__ Z,
                                                         double cre, double cim) {
+    pdl_begin();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= M * K) return;
     const long i = t / K;
@@ -164,6 +167,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(double *__restrict__ lam
 
 __global__ void param_reduce_kernel(const double *__restrict__ bacc, int nblocks,
                                     double *__restrict__ grad) {
+    pdl_begin();
     __shared__ double red[NPAR][256];
     double v[NPAR] = {0, 0, 0, 0, 0, 0};
     for (int b = threadIdx.x; b < nblocks; b += 256)
@@ -192,9 +196,8 @@ cudaError_t launch_adj_renorm_vjp(const LLGArgs &a, const double *s4, const doub
     const int nb = adjoint_blocks(a);
 #define ASD_ADJ_CASE(S, J, Hh, D)                                                          \
     case S:                                                                                \
-        adj_renorm_vjp_kernel<J, Hh, D><<<nb, TPB, 0, st>>>(a, s4, acc, lam, lam_v, P, loc, \
-                                                            bacc);                         \
-        break;
+        return launch_pdl(adj_renorm_vjp_kernel<J, Hh, D>, nb, TPB, 0, st, a, s4, acc, lam, \
+                          lam_v, P, loc, bacc);
     switch (sel) {
         ASD_ADJ_CASE(0, false, false, false)
         ASD_ADJ_CASE(1, false, false, true)
@@ -206,28 +209,26 @@ cudaError_t launch_adj_renorm_vjp(const LLGArgs &a, const double *s4, const doub
         ASD_ADJ_CASE(7, true, true, true)
     }
 #undef ASD_ADJ_CASE
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_vjp_gather(const LLGArgs &a, const double *P_in, double *loc,
                               const double *lam_v, const double *lam_y_in, double *lam_y_out,
                               double cv, double cs, const double *S, double *P_out, double *bacc,
                               cudaStream_t st) {
-    vjp_gather_kernel<<<adjoint_blocks(a), TPB, 0, st>>>(a, P_in, loc, lam_v, lam_y_in, lam_y_out,
-                                                         cv, cs, S, P_out, bacc);
-    return cudaGetLastError();
+    return launch_pdl(vjp_gather_kernel, adjoint_blocks(a), TPB, 0, st, a, P_in, loc, lam_v, lam_y_in,
+                      lam_y_out, cv, cs, S, P_out, bacc);
 }
 
 cudaError_t launch_loss_grad(double *lam, long M, int K, const double2 *u, const double2 *G,
                              const double2 *Z, double cre, double cim, cudaStream_t st) {
     const long n = M * K;
-    loss_grad_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(lam, M, K, u, G, Z, cre, cim);
-    return cudaGetLastError();
+    return launch_pdl(loss_grad_kernel, (unsigned)((n + 255) / 256), 256, 0, st, lam, M, K, u, G, Z,
+                      cre, cim);
 }
 
 cudaError_t launch_param_reduce(const double *bacc, int nblocks, double *grad, cudaStream_t st) {
-    param_reduce_kernel<<<1, 256, 0, st>>>(bacc, nblocks, grad);
-    return cudaGetLastError();
+    return launch_pdl(param_reduce_kernel, 1, 256, 0, st, bacc, nblocks, grad);
 }
 
 }  // namespace asd

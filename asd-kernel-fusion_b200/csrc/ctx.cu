@@ -365,11 +365,11 @@ int set_spins_common(asd_ctx *c, const double *aos, bool host, int as_origin) {
 }
 
 // The LLG kernel for one step of replicas [a.f0, a.f0 + a.nc) out of place: the
-// one-launch step or the four stage kernels (ASD_LLG_AUTO: the former where it
-// fills the GPU; steps in place may also run resident, llg_resident_wins).
+// one-launch step or the four stage kernels (ASD_LLG_AUTO: the faster one there;
+// steps in place may also run resident, llg_resident_wins).
 bool use_fused(const asd_ctx *c, const LLGArgs &a) {
     return c->llg_kernel == ASD_LLG_FUSED_STEP ||
-           (c->llg_kernel == ASD_LLG_AUTO && llg_fused_fills(a));
+           (c->llg_kernel == ASD_LLG_AUTO && llg_fused_wins(a));
 }
 
 int run_steps(asd_ctx *c, int nsteps) {

@@ -9,6 +9,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <type_traits>
 
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(256, 8) llg_stage_kernel(LLGArgs a, const doub
                                                         const double *__restrict__ ys,
                                                         double *__restrict__ acc,
                                                         double *__restrict__ out, int ngroups) {
+    pdl_begin();
     long site;
     int f;
     if (ngroups > 0) {
@@ -118,9 +120,8 @@ cudaError_t launch_stage_t(const LLGArgs &a, const double *y, const double *ys, 
                                         : (unsigned)((total + threads - 1) / threads);
 #define ASD_STAGE_CASE(S, J, Hh, D)                                                            \
     case S:                                                                                    \
-        llg_stage_kernel<STAGE, J, Hh, D><<<blocks, threads, 0, st>>>(a, y, ys, acc, out,      \
-                                                                       ngroups);               \
-        break;
+        return launch_pdl(llg_stage_kernel<STAGE, J, Hh, D>, blocks, threads, 0, st, a, y, ys, \
+                          acc, out, ngroups);
     switch (sel) {
         ASD_STAGE_CASE(0, false, false, false)
         ASD_STAGE_CASE(1, false, false, true)
@@ -132,7 +133,7 @@ cudaError_t launch_stage_t(const LLGArgs &a, const double *y, const double *ys, 
         ASD_STAGE_CASE(7, true, true, true)
     }
 #undef ASD_STAGE_CASE
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 // ------------------------------------------------ row-streaming step
@@ -221,6 +222,7 @@ template <bool J2, bool H, bool DAMP, bool UNIT>
 __global__ void __launch_bounds__(stream::NT_MAX, 2)
     llg_step_stream_kernel(LLGArgs a, StreamGeom g, const double *__restrict__ y,
                            double *__restrict__ yout) {
+    pdl_begin();
     using namespace stream;
     extern __shared__ double ssm[];
     const int rw = g.rw;
@@ -404,6 +406,18 @@ __global__ void __launch_bounds__(stream::NT_MAX, 2)
     }
 }
 
+StreamGeom stream_geom(const LLGArgs &a) {
+    using namespace stream;
+    StreamGeom g;
+    g.nb = (a.N + WC_MAX - 1) / WC_MAX;
+    g.wc = ((a.N + g.nb - 1) / g.nb + 7) / 8 * 8;  // wt * SF is a whole number of warps
+    g.wt = g.wc + 8;
+    g.rw = g.wt * SF * 3;
+    g.ng = (a.nc + SF - 1) / SF;
+    g.run = 0;
+    return g;
+}
+
 size_t stream_smem_bytes(const StreamGeom &g) {
     return (size_t)stream::ROWS * g.rw * sizeof(double);
 }
@@ -412,12 +426,7 @@ template <bool J2, bool H, bool DAMP, bool UNIT>
 cudaError_t launch_stream_t(const LLGArgs &a, const double *y, double *yout, cudaStream_t st) {
     using namespace stream;
     auto k = llg_step_stream_kernel<J2, H, DAMP, UNIT>;
-    StreamGeom g;
-    g.nb = (a.N + WC_MAX - 1) / WC_MAX;
-    g.wc = ((a.N + g.nb - 1) / g.nb + 7) / 8 * 8;  // wt * SF is a whole number of warps
-    g.wt = g.wc + 8;
-    g.rw = g.wt * SF * 3;
-    g.ng = (a.nc + SF - 1) / SF;
+    StreamGeom g = stream_geom(a);
     const int threads = g.wt * SF;
     const size_t smem = stream_smem_bytes(g);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -438,8 +447,7 @@ cudaError_t launch_stream_t(const LLGArgs &a, const double *y, double *yout, cud
     g.run = run;
     const long blocks = (total + run - 1) / run;
     if (blocks > 0x7fffffffL) return cudaErrorInvalidConfiguration;
-    k<<<(unsigned)blocks, threads, smem, st>>>(a, g, y, yout);
-    return cudaGetLastError();
+    return launch_pdl(k, (unsigned)blocks, threads, smem, st, a, g, y, yout);
 }
 
 cudaError_t launch_stream(const LLGArgs &a, const double *y, double *yout, cudaStream_t st) {
@@ -497,6 +505,7 @@ template <int W, bool J2, bool H, bool DAMP, bool UNIT, bool CL>
 __global__ void __launch_bounds__(resident::threads(W), resident::ctas_per_sm(W))
     llg_resident_kernel(LLGArgs a, ResGeom g, const double *y, double *yout, double *scratch,
                         int nsteps) {
+    pdl_begin();
     namespace cg = cooperative_groups;
     constexpr int RP = resident::rows_per_thread(W), WARPS = resident::threads(W) / 32;
     constexpr int RS = 3 * W;  // doubles per row
@@ -659,6 +668,7 @@ template <bool TO_SITEMAJOR>
 __global__ void __launch_bounds__(256) transpose_kernel(const double *__restrict__ src,
                                                         double *__restrict__ dst, long M,
                                                         int nfile, int fbeg, int nc) {
+    pdl_begin();
     // The AoS side holds replicas [fbeg, fbeg + nc) as [nc][M][3]; the
     // site-major side is the whole [M][nfile][3] array.  lf = local replica.
     __shared__ double tile[32][32 * 3 + 1];
@@ -809,13 +819,15 @@ static cudaError_t launch_resident_t(const LLGArgs &a, const ResGeom &g, size_t 
     cfg.blockDim = dim3(resident::threads(W));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)g.s;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)g.s;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = CL ? 1 : 0;
+    cfg.numAttrs = CL ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k, a, g, y, yout, scratch, nsteps);
 }
 
@@ -859,53 +871,55 @@ cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout,
 }
 
 // The three ways to step, compared by what each was measured to take on B200 (in
-// us a step; the lines below are within 10 % of the measurements that matter,
-// those near the crossings).  w = site-replicas, n = sites of a CTA:
-//   stage kernels   16 + 0.065e-3 w (0.073 with J2): four launches, then HBM / L2
-//   one-launch      the larger of 48 and 10 + 0.055e-3 w (0.068)
-//   resident        4 a launch, and per round of resident CTAs, q to an SM:
+// us a step; within 10 % of the measurements near the crossings).  w =
+// site-replicas, n = sites of a CTA:
+//   stage kernels   9 + 0.065e-3 w (0.073 with J2): four launches, then HBM / L2
+//   one-launch      rows per CTA + 9 iterations, for 72 columns 3.1 with two CTAs
+//                   an SM and 1.8 with one (1.29 times that with J2)
+//   resident        2.8 a launch, and per round of resident CTAs, q to an SM:
 //                   2.3 + 3.7e-3 q n a step (4.7 with J2; clusters 6.3 + 3.9e-3 n),
 //                   and 0.8 + 2.6e-3 q n once to load and store the lattice
 // Measured, stage kernels / one-launch / resident 1 step / resident 10 steps:
-//   32x32x50    16.4 /  39 / 13.7 /  7.0     64x64x8    16.4 / 47 / 31.5 / 18.5
-//   32x32x200   29.0 /  37 / 18.9 / 10.3     64x64x100  43.6 / 49 / 35.3 / 18.9
-//   32x32x1000  76.1 /  71 / 52.0 / 31.8     12x12x1000 24.6 / 50 / 18.9 / 10.1
-//   64x64x400   121 / 105 / 109 / 57.8       128x128x500 548 / 388 / 604 / 333
-//   51x51x70    29.4 /  49 / 25.1 / 13.6
+//   32x32x50    11.2 /  36 / 12.2 /  6.9     64x64x8     9.7 / 45 / 31.4 / 18.5
+//   32x32x200   22   /  37 / 16.3 / 10.2     64x64x100  35.8 / 45 / 35.3 / 18.6
+//   32x32x1000  70   /  67 / 51.9 / 31.5     12x12x1000 18   / 49 / 18.9 / 10.1
+//   64x64x400   115  /  98 / 103  / 55.6     128x128x500 548 / 368 / 604 / 335
+//   51x51x70    22   /  48 / 21.3 / 13.5     90x90x60   36.5 / 60
+static double stages_cost(const LLGArgs &a) {
+    return 9.0 + (a.use_j2 ? 0.073e-3 : 0.065e-3) * (double)a.M * a.nc;
+}
+
+static double fused_cost(const LLGArgs &a) {
+    const StreamGeom g = stream_geom(a);
+    const long total = (long)g.nb * g.ng * a.N;
+    const double run = std::max<double>(stream::MIN_RUN, total / (2.0 * 148));
+    const double two = std::min(1.0, std::max(0.0, total / run / 148.0 - 1.0));  // SMs with two
+    const double iter = std::max(1.45 + 0.45 * two, (1.8 + 1.3 * two) * (g.wt + 24) / 96.0);
+    return (run + 9.0) * iter * (a.use_j2 ? 1.29 : 1.0);
+}
+
+bool llg_fused_wins(const LLGArgs &a) { return fused_cost(a) < 0.95 * stages_cost(a); }
+
 bool llg_resident_wins(const LLGArgs &a, int nsteps) {
     ResGeom g;
     int w = 0;
     size_t smem = 0;
     if (!resident_geom(a.N, g, w, smem)) return false;
-    const double work = (double)a.M * a.nc, n = (double)g.rows * a.N;
-    const double stages = 16.0 + (a.use_j2 ? 0.073e-3 : 0.065e-3) * work;
-    const double fused = std::max(48.0, 10.0 + (a.use_j2 ? 0.068e-3 : 0.055e-3) * work);
+    const double n = (double)g.rows * a.N;
     const bool cl = g.s > 1;
-    // CTAs an SM has to take in all, and at once (clusters of 4 fill about 140
-    // of the 148 SMs)
-    const long total = (long)a.nc * g.s, per_sm = (total + (cl ? 139 : 147)) / (cl ? 140 : 148);
     const double base = cl ? 6.3 : 2.3, site = (cl ? 3.9e-3 : 3.7e-3) * (a.use_j2 ? 1.27 : 1.0);
-    double res = 4.0;
-    for (long left = per_sm; left > 0;) {
-        const long q = std::min<long>(left, resident::ctas_per_sm(w));
-        const long rounds = left / q;
-        res += rounds * (nsteps * (base + site * q * n) + 0.8 + 2.6e-3 * q * n);
-        left -= rounds * q;
+    auto round = [&](double q) { return nsteps * (base + site * q * n) + 0.8 + 2.6e-3 * q * n; };
+    // CTAs an SM takes in all (clusters of 4 fill about 140 of the 148), and q at once
+    const double per_sm = (double)a.nc * g.s / (cl ? 140.0 : 148.0);
+    const int at_once = resident::ctas_per_sm(w);
+    double res = 2.8;
+    if (per_sm > 3.0 * at_once) {  // rounds blur into one another
+        res += (per_sm / at_once + 0.3) * round(at_once);
+    } else {
+        for (int left = (int)std::ceil(per_sm); left > 0; left -= at_once)
+            res += round(std::min(left, at_once));
     }
-    return res < 0.95 * nsteps * (llg_fused_fills(a) ? fused : stages);
-}
-
-bool llg_fused_fills(const LLGArgs &a) {
-    using namespace stream;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    const long nb = (a.N + WC_MAX - 1) / WC_MAX, ng = (a.nc + SF - 1) / SF;
-    const long slots = 2L * sms;  // two CTAs of the streamed step per SM
-    return nb * ng * a.N >= 8 * slots;
+    return res < 0.95 * nsteps * std::min(stages_cost(a), fused_cost(a));
 }
 
 cudaError_t launch_llg_step_fused(const LLGArgs &a, const double *y, double *yout,
@@ -917,16 +931,14 @@ cudaError_t launch_aos_to_sitemajor_range(const double *aos, double *sm, long M,
                                           int f0, int nc, cudaStream_t st) {
     if (f0 < 0 || nc < 1 || f0 + nc > nfile) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((M + 31) / 32), (unsigned)((nc + 31) / 32));
-    transpose_kernel<true><<<grid, 256, 0, st>>>(aos, sm, M, nfile, f0, nc);
-    return cudaGetLastError();
+    return launch_pdl(transpose_kernel<true>, grid, 256, 0, st, aos, sm, M, nfile, f0, nc);
 }
 
 cudaError_t launch_sitemajor_to_aos_range(const double *sm, double *aos, long M, int nfile,
                                           int f0, int nc, cudaStream_t st) {
     if (f0 < 0 || nc < 1 || f0 + nc > nfile) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((M + 31) / 32), (unsigned)((nc + 31) / 32));
-    transpose_kernel<false><<<grid, 256, 0, st>>>(sm, aos, M, nfile, f0, nc);
-    return cudaGetLastError();
+    return launch_pdl(transpose_kernel<false>, grid, 256, 0, st, sm, aos, M, nfile, f0, nc);
 }
 
 cudaError_t launch_aos_to_sitemajor(const double *aos, double *sm, long M, int nfile,

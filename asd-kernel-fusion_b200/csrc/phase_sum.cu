@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(PS_THREADS) phase_sum_kernel(const double *__r
                                                                const double2 *__restrict__ ph,
                                                                long rows,
                                                                double2 *__restrict__ Fpart) {
+    pdl_begin();
     const int k = (blockIdx.x * PS_THREADS + threadIdx.x) * VEC;
     if (k >= K) return;
     const long i0 = (long)blockIdx.y * rows, i1 = min(M, i0 + rows);
@@ -124,6 +125,7 @@ __device__ __forceinline__ double2 column_sum(const double2 *__restrict__ Fpart,
 __global__ void __launch_bounds__(PV_K *PV_SLICES) phase_origin_kernel(
     const double2 *__restrict__ Fpart, int nchunks, int K, int nfile, double2 *__restrict__ G,
     double2 *__restrict__ Z, unsigned *__restrict__ count) {
+    pdl_begin();
     const int k = blockIdx.x * PV_K + threadIdx.x % PV_K;
     const double2 f = column_sum(Fpart, nchunks, K, k);
     if (threadIdx.x < PV_K && k < K) G[k] = f;
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(PV_K *PV_SLICES) phase_value_kernel(
     const double2 *__restrict__ Fpart, int nchunks, int K, const double2 *__restrict__ G,
     const double2 *__restrict__ Z, double scale, double2 *__restrict__ part,
     unsigned *__restrict__ count, double *__restrict__ out) {
+    pdl_begin();
     const int k = blockIdx.x * PV_K + threadIdx.x % PV_K;
     const double2 f = column_sum(Fpart, nchunks, K, k);
     if (threadIdx.x < PV_K) {
@@ -202,11 +205,8 @@ cudaError_t sum_columns(const double *A, long M, int K, const double2 *ph, const
     const int vec = (K % 2 == 0 && ((uintptr_t)A & 15) == 0) ? 2 : 1;
     const int cols = PS_THREADS * vec;
     const dim3 grid((unsigned)((K + cols - 1) / cols), (unsigned)chunks_for(M, K));
-    if (vec == 2)
-        phase_sum_kernel<2><<<grid, PS_THREADS, 0, st>>>(A, M, K, ph, rows, w.Fpart);
-    else
-        phase_sum_kernel<1><<<grid, PS_THREADS, 0, st>>>(A, M, K, ph, rows, w.Fpart);
-    return cudaGetLastError();
+    return launch_pdl(vec == 2 ? phase_sum_kernel<2> : phase_sum_kernel<1>, grid, PS_THREADS, 0, st,
+                      A, M, K, ph, rows, w.Fpart);
 }
 
 }  // namespace
@@ -227,9 +227,8 @@ cudaError_t launch_phase_origin(const double *B, long M, int K, int nfile, const
                                 const PhaseWork &w, double2 *G, double2 *Z, cudaStream_t st) {
     cudaError_t e = sum_columns(B, M, K, wphase, w, st);
     if (e != cudaSuccess) return e;
-    phase_origin_kernel<<<value_blocks(K), PV_K * PV_SLICES, 0, st>>>(
-        w.Fpart, chunks_for(M, K), K, nfile, G, Z, w.count);
-    return cudaGetLastError();
+    return launch_pdl(phase_origin_kernel, value_blocks(K), PV_K * PV_SLICES, 0, st, w.Fpart,
+                      chunks_for(M, K), K, nfile, G, Z, w.count);
 }
 
 cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *uphase,
@@ -237,9 +236,8 @@ cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *upha
                              double *out, cudaStream_t st) {
     cudaError_t e = sum_columns(A, M, K, uphase, w, st);
     if (e != cudaSuccess) return e;
-    phase_value_kernel<<<value_blocks(K), PV_K * PV_SLICES, 0, st>>>(
-        w.Fpart, chunks_for(M, K), K, G, Z, scale, w.part, w.count, out);
-    return cudaGetLastError();
+    return launch_pdl(phase_value_kernel, value_blocks(K), PV_K * PV_SLICES, 0, st, w.Fpart,
+                      chunks_for(M, K), K, G, Z, scale, w.part, w.count, out);
 }
 
 }  // namespace asd

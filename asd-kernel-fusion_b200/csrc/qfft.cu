@@ -210,6 +210,7 @@ struct Chunk {
 __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
     FftPlan p, const double *__restrict__ A, const double *__restrict__ B, int K, int k0, Chunk X,
     const double *__restrict__ m, const double *__restrict__ z, const double2 *__restrict__ tw) {
+    pdl_begin();
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lk;
     double2 *b0 = fsm, *b1 = fsm + (n << p.lk), *stw = b1 + (n << p.lk);
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
 // k blocks of this chunk.  add: onto the sums of the earlier chunks.
 __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
     FftPlan p, Chunk X, const double2 *__restrict__ tw, int add, double2 *__restrict__ part) {
+    pdl_begin();
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lkc, lt = p.lkc + 1, len = n << p.lkc;
     double2 *b0 = fsm, *b1 = b0 + (n << lt), *sum = b1 + (n << lt), *stw = sum + n;
@@ -293,6 +295,7 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
 __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict__ part, int n,
                                                        int slices, double scale,
                                                        double2 *__restrict__ out) {
+    pdl_begin();
     __shared__ double2 red[8][16];
     const int tl = threadIdx.x & 15, sl = threadIdx.x >> 4;
     const long t = (long)blockIdx.x * 16 + tl;
@@ -328,6 +331,7 @@ __global__ void __launch_bounds__(MAX_THREADS) bins_dft_kernel(FftPlan p,
                                                                const double2 *__restrict__ tw,
                                                                double scale,
                                                                double2 *__restrict__ out) {
+    pdl_begin();
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lk;
     double2 *b0 = fsm, *b1 = fsm + (n << p.lk), *stw = b1 + (n << p.lk);
@@ -437,18 +441,17 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
         for (int q = 0; q < 3; ++q) X.buf[q] = reinterpret_cast<double2 *>(scratch[q]);
         X.blocks = all - b0 < g.blocks ? all - b0 : g.blocks;
         X.per = g.per;
-        qfft_rows_kernel<<<dim3((unsigned)X.blocks, (unsigned)lat_n), rows_t, rows_smem(p), st>>>(
-            p, A, B, K, b0 * kc, X, m, z, tw);
+        ASD_CUDA_TRY(launch_pdl(qfft_rows_kernel, dim3((unsigned)X.blocks, (unsigned)lat_n), rows_t,
+                                rows_smem(p), st, p, A, B, K, b0 * kc, X, m, z, tw));
         // a last, shorter chunk still visits every slice (with no block it adds zero)
-        qfft_cols_kernel<<<dim3((unsigned)(lat_n / 2 + 1), (unsigned)g.slices), cols_t,
-                           cols_smem(p), st>>>(p, X, tw, b0 > 0, part);
-        ASD_CUDA_TRY(cudaGetLastError());
+        ASD_CUDA_TRY(launch_pdl(qfft_cols_kernel,
+                                dim3((unsigned)(lat_n / 2 + 1), (unsigned)g.slices), cols_t,
+                                cols_smem(p), st, p, X, tw, b0 > 0, part));
         launches += 2;
     }
     const long half = (long)lat_n * (lat_n / 2 + 1);
-    qfft_sum_kernel<<<(unsigned)((half + 15) / 16), 128, 0, st>>>(
-        part, lat_n, g.slices, scale, reinterpret_cast<double2 *>(out));
-    ASD_CUDA_TRY(cudaGetLastError());
+    ASD_CUDA_TRY(launch_pdl(qfft_sum_kernel, (unsigned)((half + 15) / 16), 128, 0, st, part, lat_n,
+                            g.slices, scale, reinterpret_cast<double2 *>(out)));
     return launches + 1;
 }
 
@@ -465,10 +468,11 @@ cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const doub
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
             cudaSuccess)
         return e;
-    bins_dft_kernel<true><<<blocks, threads, smem, st>>>(p, G, nullptr, tw, 1.0, T);
-    bins_dft_kernel<false><<<blocks, threads, smem, st>>>(p, nullptr, T, tw, scale,
-                                                          reinterpret_cast<double2 *>(out));
-    return cudaGetLastError();
+    if ((e = launch_pdl(bins_dft_kernel<true>, blocks, threads, smem, st, p, G, nullptr, tw, 1.0,
+                        T)) != cudaSuccess)
+        return e;
+    return launch_pdl(bins_dft_kernel<false>, blocks, threads, smem, st, p, nullptr, T, tw, scale,
+                      reinterpret_cast<double2 *>(out));
 }
 
 }  // namespace asd

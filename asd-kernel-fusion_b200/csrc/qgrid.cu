@@ -32,6 +32,7 @@ __device__ __forceinline__ long floordiv(long a, long b) {  // b > 0
 
 __global__ void qgrid_keys_kernel(const double *__restrict__ tdiag, int num_m, int num_n, int bm,
                                   int bn, double *__restrict__ ds) {
+    pdl_begin();
     const int R = bn / bm, nd = bm + bn - 1;
     const long nkeys = num_m + (long)R * (num_n - 1);
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -53,6 +54,7 @@ __global__ void qgrid_keys_kernel(const double *__restrict__ tdiag, int num_m, i
 
 __global__ void qgrid_bins_kernel(const double *__restrict__ ds, int num_m, int num_n, int bm,
                                   int bn, int N, double *__restrict__ G) {
+    pdl_begin();
     const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= (long)N * N) return;
     const int R = bn / bm, nd = bm + bn - 1;
@@ -86,10 +88,12 @@ cudaError_t launch_qgrid_bins(const double *tdiag, int num_m, int num_n, int bm,
                               double *ds, double *G, cudaStream_t st) {
     if (bn % bm != 0) return cudaErrorInvalidValue;
     const long n1 = qgrid_keys(num_m, num_n, bm, bn) * (bm + bn - 1) * 2;
-    qgrid_keys_kernel<<<(unsigned)((n1 + 255) / 256), 256, 0, st>>>(tdiag, num_m, num_n, bm, bn, ds);
+    const cudaError_t e = launch_pdl(qgrid_keys_kernel, (unsigned)((n1 + 255) / 256), 256, 0, st,
+                                     tdiag, num_m, num_n, bm, bn, ds);
+    if (e != cudaSuccess) return e;
     const long n2 = (long)lat_n * lat_n;
-    qgrid_bins_kernel<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>(ds, num_m, num_n, bm, bn, lat_n, G);
-    return cudaGetLastError();
+    return launch_pdl(qgrid_bins_kernel, (unsigned)((n2 + 255) / 256), 256, 0, st, ds, num_m, num_n,
+                      bm, bn, lat_n, G);
 }
 
 }  // namespace asd

@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(256) site_mean_kernel(const double *__restrict
                                                         double *__restrict__ mean,
                                                         float4 *__restrict__ vec4,
                                                         float *__restrict__ vec1) {
+    pdl_begin();
     const long site = (long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
     if (site >= M) return;
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const double *__restric
                                                          int K, int Kp, int kbeg, int kend,
                                                          float2 *__restrict__ hi,
                                                          float2 *__restrict__ lo) {
+    pdl_begin();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int pairs = (kend - kbeg) / 2;
     if (t >= M * pairs) return;
@@ -158,6 +160,7 @@ __global__ void __launch_bounds__(256) split_bf16_kernel(const double *__restric
                                                          int K, int Kp, int kbeg, int kend,
                                                          __nv_bfloat162 *__restrict__ hi,
                                                          __nv_bfloat162 *__restrict__ lo) {
+    pdl_begin();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int pairs = (kend - kbeg) / 2;
     if (t >= M * pairs) return;
@@ -181,6 +184,7 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const double *__restrict
                                                         int K, int Kp, int kbeg, int kend,
                                                         double scale, __half2 *__restrict__ hi,
                                                         __half2 *__restrict__ lo) {
+    pdl_begin();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int pairs = (kend - kbeg) / 2;
     if (t >= M * pairs) return;
@@ -203,6 +207,7 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const double *__restrict
 __global__ void __launch_bounds__(256) finalize_kernel(const double2 *__restrict__ part,
                                                        int nparts, double scale,
                                                        double *__restrict__ out) {
+    pdl_begin();
     __shared__ double sre[256], sim[256];
     double a = 0.0, b = 0.0;
     for (int k = threadIdx.x; k < nparts; k += 256) {
@@ -230,8 +235,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(const double2 *__restrict
 cudaError_t launch_site_mean(const double *state, long M, int nfile, const double2 *phase,
                              double *mean, float4 *vec4, float *vec1, cudaStream_t st) {
     const unsigned blocks = (unsigned)((M + 7) / 8);
-    site_mean_kernel<<<blocks, 256, 0, st>>>(state, M, nfile, phase, mean, vec4, vec1);
-    return cudaGetLastError();
+    return launch_pdl(site_mean_kernel, blocks, 256, 0, st, state, M, nfile, phase, mean, vec4, vec1);
 }
 
 cudaError_t launch_site_sum(const double *state, long M, int nfile, double *sums,
@@ -255,15 +259,13 @@ cudaError_t launch_split_range(int kind, const double *state, long M, int K, int
     const long total = M * ((kend - kbeg) / 2);
     const unsigned blocks = (unsigned)((total + 255) / 256);
     if (kind == 1)
-        split_tf32_kernel<<<blocks, 256, 0, st>>>(state, M, K, Kp, kbeg, kend, (float2 *)hi,
-                                                  (float2 *)lo);
-    else if (kind == 2)
-        split_bf16_kernel<<<blocks, 256, 0, st>>>(state, M, K, Kp, kbeg, kend,
-                                                  (__nv_bfloat162 *)hi, (__nv_bfloat162 *)lo);
-    else
-        split_f16_kernel<<<blocks, 256, 0, st>>>(state, M, K, Kp, kbeg, kend, scale,
-                                                 (__half2 *)hi, (__half2 *)lo);
-    return cudaGetLastError();
+        return launch_pdl(split_tf32_kernel, blocks, 256, 0, st, state, M, K, Kp, kbeg, kend,
+                          (float2 *)hi, (float2 *)lo);
+    if (kind == 2)
+        return launch_pdl(split_bf16_kernel, blocks, 256, 0, st, state, M, K, Kp, kbeg, kend,
+                          (__nv_bfloat162 *)hi, (__nv_bfloat162 *)lo);
+    return launch_pdl(split_f16_kernel, blocks, 256, 0, st, state, M, K, Kp, kbeg, kend, scale,
+                      (__half2 *)hi, (__half2 *)lo);
 }
 
 cudaError_t launch_split(int kind, const double *state, long M, int K, int Kp, void *hi, void *lo,
@@ -278,8 +280,7 @@ double split_scale(int kind, double spin_len) {
 
 cudaError_t launch_finalize(const double2 *part, int nparts, double scale, double *out,
                             cudaStream_t st) {
-    finalize_kernel<<<1, 256, 0, st>>>(part, nparts, scale, out);
-    return cudaGetLastError();
+    return launch_pdl(finalize_kernel, 1, 256, 0, st, part, nparts, scale, out);
 }
 
 }  // namespace asd

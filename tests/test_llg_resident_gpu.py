@@ -34,10 +34,9 @@ def lib_resident(N, nfile, nsteps, kw):
 @pytest.mark.parametrize("model", range(len(MODELS)))
 @pytest.mark.parametrize("N", [3, 5, 12, 31, 32, 33, 47, 63, 64])
 def test_one_cta_per_replica(oracle, N, model):
-    nfile, nsteps = 30, 12
+    nfile, nsteps = 30 if N <= 33 else 100, 12
     s0, st, launches = lib_resident(N, nfile, nsteps, MODELS[model])
-    if N < 63:
-        assert launches == 1  # otherwise this would not test the resident kernel
+    assert launches == 1  # otherwise this would not test the resident kernel
     want = oracle.steps(orc.make_params(N, nfile, **MODELS[model]), s0, nsteps)
     assert np.array_equal(st, want)
 
@@ -52,7 +51,7 @@ def test_clusters_per_replica(oracle, N, nfile, model):
     assert np.array_equal(st, want)
 
 
-@pytest.mark.parametrize("N,nfile,nsteps", [(8, 1000, 1), (32, 500, 1), (64, 160, 6), (64, 100, 1)])
+@pytest.mark.parametrize("N,nfile,nsteps", [(8, 1000, 3), (32, 500, 1), (64, 160, 6), (64, 100, 1)])
 def test_more_replicas_than_resident_and_single_steps(oracle, N, nfile, nsteps):
     kw = MODELS[1]
     s0, st, launches = lib_resident(N, nfile, nsteps, kw)
