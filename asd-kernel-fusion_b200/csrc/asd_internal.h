@@ -212,12 +212,12 @@ cudaError_t launch_transpose_f64(const double *in, long rows, long cols, double 
 // C[i + j ldc] *= beta for i < m, j < n (beta == 0: set to +0).
 cudaError_t launch_scale_f64(double *c, long m, long n, long ldc, double beta, cudaStream_t st);
 
-// q grid (qgrid.cu): from per-tile diagonal partials tdiag[mb][nb][bm+bn-1][2]
+// q grid (qgrid.cu): from per-tile diagonal partials (pairs hi + lo) tdiag[mb][nb][bm+bn-1][2]
 // of num_m x num_n tiles of bm x bn sites (bn a multiple of bm) to the N*N
 // displacement bins G, in a fixed order; ds holds qgrid_keys() * (bm+bn-1) * 2
 // doubles of work space.
 long qgrid_keys(int num_m, int num_n, int bm, int bn);
-cudaError_t launch_qgrid_bins(const double *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
+cudaError_t launch_qgrid_bins(const float2 *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
                               double *ds, double *G, cudaStream_t st);
 // out[2*(a*N+b)+{0,1}] = scale * sum_d G[d] e^{-2 pi i (a dr + b dc)/N} (qfft.cu); tw: N twiddles
 // (launch_qfft_twiddles), T: N*N of work space.
@@ -278,8 +278,8 @@ struct UmmaSqtArgs {
     int chunk_k = 0;          // K elements per TMEM accumulation chunk (0: all)
     float *dbg_c = nullptr;   // diagnostic: store the accumulator instead
     long dbg_ldc = 0;
-    double *tdiag = nullptr;  // q grid: per-tile diagonal partials
-                              // [Mp/BM][Mp/BN][BM+BN-1][2] (qgrid.cu)
+    float2 *tdiag = nullptr;  // q grid: per-tile diagonal partials, each a pair
+                              // hi + lo, [Mp/BM][Mp/BN][BM+BN-1][2] (qgrid.cu)
     int lat_n = 0;            // lattice side (q grid)
     // K sub-range [k_begin, k_end) in elements (multiples of the k block;
     // k_end = 0: to Kp).  The epilogue applies the connected-part term only

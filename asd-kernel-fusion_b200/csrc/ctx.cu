@@ -91,7 +91,7 @@ struct asd_ctx {
     double *grid_g = nullptr;     // q grid, split modes: N*N displacement bins (FP64)
     double2 *grid_t = nullptr;    // q grid, split modes: DFT intermediate, then N twiddles
     double *grid_out = nullptr;   // q grid: device result for the host-buffer form
-    double *grid_tdiag = nullptr; // q grid: per-tile diagonal partials
+    float2 *grid_tdiag = nullptr; // q grid: per-tile diagonal partials
     size_t grid_tdiag_n = 0;
     double *grid_ds = nullptr;    // q grid: diagonal partials summed by tile key
     size_t grid_ds_n = 0;
@@ -902,7 +902,7 @@ int ensure_grid_work(asd_ctx *c, size_t tdiag_n, size_t ds_n) {
         if (c->grid_tdiag) cudaFree(c->grid_tdiag);
         c->grid_tdiag = nullptr;
         c->grid_tdiag_n = 0;
-        if ((rc = dalloc(&c->grid_tdiag, tdiag_n * sizeof(double))) != ASD_OK) return rc;
+        if ((rc = dalloc(&c->grid_tdiag, tdiag_n * sizeof(float2))) != ASD_OK) return rc;
         c->grid_tdiag_n = tdiag_n;
     }
     if (ds_n > c->grid_ds_n) {

@@ -30,7 +30,7 @@ __device__ __forceinline__ long floordiv(long a, long b) {  // b > 0
     return (a % b != 0 && a < 0) ? q - 1 : q;
 }
 
-__global__ void qgrid_keys_kernel(const double *__restrict__ tdiag, int num_m, int num_n, int bm,
+__global__ void qgrid_keys_kernel(const float2 *__restrict__ tdiag, int num_m, int num_n, int bm,
                                   int bn, double *__restrict__ ds) {
     pdl_begin();
     const int R = bn / bm, nd = bm + bn - 1;
@@ -44,11 +44,14 @@ __global__ void qgrid_keys_kernel(const double *__restrict__ tdiag, int num_m, i
     long mb = kp >= 0 ? kp : ((kp % R) + R) % R;
     const long mb_end = kp + (long)R * num_n;  // nb < num_n
     // consecutive tiles of a key lie a constant distance apart
-    const double *t = tdiag + (mb * num_n + (mb - kp) / R) * nd * 2 + rem;
+    const float2 *t = tdiag + (mb * num_n + (mb - kp) / R) * nd * 2 + rem;
     const long step = ((long)R * num_n + 1) * nd * 2, end = num_m < mb_end ? num_m : mb_end;
     double s = 0.0;
 #pragma unroll 8
-    for (; mb < end; mb += R, t += step) s += *t;
+    for (; mb < end; mb += R, t += step) {
+        const float2 v = *t;
+        s += (double)v.x + (double)v.y;
+    }
     ds[idx] = s;
 }
 
@@ -84,7 +87,7 @@ long qgrid_keys(int num_m, int num_n, int bm, int bn) {
     return num_m + (long)(bn / bm) * (num_n - 1);
 }
 
-cudaError_t launch_qgrid_bins(const double *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
+cudaError_t launch_qgrid_bins(const float2 *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
                               double *ds, double *G, cudaStream_t st) {
     if (bn % bm != 0) return cudaErrorInvalidValue;
     const long n1 = qgrid_keys(num_m, num_n, bm, bn) * (bm + bn - 1) * 2;

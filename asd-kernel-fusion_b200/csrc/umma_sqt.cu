@@ -46,12 +46,12 @@ constexpr uint32_t WAIT_LIMIT = 1u << 24;
 constexpr int GROUP_M = 16;
 // q grid: per warp, a transposition buffer for half a block (32 rows x 16
 // columns FP32, row stride 17) while a tile is binned, then the warp's
-// tile-diagonal partials (5 x 32 x 2 FP64) when it is combined; the two uses
+// tile-diagonal partials (5 x 32 x 2 pairs) when it is combined; the two uses
 // alternate, so they share one region.
 constexpr int GRID_DIAG_M = 5;  // diagonals per lane and warp: 32 m + lane, 5 values of m
 constexpr int GRID_XPOSE = 32 * 17;
 constexpr int GRID_SCRATCH_BYTES = EW * GRID_DIAG_M * 32 * 2 * 8;
-static_assert(GRID_SCRATCH_BYTES >= EW * GRID_XPOSE * 4, "the transposition buffers fit");
+static_assert(GRID_DIAG_M * 32 * 2 * 8 >= GRID_XPOSE * 4, "a warp's two uses share its part");
 constexpr int GRID_ND = BM + BN - 1;  // diagonals r - c of a 128 x 256 tile
 
 // Pipeline geometry: 128 bytes of K per operand row per stage (the 128-byte
@@ -141,6 +141,26 @@ __device__ __forceinline__ uint32_t grid_below_mask(int x0, int thr, int N) {
     return m;
 }
 
+// A sum of floats as an unevaluated pair: each add's rounding error (Knuth's
+// two-sum) goes to lo, so hi + lo carries about 48 bits.  Overflow is that of
+// FP32, as in the block sums that go in; an infinite sum leaves lo NaN, which
+// the reader has to drop (value()).  The q grid's sums over blocks, K chunks and
+// warps are kept so: with FP64 registers in their place the FP16x3 grid took
+// 496 us at 100 x 100 x 240 and 1880 at 128 x 128 x 500, with pairs 388 and 1710
+// (the one-q epilogue: 329 and 1740).  Against the FP64 grid the error is the
+// same to nine digits, from 12 x 12 to 128 x 128 sites in the three modes.
+struct Pair32 {
+    float hi, lo;
+    __device__ __forceinline__ void add(float x) {
+        const float s = hi + x, b = s - hi;
+        lo += (hi - (s - b)) + (x - b);
+        hi = s;
+    }
+    __device__ __forceinline__ float2 value() const {
+        return make_float2(hi, fabsf(hi) <= 3.402823466e38f ? lo : 0.f);
+    }
+};
+
 // val added to the sums whose mask has the step's bit set (one of the four):
 // predicated adds, so no lane branches and each sum sees its values in step
 // order.
@@ -171,55 +191,50 @@ __device__ __forceinline__ void grid_add4(float &pa0, float &pa1, float &pb0, fl
 // step (class 0 iff the row's lattice column x >= a, a = (i - j) mod N of the
 // diagonal) and the diagonal choose one of four sums through four 32-bit masks
 // formed once per block, so a step is a shared load at a fixed offset and one
-// predicated add.
-__device__ __forceinline__ void grid_block(const uint32_t (&v)[32], int c, int lane,
-                                           const float4 &r4, const float4 *z_tab, float alpha,
-                                           bool last, int x_row, int a_first, int N, float *xp,
-                                           double (&ga)[2], double (&gb)[2]) {
-    const float4 *zq = z_tab + c * 32;
-    // diagonal lambda = L of block c: i - j shifted by -32 c from block 0
-    int aa = (a_first - ((32 * c) % N)) % N;
-    if (aa < 0) aa += N;
-    int ab = (aa - (32 % N)) % N;  // lambda = L - 32
-    if (ab < 0) ab += N;
-    const int x0 = __shfl_sync(0xffffffffu, x_row, 0);  // row 32 q + 0
+// predicated add.  The masks of lambda = L - 32 are the next block's of lambda = L
+// (columns 32 further on), so each is formed once.
+struct GridMasks {
+    uint32_t a0, a1, b0, b1;
+};
+__device__ __forceinline__ GridMasks grid_masks(uint32_t below_a, uint32_t below_b, int lane) {
     // class-1 rows: lambda = L on rows l >= L, lambda = L - 32 on rows l < L;
     // rotated right by L so that bit s is the row read at step s
     const uint32_t lowL = (1u << lane) - 1u;
-    const uint32_t cm = (grid_below_mask(x0, aa, N) & ~lowL) | (grid_below_mask(x0, ab, N) & lowL);
-    const uint32_t cbits = __funnelshift_r(cm, cm, lane);
-    const uint32_t bbits = __funnelshift_r(lowL, lowL, lane);  // steps on lambda = L - 32
-    const uint32_t ma0 = ~bbits & ~cbits, ma1 = ~bbits & cbits, mb0 = bbits & ~cbits,
-                   mb1 = bbits & cbits;
+    const uint32_t cm = (below_a & ~lowL) | (below_b & lowL);
+    const uint32_t c = __funnelshift_r(cm, cm, lane);
+    const uint32_t b = __funnelshift_r(lowL, lowL, lane);  // steps on lambda = L - 32
+    return GridMasks{~b & ~c, ~b & c, b & ~c, b & c};
+}
+
+// Half H (columns 16 H .. 16 H + 15) of a block: v the lane's 16 values, z the
+// columns' replica means, p the block's four sums (a0, a1, b0, b1).
+template <int H>
+__device__ __forceinline__ void grid_half(const uint32_t (&v)[16], int lane, const float4 &r4,
+                                          const float4 *z, float alpha, bool last,
+                                          const GridMasks &m, float *xp, float (&p)[4]) {
     float *const wlo = xp + lane * 17, *const whi = wlo + 32 * 17;  // rows l - jj, l - jj + 32
     const float *const row = xp + lane * 17;
-    float pa0 = 0.f, pa1 = 0.f, pb0 = 0.f, pb1 = 0.f;
 #pragma unroll
-    for (int h = 0; h < 32; h += 16) {
-#pragma unroll
-        for (int jj = h; jj < h + 16; ++jj) {
-            float val = alpha * __uint_as_float(v[jj]);
-            if (last) {
-                const float4 z = zq[jj];
-                float o = r4.x * z.x;
-                o = fmaf(r4.y, z.y, o);
-                o = fmaf(r4.z, z.z, o);
-                val -= o;
-            }
-            float *const w = jj > lane ? whi : wlo;
-            w[(jj - h) - 17 * jj] = val;
+    for (int q = 0; q < 16; ++q) {
+        const int jj = 16 * H + q;
+        float val = alpha * __uint_as_float(v[q]);
+        if (last) {
+            const float4 zq = z[jj];
+            float o = r4.x * zq.x;
+            o = fmaf(r4.y, zq.y, o);
+            o = fmaf(r4.z, zq.z, o);
+            val -= o;
         }
-        __syncwarp();
-#pragma unroll
-        for (int s = h; s < h + 16; ++s)
-            grid_add4(pa0, pa1, pb0, pb1, row[s - h], ma0 & (1u << s), ma1 & (1u << s),
-                      mb0 & (1u << s), mb1 & (1u << s));
-        __syncwarp();  // the buffer is free for the next half
+        float *const w = jj > lane ? whi : wlo;
+        w[q - 17 * jj] = val;
     }
-    ga[0] += (double)pa0;
-    ga[1] += (double)pa1;
-    gb[0] += (double)pb0;  // zero in lane 0, which has no lambda = -32
-    gb[1] += (double)pb1;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        const uint32_t bit = 1u << (16 * H + q);
+        grid_add4(p[0], p[1], p[2], p[3], row[q], m.a0 & bit, m.a1 & bit, m.b0 & bit, m.b1 & bit);
+    }
+    __syncwarp();  // the buffer is free for the next half
 }
 
 // KIND: 1 = TF32x3, 2 = BF16x3, 3 = FP16x3.  EPI selects the epilogue:
@@ -233,8 +248,8 @@ __device__ __forceinline__ void grid_block(const uint32_t (&v)[32], int c, int l
 //              warp's 32 rows and 128 columns: a 32 x 32 block of the
 //              accumulator goes through shared memory transposed along its
 //              diagonals, each lane sums its two diagonals of the block in a
-//              fixed order (FP32, at most 32 terms) into FP64 registers, and
-//              the eight warps' registers are combined per tile in warp order.
+//              fixed order (FP32, at most 32 terms) into pairs of floats, and
+//              the eight warps' pairs are combined per tile in warp order.
 //              No atomics: the bins repeat bit for bit.
 constexpr int EPI_PHASE = 0, EPI_STORE = 1, EPI_GRID = 2;
 template <int KIND, int EPI>
@@ -247,7 +262,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                     const float *__restrict__ row1, const float4 *__restrict__ col4,
                     const float *__restrict__ col1, float alpha, double2 *__restrict__ part,
                     unsigned *__restrict__ status, float *__restrict__ dbg_c, long dbg_ldc,
-                    int lat_n, double *__restrict__ tdiag, int group_m) {
+                    int lat_n, float2 *__restrict__ tdiag, int group_m) {
     using G = Geo;
     constexpr bool STORE = (EPI == EPI_STORE);
     constexpr int NHALF = EW / 4;              // warps per TMEM lane quarter
@@ -430,9 +445,36 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
         double tot_re = 0.0, tot_im = 0.0;
         int tcount = 0;
         uint32_t ephase = 0;
-        float *xpose = reinterpret_cast<float *>(gscr) + (warp - 2) * GRID_XPOSE;
-        double *wdiag = reinterpret_cast<double *>(gscr);  // [EW][5][32][2]
-        for (long tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcount) {
+        float2 *wdiag = reinterpret_cast<float2 *>(gscr);  // [EW][5][32][2] (hi, lo)
+        float2 *const wq = wdiag + (warp - 2) * (GRID_DIAG_M * 32 * 2);  // this warp's
+        float *const xpose = reinterpret_cast<float *>(wq);
+        // Column table of a tile (double-buffered by tile: every epilogue warp
+        // finished tile - 2 before it passed the barrier of tile - 1).
+        auto load_table = [&](long tile, int tb) {
+            int mb, nb;
+            tile_coords(tile, num_m, num_n, group_m, mb, nb);
+            const long j0 = (long)nb * BN;
+#pragma unroll
+            for (int h = 0; h < BN / (32 * EW); ++h) {
+                const int jl = etid + 32 * EW * h;
+                const float4 cz = __ldg(&col4[j0 + jl]);
+                tab_w[tb * BN + jl] = make_float2(cz.w, __ldg(&col1[j0 + jl]));
+                tab_z[tb * BN + jl] = make_float4(cz.x, cz.y, cz.z, 0.f);
+            }
+        };
+        auto sync = [&] {
+            if (epilogue_sync(&tail->ebar, ephase, abort_flag)) return true;
+            raise_abort(tail, status);
+            return false;
+        };
+        // q grid: the first tile's table here, each later one's before the
+        // barrier that ends the tile before it
+        bool go = true;
+        if (EPI == EPI_GRID && (long)blockIdx.x < num_tiles) {
+            load_table(blockIdx.x, 0);
+            go = sync();
+        }
+        for (long tile = blockIdx.x; go && tile < num_tiles; tile += gridDim.x, ++tcount) {
             int mb, nb;
             tile_coords(tile, num_m, num_n, group_m, mb, nb);
             const long i = (long)mb * BM + rloc;
@@ -440,39 +482,30 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
             const int tb = tcount & 1;
             float2 *w_tab = tab_w + tb * BN;
             float4 *z_tab = tab_z + tb * BN;
-            if (!STORE) {
-                // Column table of this tile (double-buffered by tile: every
-                // epilogue warp finished tile - 2 before it passed the
-                // barrier of tile - 1).
-#pragma unroll
-                for (int h = 0; h < BN / (32 * EW); ++h) {
-                    const int jl = etid + 32 * EW * h;
-                    const float4 cz = __ldg(&col4[j0 + jl]);
-                    w_tab[jl] = make_float2(cz.w, __ldg(&col1[j0 + jl]));
-                    z_tab[jl] = make_float4(cz.x, cz.y, cz.z, 0.f);
-                }
-                if (!epilogue_sync(&tail->ebar, ephase, abort_flag)) {
-                    raise_abort(tail, status);
-                    break;
-                }
+            if (EPI == EPI_PHASE) {
+                load_table(tile, tb);
+                if (!sync()) break;
             }
             const float4 r4 = STORE ? make_float4(0.f, 0.f, 0.f, 0.f) : row4[i];
             const float ui = STORE ? 0.f : row1[i];
             double s_re = 0.0, s_im = 0.0;
             bool ok = true;
             // q grid: this lane's diagonals d = 32 (quarter - c_first - 4 + mm)
-            // + lane of the tile, both classes; the column of its own row's
-            // site; the columns a = (i - j) mod N of block 0's two diagonals.
-            double gd[GRID_DIAG_M][2];
-            int x_row = 0, a_first = 0;
+            // + lane of the tile, both classes; the lattice column of the warp's
+            // first row; a = (i - j) mod N of its first block's lambda = L, and the
+            // step of a from block to block.
+            Pair32 gd[GRID_DIAG_M][2];
+            int x_first = 0, a_first = 0, n32 = 0;
             if (EPI == EPI_GRID) {
 #pragma unroll
-                for (int mm = 0; mm < GRID_DIAG_M; ++mm) gd[mm][0] = gd[mm][1] = 0.0;
-                x_row = (int)((mb * (long)BM + quarter * 32 + lane) % lat_n);
-                // diagonal d = 32 quarter + lane of block c = 0: i - j = i0 - j0 + d
-                long dl = (long)mb * BM - (long)nb * BN + quarter * 32 + lane;
+                for (int mm = 0; mm < GRID_DIAG_M; ++mm)
+                    gd[mm][0] = gd[mm][1] = Pair32{0.f, 0.f};
+                x_first = (int)((mb * (long)BM + quarter * 32) % lat_n);
+                // diagonal d = 32 quarter + lane - 32 c_first: i - j = i0 - j0 + d
+                long dl = (long)mb * BM - (long)nb * BN + quarter * 32 + lane - 32 * c_first;
                 dl %= lat_n;
                 a_first = (int)(dl < 0 ? dl + lat_n : dl);
+                n32 = 32 % lat_n;
             }
             for (int kb0 = kb_begin; kb0 < kb_end; kb0 += kb_per_chunk) {
                 const bool first = (kb0 == kb_begin);
@@ -487,11 +520,40 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                 ptx::tc_fence_after();
                 // Per 32-column group, in FP32: a = sum_j w_j acc_ij and, in the
                 // last chunk only, o = sum_j w_j (m_i . z_j); the row sum
-                // s_i = alpha * a - o is carried in FP64.  (The q grid unrolls
-                // the groups: its per-lane diagonal registers are indexed by cc.)
-                constexpr int CU = (EPI == EPI_GRID) ? GPH : 1;
-#pragma unroll CU
-                for (int cc = 0; cc < GPH; ++cc) {
+                // s_i = alpha * a - o is carried in FP64.
+                if (EPI == EPI_GRID) {
+                    // half blocks in order, the next one's TMEM load in flight
+                    const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) +
+                                        (uint32_t)(abuf * BN + c_first * 32);
+                    uint32_t v[2][16];
+                    ptx::tmem_ld_32x32b_x16(t0, v[0]);
+                    int a = a_first;  // (i - j) mod N of the block's lambda = L
+                    uint32_t below = grid_below_mask(x_first, a, lat_n);
+#pragma unroll
+                    for (int cc = 0; cc < GPH; ++cc) {
+                        a -= n32;
+                        if (a < 0) a += lat_n;
+                        const uint32_t below_b = grid_below_mask(x_first, a, lat_n);
+                        const GridMasks m = grid_masks(below, below_b, lane);
+                        below = below_b;
+                        const float4 *zq = z_tab + (c_first + cc) * 32;
+                        float p[4] = {0.f, 0.f, 0.f, 0.f};
+                        ptx::tmem_ld_wait();
+                        ptx::tmem_ld_32x32b_x16(t0 + cc * 32 + 16, v[1]);
+                        grid_half<0>(v[0], lane, r4, zq, alpha, last, m, xpose, p);
+                        ptx::tmem_ld_wait();
+                        if (cc + 1 < GPH) ptx::tmem_ld_32x32b_x16(t0 + cc * 32 + 32, v[0]);
+                        grid_half<1>(v[1], lane, r4, zq, alpha, last, m, xpose, p);
+                        // lambda = L: local diagonal GPH - cc; lambda = L - 32 (zero in
+                        // lane 0, which has none): GPH - 1 - cc
+                        gd[GPH - cc][0].add(p[0]);
+                        gd[GPH - cc][1].add(p[1]);
+                        gd[GPH - 1 - cc][0].add(p[2]);
+                        gd[GPH - 1 - cc][1].add(p[3]);
+                    }
+                }
+#pragma unroll 1
+                for (int cc = 0; cc < (EPI == EPI_GRID ? 0 : GPH); ++cc) {
                     const int c = c_first + cc;
                     uint32_t v[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
@@ -503,11 +565,6 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
 #pragma unroll
                         for (int jj = 0; jj < 32; ++jj)
                             dst[jj] = (first ? 0.f : dst[jj]) + __uint_as_float(v[jj]);
-                        continue;
-                    }
-                    if (EPI == EPI_GRID) {
-                        grid_block(v, c, lane, r4, z_tab, alpha, last, x_row, a_first, lat_n,
-                                   xpose, gd[GPH - cc], gd[GPH - 1 - cc]);
                         continue;
                     }
                     const float4 *wq = reinterpret_cast<const float4 *>(w_tab + c * 32);
@@ -550,40 +607,32 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
             }
             if (!ok) break;
             if (EPI == EPI_GRID) {
-                // the warps' diagonals -> tdiag[tile], in warp order; the
-                // shared region served as transposition buffers until now
-                if (!epilogue_sync(&tail->ebar, ephase, abort_flag)) {
-                    raise_abort(tail, status);
-                    break;
-                }
-                double *wq = wdiag + (warp - 2) * (GRID_DIAG_M * 32 * 2);
+                // the warps' diagonals -> tdiag[tile], in warp order; each warp
+                // leaves them where its transposition buffer was
 #pragma unroll
-                for (int mm = 0; mm < GRID_DIAG_M; ++mm) {
-                    wq[(mm * 32 + lane) * 2] = gd[mm][0];
-                    wq[(mm * 32 + lane) * 2 + 1] = gd[mm][1];
-                }
-                if (!epilogue_sync(&tail->ebar, ephase, abort_flag)) {
-                    raise_abort(tail, status);
-                    break;
-                }
-                double *td = tdiag + ((long)mb * num_n + nb) * GRID_ND * 2;
+                for (int mm = 0; mm < GRID_DIAG_M; ++mm)
+                    reinterpret_cast<float4 *>(wq)[mm * 32 + lane] =
+                        make_float4(gd[mm][0].hi, gd[mm][0].lo, gd[mm][1].hi, gd[mm][1].lo);
+                if (!sync()) break;
+                float2 *td = tdiag + ((long)mb * num_n + nb) * GRID_ND * 2;
                 for (int idx = etid; idx < GRID_ND * 2; idx += 32 * EW) {
                     const int d = idx / 2 - (BN - 1), cls = idx & 1;
                     const int L = (d + 256) & 31, m = (d - L) / 32;
-                    double sum = 0.0;
+                    Pair32 sum{0.f, 0.f};
 #pragma unroll
                     for (int w = 0; w < EW; ++w) {
                         // warp 2 + w: quarter (2 + w) % 4, column half w / 4
                         const int mm = m - ((2 + w) & 3) + (w / 4) * GPH + GPH;
-                        if (mm >= 0 && mm < GRID_DIAG_M)
-                            sum += wdiag[((w * GRID_DIAG_M + mm) * 32 + L) * 2 + cls];
+                        if (mm >= 0 && mm < GRID_DIAG_M) {
+                            const float2 t = wdiag[((w * GRID_DIAG_M + mm) * 32 + L) * 2 + cls];
+                            sum.add(t.x);
+                            sum.lo += t.y;
+                        }
                     }
-                    td[idx] = sum;
+                    td[idx] = sum.value();
                 }
-                if (!epilogue_sync(&tail->ebar, ephase, abort_flag)) {
-                    raise_abort(tail, status);
-                    break;
-                }
+                if (tile + gridDim.x < num_tiles) load_table(tile + gridDim.x, tb ^ 1);
+                if (!sync()) break;
             }
             // u_i * s_i with u_i = (r4.w, ui)
             tot_re += (double)r4.w * s_re - (double)ui * s_im;
