@@ -408,8 +408,8 @@ class Context:
                                                C.c_void_p(_addr(d_out))))
 
     def set_llg_kernel(self, kernel) -> None:
-        """"auto" (the default: the one-launch step where the lattice fills the
-        GPU, else the stage kernels), "fused" (one launch per step) or
+        """"auto" (the default: the fastest of the resident steps, the one-launch
+        step and the stage kernels for the sizes), "fused" (one launch per step) or
         "stages" (four launches, one per RK4 stage)."""
         k = {"fused": LLG_FUSED_STEP, "stages": LLG_STAGES, "auto": LLG_AUTO}.get(kernel, kernel)
         _check(load().asd_ctx_set_llg_kernel(self._h, int(k)))
@@ -422,12 +422,12 @@ class Context:
 
     def time_kernels(self, on: bool = True) -> None:
         """asd_ctx_time_kernels: record CUDA events around the RK4 step kernels
-        and the S(q,t) GEMM on the stream each is launched on."""
+        and each S(q,t) evaluation's main pass on the stream each is launched on."""
         _check(load().asd_ctx_time_kernels(self._h, int(bool(on))))
 
     def kernel_time(self, which: str):
         """asd_ctx_kernel_time: (total ms, launches) of the timed RK4 step
-        kernels ("llg") or S(q,t) GEMMs ("gemm") since the last read."""
+        kernels ("llg") or S(q,t) main passes ("gemm") since the last read."""
         ms = C.c_double(0.0)
         n = C.c_int(0)
         _check(load().asd_ctx_kernel_time(self._h, {"llg": 0, "gemm": 1}[which], C.byref(ms),

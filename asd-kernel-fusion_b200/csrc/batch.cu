@@ -1,9 +1,11 @@
 // batch.cu -- many independent lattices of different sizes and parameters in
 // one persistent launch.  The reference runs one lattice per program; this is
 // the B200 form of running an ensemble of them (e.g. different temperatures
-// and dampings): all lattices' spins stay resident in L2 (FP32, a few MB),
-// one cooperative kernel runs every RK4 step of every lattice, and a bounded
-// grid barrier separates the four stages of a step.
+// and dampings).  Where the batch fits, each lattice stays in the shared memory
+// of one thread-block cluster for all steps (batch_cluster_kernel, below).
+// Otherwise all lattices' spins stay resident in L2 (FP32, a few MB), one
+// cooperative kernel runs every RK4 step of every lattice, and a bounded grid
+// barrier separates the four stages of a step.
 //
 // Arithmetic: the RK4 stages in FP32 with explicitly rounded operations in the
 // reference's order (euler / runge_kutta, llg_sqt_baseline.c:29-142), the
@@ -12,8 +14,8 @@
 // for bit.
 //
 // Layout: lattice l occupies planes x, y, z of N_l * N_l floats at offset
-// off_l (structure of arrays, one replica per lattice).  Work items are tiles
-// of `tile` consecutive sites of one lattice; CTA b processes items b,
+// off_l (structure of arrays, one replica per lattice).  In the L2 form work
+// items are tiles of `tile` consecutive sites of one lattice; CTA b processes items b,
 // b + grid, ...  The tile width and the CTAs per SM come from the autotuner.
 #include <cooperative_groups.h>
 

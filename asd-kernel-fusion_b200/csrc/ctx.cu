@@ -5,9 +5,10 @@
 // stream.  Device memory (site-major FP64 spins, M = N*N sites,
 // K = 3*nfile values per site):
 //   y, ys_a, ys_b, acc   RK4 state, stage inputs, running combination  4*M*K
-//   origin               the t = 0 snapshot (B of the GEMM)               M*K
+//   origin               the t = 0 snapshot (B of the product)            M*K
 //   a/b hi/lo            split operands, [Mp][Kp] per enabled split kind
-//   q-grid work          per-tile diagonal partials (on the first q grid)
+//   q-grid work          split modes: per-tile diagonal partials (on the first
+//                        q grid); FP64: the transforms lie in ys_a, ys_b, acc
 // The AoS <-> site-major transposes stage through ys_b.
 
 #include <algorithm>

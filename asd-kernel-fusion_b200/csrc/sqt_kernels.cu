@@ -1,6 +1,6 @@
 // sqt_kernels.cu -- the memory-bound pieces around the S(q,t) correlation
-// GEMM: replica means, operand splitting, the FP64 phase epilogue of the
-// plain path, and the deterministic final reduction.
+// GEMM: replica means, operand splitting, the transposes to and from the
+// site-major layout, and the deterministic final reduction.
 //
 // S(q,t) = (1/M) sum_ij u_i w_j (C_ij - m_i . z_j),  C = (1/nfile) A B^T,
 // with u_i = e^{-i q.r_i}, w_j = e^{+i q.r_j} (so u_i w_j is the reference's

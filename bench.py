@@ -61,7 +61,8 @@ DEFAULT_CHUNK_K = {"tf32x3": 512, "bf16x3": 1024, "fp16x3": 1024}
 
 
 def llg_fp64_ops(J2: bool, H: bool, damp: bool) -> int:
-    """FP64 operations of one site-step as the kernels write them (add, sub,
+    """FP64 operations of one site-step as the reference orders them (at |J1| = 1
+    the kernels leave out the products by it, which are exact) (add, sub,
     mul and fma 1 each; a division or square root 1 each, although the
     hardware runs a short sequence for them): the right-hand side (exchange
     12 mul + 12 add, J2 as much again, the field 3 add, H x S 9, damping 18)
@@ -800,7 +801,7 @@ def run_secondary(args):
         ctx.close()
     elif args.workload == "grid32":
         # 32x32 lattice, 200 replicas, J=1, alpha=0.1, dt=0.01, 2000 RK4 steps, S(q,t) on the
-        # whole 32x32 q grid after every step (FP64 GEMM + displacement bins + 2-D DFT)
+        # whole 32x32 q grid after every step (2-D transforms of the spins, FP64)
         N, nf, nsteps = 32, 200, 2000
         M = N * N
         ctx = asd.Context(asd.Params.make(N, nf, J1=1.0, alpha=0.1, dt=0.01), modes=["fp64"])

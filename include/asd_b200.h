@@ -22,7 +22,7 @@
  *
  *  2. A context API (asd_ctx_*) that keeps the replicas' spins resident in
  *     HBM and runs a whole step on one CUDA stream: the RK4 step with its
- *     renormalisation (one launch, or one kernel per stage), then S(q,t)
+ *     renormalisation (resident, one launch, or one kernel per stage), then S(q,t)
  *     through a tcgen05 tensor-core GEMM in split precision (TF32x3,
  *     BF16x3 or FP16x3) whose epilogue applies the phase, the connected-part
  *     subtraction and the reduction, or through the FP64 path.  It replaces
@@ -305,7 +305,7 @@ int asd_ctx_check_device_status(asd_ctx *ctx);
 /* Diagnostic, host-side fault injection: the n-th device allocation of the
  * context API from now on (asd_ctx_create and the calls that allocate work
  * space on first use: host-buffer steps, the q grid, the adjoint, the FP64
- * partials) fails as cudaMalloc does on a full device, so the call returns
+ * work spaces) fails as cudaMalloc does on a full device, so the call returns
  * ASD_ERR_NOMEM and frees what it had taken; n = 0 switches it off.  Process
  * wide.  No counterpart in the reference (which never checks an allocation);
  * the failure-path tests use it. */
@@ -314,7 +314,7 @@ int asd_debug_fail_alloc(long n);
 /* Diagnostic: waits until the context is idle, then fills with NaN bytes
  * (0xFF) every device buffer of the context whose contents do not carry over
  * between calls (stage states, the running RK4 combination, replica means at
- * t, the FP64 band, GEMM partials and result, q-grid bins, host-step staging,
+ * t, the phase sums, GEMM partials and result, q-grid bins, host-step staging,
  * the adjoint's state-sized work buffers).  A kernel that read any of them
  * before writing it would show NaN or changed results.  The spins, the
  * origin, the phases, the epilogue vectors and the split operands are kept.
