@@ -663,46 +663,46 @@ __global__ void __launch_bounds__(resident::threads(W), resident::ctas_per_sm(W)
 }
 
 // Tiled transpose between [nfile][M][3] and [M][nfile][3] through shared
-// memory: 32 sites x 32 replicas x 3 doubles per block.
+// memory: 32 sites x 32 replicas x 3 doubles per block.  Bound by HBM: a thread
+// keeps one of a row's 96 doubles, so its 16 rows are a constant stride apart
+// and all its loads are in flight at once; rows of 99 doubles (3 mod 16) make
+// the transposed reads free of bank conflicts.  Measured on B200, site-major to
+// AoS, against 256 threads with a division per element and rows of 97:
+// 128x128x500 94 -> 63.5 us (6.2 TB/s), 256x256x1000 689 -> 502, 64x64x100 8.5 -> 6.2.
+constexpr int TR_THREADS = 192, TR_ROWS = TR_THREADS / 96, TR_N = 32 / TR_ROWS;
 template <bool TO_SITEMAJOR>
-__global__ void __launch_bounds__(256) transpose_kernel(const double *__restrict__ src,
-                                                        double *__restrict__ dst, long M,
-                                                        int nfile, int fbeg, int nc) {
+__global__ void __launch_bounds__(TR_THREADS) transpose_kernel(const double *__restrict__ src,
+                                                               double *__restrict__ dst, long M,
+                                                               int nfile, int fbeg, int nc) {
     pdl_begin();
     // The AoS side holds replicas [fbeg, fbeg + nc) as [nc][M][3]; the
-    // site-major side is the whole [M][nfile][3] array.  lf = local replica.
-    __shared__ double tile[32][32 * 3 + 1];
+    // site-major side is the whole [M][nfile][3] array.
+    __shared__ double tile[32][32 * 3 + 3];
     const long s0 = (long)blockIdx.x * 32;
     const int l0 = blockIdx.y * 32;
-    // read
-    for (int idx = threadIdx.x; idx < 32 * 96; idx += blockDim.x) {
-        const int r = idx / 96, w = idx % 96;
-        if (TO_SITEMAJOR) {
-            // AoS: for replica l0+r, 96 contiguous doubles of sites s0..s0+31
-            const int lf = l0 + r;
-            const long s = s0 + w / 3;
-            if (lf < nc && s < M) tile[r][w] = src[((long)lf * M + s0) * 3 + w];
-        } else {
-            // site-major: for site s0+r, 96 contiguous doubles of replicas l0..l0+31
-            const long s = s0 + r;
-            const int lf = l0 + w / 3;
-            if (lf < nc && s < M) tile[r][w] = src[(s * nfile + fbeg + l0) * 3 + w];
-        }
+    const int w = threadIdx.x % 96, r0 = threadIdx.x / 96, q = w / 3, c = w - 3 * q;
+    const int ns = (int)min(32L, M - s0), nl = min(32, nc - l0);  // sites, replicas here
+    // 96 contiguous doubles a row: sites of a replica, replicas of a site
+    const long aos = ((long)l0 * M + s0) * 3 + w, sm = (s0 * nfile + fbeg + l0) * 3 + w;
+    const long aos_row = 3 * M, sm_row = 3L * nfile;
+    const double *p = src + (TO_SITEMAJOR ? aos : sm);
+    double *o = dst + (TO_SITEMAJOR ? sm : aos);
+    const long prow = TO_SITEMAJOR ? aos_row : sm_row, orow = TO_SITEMAJOR ? sm_row : aos_row;
+    const int prows = q < (TO_SITEMAJOR ? ns : nl) ? (TO_SITEMAJOR ? nl : ns) : 0;
+    const int orows = q < (TO_SITEMAJOR ? nl : ns) ? (TO_SITEMAJOR ? ns : nl) : 0;
+    double x[TR_N];
+#pragma unroll
+    for (int t = 0; t < TR_N; ++t) {
+        const int r = r0 + TR_ROWS * t;
+        x[t] = r < prows ? p[r * prow] : 0.0;
     }
+#pragma unroll
+    for (int t = 0; t < TR_N; ++t) tile[r0 + TR_ROWS * t][w] = x[t];
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 32 * 96; idx += blockDim.x) {
-        const int r = idx / 96, w = idx % 96;
-        const int c = w % 3, q = w / 3;
-        if (TO_SITEMAJOR) {
-            // write site s0+r, replicas l0..: value from tile[lf-l0][(s-s0)*3+c]
-            const long s = s0 + r;
-            const int lf = l0 + q;
-            if (lf < nc && s < M) dst[(s * nfile + fbeg + lf) * 3 + c] = tile[q][r * 3 + c];
-        } else {
-            const int lf = l0 + r;
-            const long s = s0 + q;
-            if (lf < nc && s < M) dst[((long)lf * M + s) * 3 + c] = tile[q][r * 3 + c];
-        }
+#pragma unroll
+    for (int t = 0; t < TR_N; ++t) {
+        const int r = r0 + TR_ROWS * t;
+        if (r < orows) o[r * orow] = tile[q][r * 3 + c];
     }
 }
 
@@ -931,14 +931,14 @@ cudaError_t launch_aos_to_sitemajor_range(const double *aos, double *sm, long M,
                                           int f0, int nc, cudaStream_t st) {
     if (f0 < 0 || nc < 1 || f0 + nc > nfile) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((M + 31) / 32), (unsigned)((nc + 31) / 32));
-    return launch_pdl(transpose_kernel<true>, grid, 256, 0, st, aos, sm, M, nfile, f0, nc);
+    return launch_pdl(transpose_kernel<true>, grid, TR_THREADS, 0, st, aos, sm, M, nfile, f0, nc);
 }
 
 cudaError_t launch_sitemajor_to_aos_range(const double *sm, double *aos, long M, int nfile,
                                           int f0, int nc, cudaStream_t st) {
     if (f0 < 0 || nc < 1 || f0 + nc > nfile) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((M + 31) / 32), (unsigned)((nc + 31) / 32));
-    return launch_pdl(transpose_kernel<false>, grid, 256, 0, st, sm, aos, M, nfile, f0, nc);
+    return launch_pdl(transpose_kernel<false>, grid, TR_THREADS, 0, st, sm, aos, M, nfile, f0, nc);
 }
 
 cudaError_t launch_aos_to_sitemajor(const double *aos, double *sm, long M, int nfile,
