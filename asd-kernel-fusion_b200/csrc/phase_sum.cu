@@ -12,14 +12,16 @@
 //
 // phase_sum_kernel is bound by HBM: it reads A once (8 M K bytes), a thread
 // per column pair (16-byte loads; one column and 8 bytes where K is odd), a
-// block walking `rows` sites.  phase_value_kernel sums the blocks' partials
+// block walking `rows` sites, 16 loads in flight.  phase_value_kernel sums the blocks' partials
 // per column, forms the products and the final sum; its last block to finish
 // adds the block sums.  Every sum runs in a fixed order.
 //
 // Measured on B200, one RK4 step, one S(q,t) and the spins' read-out at
 // 128x128x500: 26.36 ms with the FP64 tensor-core GEMM (25.85 ms of it) that
 // served the FP64 mode before, 0.548 ms with these sums; four S(q,t) and 20
-// steps at 51x51x70: 1.150 -> 0.668 ms.  Relative difference of the values
+// steps at 51x51x70: 1.150 -> 0.668 ms.  S(q,t) alone, 8 -> 16 loads in flight,
+// 8 -> 16 slices and shorter chunks: 128x128x500 70 -> 40 us, 256x256x1000 294 ->
+// 245 (6.4 TB/s), 100x100x240 23 -> 14, 64x64x100 17 -> 10.  Relative difference of the values
 // 1.5e-16, their error against a 64-bit reference 1.7e-16 (before 2.2e-16).
 #include "asd_internal.h"
 
@@ -27,7 +29,7 @@ namespace asd {
 namespace {
 
 constexpr int PS_THREADS = 128;
-constexpr int PV_K = 32, PV_SLICES = 8;  // columns per value block, slices of the chunk sum
+constexpr int PV_K = 32, PV_SLICES = 16;  // columns per value block, slices of the chunk sum
 
 template <int VEC>
 __global__ void __launch_bounds__(PS_THREADS) phase_sum_kernel(const double *__restrict__ A, long M,
@@ -43,7 +45,7 @@ __global__ void __launch_bounds__(PS_THREADS) phase_sum_kernel(const double *__r
 #pragma unroll
     for (int v = 0; v < VEC; ++v) re[v] = im[v] = 0.0;
     const double *p = A + i0 * K + k;
-#pragma unroll 8
+#pragma unroll 16
     for (long i = i0; i < i1; ++i, p += K) {
         double x[VEC];
         if (VEC == 2) {
@@ -77,7 +79,7 @@ __device__ __forceinline__ bool last_block(unsigned *count) {
     return s_last != 0;
 }
 
-// Sum of v over the block's 256 threads, a tree of fixed order.
+// Sum of v over the block's 512 threads, a tree of fixed order.
 __device__ __forceinline__ double2 block_sum(double2 v) {
     __shared__ double2 red[PV_K * PV_SLICES];
     red[threadIdx.x] = v;
@@ -94,15 +96,15 @@ __device__ __forceinline__ double2 block_sum(double2 v) {
     return r;
 }
 
-// F_k of 32 columns from the chunk partials: slice s adds chunks s, s + 8, ...
-// and the slices are added in order; valid in the threads of slice 0.
+// F_k of 32 columns from the chunk partials: slice s adds chunks s, s + 16,
+// ... and the slices are added in order; valid in the threads of slice 0.
 __device__ __forceinline__ double2 column_sum(const double2 *__restrict__ Fpart, int nchunks, int K,
                                               int k) {
     __shared__ double2 red[PV_SLICES][PV_K];
     const int kl = threadIdx.x % PV_K, sl = threadIdx.x / PV_K;
     double2 f = make_double2(0.0, 0.0);
     if (k < K) {
-#pragma unroll 4
+#pragma unroll 16
         for (int c = sl; c < nchunks; c += PV_SLICES) {
             const double2 t = Fpart[(long)c * K + k];
             f.x += t.x;
@@ -183,11 +185,14 @@ __global__ void __launch_bounds__(PV_K *PV_SLICES) phase_value_kernel(
     }
 }
 
-// Rows per chunk: 256, halved (down to 16) until the grid has at least four
-// blocks per SM of a B200, so that small lattices still fill the GPU; doubled
-// where the chunks would exceed the grid's y extent (N = 4096).
+// Rows per chunk: 256, halved (down to 16) until the grid has at least six
+// blocks per SM of a B200, so that the blocks' last round is a small part of the
+// whole and small lattices still fill the GPU; doubled where the chunks would
+// exceed the grid's y extent (N = 4096).  Measured with at least 2 / 4 / 6 / 9
+// blocks per SM: 79 / 51 / 41 / 41 us at 128x128x500, 14 / 17 / 15 / 19 at
+// 100x100x240 (more chunks cost the value kernel), 20 / 20 / 20 / 20 at 160x160x9.
 int chunk_rows(long M, int K) {
-    constexpr long kMinBlocks = 4 * 148;
+    constexpr long kMinBlocks = 6 * 148;
     const int cols = PS_THREADS * (K % 2 == 0 ? 2 : 1);
     const long kb = (K + cols - 1) / cols;
     int rows = 256;
