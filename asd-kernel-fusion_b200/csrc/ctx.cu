@@ -432,8 +432,9 @@ DmmaSqtArgs dmma_args(const asd_ctx *c) {
 PhaseWork phase_ws(const asd_ctx *c) { return phase_work(c->phase_ws, c->M, c->K); }
 
 // The work space of the phase sums, and the origin's column sums up to date
-// (formed once per origin and q).
-int ensure_phase_origin(asd_ctx *c) {
+// (formed once per origin and q; a captured call forms them itself, as its
+// replays may follow other origins, and leaves the version of the sums alone).
+int ensure_phase_work(asd_ctx *c) {
     int rc;
     if (!c->phase_ws) {
         const size_t n = phase_work_bytes(c->M, c->K);
@@ -447,10 +448,17 @@ int ensure_phase_origin(asd_ctx *c) {
     }
     if (!c->phase_G && (rc = dalloc(&c->phase_G, ((size_t)c->K + 3) * sizeof(double2))) != ASD_OK)
         return rc;
-    if (c->g_version == c->origin_version) return ASD_OK;
+    return ASD_OK;
+}
+
+int ensure_phase_origin(asd_ctx *c) {
+    const int rc = ensure_phase_work(c);
+    if (rc != ASD_OK) return rc;
+    const bool capturing = stream_capturing(c->stream);
+    if (!capturing && c->g_version == c->origin_version) return ASD_OK;
     ASD_CUDA_TRY(launch_phase_origin(c->origin, c->M, c->K, c->p.nfile, c->wphase, phase_ws(c),
                                      c->phase_G, c->phase_G + c->K, c->stream));
-    c->g_version = c->origin_version;
+    if (!capturing) c->g_version = c->origin_version;
     c->last_launches += 2;
     return ASD_OK;
 }
@@ -1412,6 +1420,12 @@ int asd_ctx_create(const asd_params *p, unsigned mode_mask, asd_ctx **out) {
     if (e != cudaSuccess) {
         destroy(c);
         return cuda_fail(e, "cudaMallocHost");
+    }
+    // Small lattices take the phase sums' work space here (a small part of a
+    // state array), so that their first FP64 S(q,t) can be captured into a graph.
+    if (dmma_sqt_tiles(c->M) <= c->num_sms && (rc = ensure_phase_work(c)) != ASD_OK) {
+        destroy(c);
+        return rc;
     }
     // Phases u_i = e^{-i q.r_i} and w_j = e^{+i q.r_j}, q = 2 pi (vx, vy) / N
     // (llg_sqt_baseline.c:267-268), so that u_i w_j = e^{-i q.(r_i - r_j)}.
