@@ -382,7 +382,11 @@ int run_steps(asd_ctx *c, int nsteps) {
         c->state_version += nsteps;
         return ASD_OK;
     }
-    if (use_fused(c, c->a)) {
+    // A captured odd number of one-launch steps would leave its replays reading
+    // the same buffer again, so while the stream is captured the default takes
+    // them only on lattices that fill the GPU with rows.
+    if (use_fused(c, c->a) && (c->llg_kernel != ASD_LLG_AUTO || llg_fused_fills(c->a) ||
+                               !stream_capturing(c->stream))) {
         for (int s = 0; s < nsteps; ++s) {
             cudaEvent_t t0 = time_begin(c, c->stream);
             ASD_CUDA_TRY(launch_llg_step_fused(c->a, c->y, c->ys_a, c->stream));

@@ -2,7 +2,8 @@
 last replay left the spins, and S(q,t) is that of the state and the origin at the
 time of the replay, bit for bit what the same calls give one by one.  Sizes: S(q,t)
 in FP64 captured as the first call on a small lattice, resident steps of one SM and
-of a cluster."""
+of a cluster, stage kernels, and lattices whose uncaptured steps alternate between
+two buffers."""
 from __future__ import annotations
 
 import numpy as np
@@ -28,7 +29,8 @@ def eager(N, nfile, s0, origin, replays, nsteps):
     return out
 
 
-@pytest.mark.parametrize("N,nfile,nsteps", [(12, 16, 1), (32, 40, 3), (64, 20, 2), (100, 24, 4)])
+@pytest.mark.parametrize("N,nfile,nsteps", [(12, 16, 1), (32, 40, 3), (64, 20, 2), (100, 24, 4),
+                                            (160, 4, 1), (160, 16, 1), (128, 30, 1), (256, 8, 1)])
 def test_replayed_steps_and_sqt(N, nfile, nsteps):
     a, b = (asd.random_spins(N, nfile, seed=N + k) for k in (0, 1))
     stream = torch.cuda.Stream()
