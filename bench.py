@@ -167,6 +167,12 @@ def env_rank():
             int(os.environ.get("LOCAL_RANK", "0")))
 
 
+def compute_dtype(mode: str) -> str:
+    if mode == "fp64":
+        return "f64 RK4 + f64 phase sums"
+    return f"f64 RK4 + {mode} GEMM (fp32 accumulate, f64 reduction)"
+
+
 def bench_config(name: str, args) -> dict:
     """The workload description both arms print, key for key."""
     w = WORKLOADS[name]
@@ -525,7 +531,7 @@ def run_ours(args):
         "metric": METRIC, "value": value, "unit": "site-steps/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None,
-        "dtype": f"f64 RK4 + {mode} GEMM (fp32 accumulate, f64 reduction)",
+        "dtype": compute_dtype(mode),
         "data": "synthetic: seeded spins uniform on the sphere",
         "config": bench_config(name, args),
         "roofline": roofline,
@@ -973,7 +979,7 @@ def run_sharded(args):
         "metric": METRIC, "value": value, "unit": "site-steps/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
         "scaling": "strong", "vs_baseline": None,
-        "dtype": f"f64 RK4 + {mode} GEMM (fp32 accumulate, f64 reduction)",
+        "dtype": compute_dtype(mode),
         "data": "synthetic: seeded spins uniform on the sphere",
         "config": {**bench_config(args.workload, args),
                    "workload": w["desc"] + ", one ensemble split by replicas",
