@@ -14,7 +14,7 @@
 //
 // Tiles with the same key k = mb - (bn / bm) nb have the same i - j on each
 // diagonal: delta = k bm + d.  So the bins follow in two fixed-order passes:
-//   keys: ds[k][d][cls] = sum over the tiles of key k (mb ascending)
+//   keys: ds[k][d][cls] = sum over the tiles of key k (slices of them, mb ascending)
 //   bins: G(dr, dc) = sum over the (delta, cls) that land there (at most 4)
 //         and over the keys whose tiles hold that delta (ascending)
 // with no atomics: the bins repeat bit for bit.
@@ -30,28 +30,41 @@ __device__ __forceinline__ long floordiv(long a, long b) {  // b > 0
     return (a % b != 0 && a < 0) ? q - 1 : q;
 }
 
-__global__ void qgrid_keys_kernel(const float2 *__restrict__ tdiag, int num_m, int num_n, int bm,
-                                  int bn, double *__restrict__ ds) {
+// A thread takes every KEY_SLICES-th tile of a key, and the slices are added in
+// order: a key has up to min(num_m / R, num_n) tiles, a serial chain of L2 loads.
+// At 100 x 100 (79 x 40 tiles) 25.7 -> 11.5 us against one thread a sum.
+constexpr int KEY_X = 64, KEY_SLICES = 4;
+__global__ void __launch_bounds__(KEY_X *KEY_SLICES)
+    qgrid_keys_kernel(const float2 *__restrict__ tdiag, int num_m, int num_n, int bm, int bn,
+                      double *__restrict__ ds) {
     pdl_begin();
+    __shared__ double red[KEY_SLICES][KEY_X];
+    const int x = threadIdx.x % KEY_X, slice = threadIdx.x / KEY_X;
     const int R = bn / bm, nd = bm + bn - 1;
     const long nkeys = num_m + (long)R * (num_n - 1);
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nkeys * nd * 2) return;
+    const long n = nkeys * nd * 2, want = (long)blockIdx.x * KEY_X + x;
+    const long idx = want < n ? want : n - 1;  // every thread reaches the barrier
     const long key = idx / (nd * 2);
     const int rem = (int)(idx - key * nd * 2);  // d index * 2 + class
     const long kp = key - (long)R * (num_n - 1);  // mb - R nb
     // tiles: mb = kp (mod R), 0 <= mb < num_m, 0 <= nb = (mb - kp) / R < num_n
-    long mb = kp >= 0 ? kp : ((kp % R) + R) % R;
+    const long mb0 = kp >= 0 ? kp : ((kp % R) + R) % R;
     const long mb_end = kp + (long)R * num_n;  // nb < num_n
     // consecutive tiles of a key lie a constant distance apart
-    const float2 *t = tdiag + (mb * num_n + (mb - kp) / R) * nd * 2 + rem;
+    const float2 *t = tdiag + (mb0 * num_n + (mb0 - kp) / R) * nd * 2 + rem;
     const long step = ((long)R * num_n + 1) * nd * 2, end = num_m < mb_end ? num_m : mb_end;
     double s = 0.0;
-#pragma unroll 8
-    for (; mb < end; mb += R, t += step) {
+    t += slice * step;
+#pragma unroll 4
+    for (long mb = mb0 + slice * R; mb < end; mb += R * KEY_SLICES, t += step * KEY_SLICES) {
         const float2 v = *t;
         s += (double)v.x + (double)v.y;
     }
+    red[slice][x] = s;
+    __syncthreads();
+    if (slice || want >= n) return;
+#pragma unroll
+    for (int k = 1; k < KEY_SLICES; ++k) s += red[k][x];
     ds[idx] = s;
 }
 
@@ -91,8 +104,8 @@ cudaError_t launch_qgrid_bins(const float2 *tdiag, int num_m, int num_n, int bm,
                               double *ds, double *G, cudaStream_t st) {
     if (bn % bm != 0) return cudaErrorInvalidValue;
     const long n1 = qgrid_keys(num_m, num_n, bm, bn) * (bm + bn - 1) * 2;
-    const cudaError_t e = launch_pdl(qgrid_keys_kernel, (unsigned)((n1 + 255) / 256), 256, 0, st,
-                                     tdiag, num_m, num_n, bm, bn, ds);
+    const cudaError_t e = launch_pdl(qgrid_keys_kernel, (unsigned)((n1 + KEY_X - 1) / KEY_X),
+                                     KEY_X * KEY_SLICES, 0, st, tdiag, num_m, num_n, bm, bn, ds);
     if (e != cudaSuccess) return e;
     const long n2 = (long)lat_n * lat_n;
     return launch_pdl(qgrid_bins_kernel, (unsigned)((n2 + 255) / 256), 256, 0, st, ds, num_m, num_n,

@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(256) site_mean_kernel(const double *__restrict
     if (site >= M) return;
     const double *p = state + site * 3L * nfile;
     double sx = 0.0, sy = 0.0, sz = 0.0;
+#pragma unroll 4
     for (int f = lane; f < nfile; f += 32) {
         sx += p[3 * f];
         sy += p[3 * f + 1];
