@@ -180,12 +180,12 @@ cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *upha
 // ------------------------------------- FP64 S(q,t) on the q grid (qfft.cu)
 // out[2 (a N + b)] = scale * sum_k A~_k conj(B~_k) at q = 2 pi (a, b) / N, the
 // transforms of A - m and B - z (m, z [M][3]); work: qfft_work_bytes, its first
-// N complex values written once by launch_qfft_twiddles; scratch: three buffers
+// N complex values written once by launch_qfft_twiddles; scratch: two buffers
 // of M K doubles.  Returns the number of launches or a negative error.
 size_t qfft_work_bytes(int lat_n, int K);
 cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st);
 int launch_qfft(const double *A, const double *B, int lat_n, int K, const double *m,
-                const double *z, double scale, void *work, double *const scratch[3], double *out,
+                const double *z, double scale, void *work, double *const scratch[2], double *out,
                 cudaStream_t st);
 
 // ------------------------------------------------- FP64 tensor-core GEMM

@@ -8,7 +8,7 @@
 //   origin               the t = 0 snapshot (B of the product)            M*K
 //   a/b hi/lo            split operands, [Mp][Kp] per enabled split kind
 //   q-grid work          split modes: per-tile diagonal partials (on the first
-//                        q grid); FP64: the transforms lie in ys_a, ys_b, acc
+//                        q grid); FP64: the transforms lie in ys_b and acc
 // The AoS <-> site-major transposes stage through ys_b.
 
 #include <algorithm>
@@ -955,7 +955,9 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
                                       c->row1, c->stream));
         c->rows_ready = true;
         c->last_launches += 1;
-        double *const scratch[3] = {c->ys_a, c->ys_b, c->acc};  // RK4 state only within a step
+        // RK4 state only within a step; not ys_a, which the one-launch step swaps
+        // with y: where this call is captured, a replay may find the spins there
+        double *const scratch[2] = {c->ys_b, c->acc};
         rc = launch_qfft(c->y, c->origin, N, c->K, c->mean_t, c->mean_0,
                          1.0 / ((double)M * c->p.nfile), c->grid_fft, scratch, d_out, c->stream);
         if (rc < 0) return rc;

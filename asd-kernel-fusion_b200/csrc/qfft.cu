@@ -13,7 +13,10 @@
 // About 5 M log2(M) operations per column instead of 2 M^2.
 //
 // Columns go in chunks whose transform (16 M bytes a column) stays in L2, held
-// in the context's RK4 scratch (no memory of their own):
+// in two buffers of the context's RK4 scratch (the caller leaves out the one that
+// the one-launch step alternates with the state, as a captured call's replays may
+// find the state in it) and, for the last blocks of a lattice whose columns make
+// one chunk, in a small one of their own:
 //   qfft_rows_kernel  a block takes one lattice row of KC columns, transforms
 //                     along it in shared memory, writes X[r][b][columns]
 //   qfft_cols_kernel  a block takes the lattice columns b and N - b of up to
@@ -192,15 +195,16 @@ __global__ void qfft_twiddle_kernel(int n, double2 *__restrict__ tw) {
     tw[j] = make_double2(cs, -sn);
 }
 
-// The transforms of a chunk's blocks of KC columns: block kb in buffer
-// kb / per, as [n][n][width] with width = the blocks there (at most per) * KC.
+// The transforms of a chunk's blocks of KC columns: `per` blocks in each of the
+// first two buffers, the rest in the third, each as [n][n][width] with width = the
+// blocks there * KC.
 struct Chunk {
     double2 *buf[3];
     int blocks, per;
     // column k of the chunk
     __device__ __forceinline__ double2 *at(int k, int lk, int &width) const {
-        const int q = (k >> lk) / per, first = q * per;
-        width = min(per, blocks - first) << lk;
+        const int q = min(2, (k >> lk) / per), first = q * per;
+        width = (q == 2 ? blocks - first : min(per, blocks - first)) << lk;
         return buf[q] + (k - (first << lk));
     }
 };
@@ -394,6 +398,7 @@ int threads_for(int points) {
 struct Geometry {
     int per;     // blocks of KC columns a scratch buffer holds
     int blocks;  // blocks per chunk
+    int own;     // of those, in the third buffer (0 to 2)
     int slices;  // sums over k kept apart
 };
 
@@ -403,8 +408,12 @@ Geometry geometry(const FftPlan &p, int K) {
     g.per = K / (2 * kc);
     long b = (48L << 20) / (16L * p.n * p.n * kc);  // the chunk's transform stays in L2
     if (b < 1) b = 1;
-    if (b > 3L * g.per) b = 3L * g.per;
-    g.blocks = b < all ? (int)b : all;
+    // two buffers hold all blocks but the odd one or two: those, where that makes
+    // one chunk of the lattice (32x32x200: 75 blocks of 8 columns, 37 a buffer)
+    if (b >= all) b = all;
+    else if (b > 2L * g.per) b = 2L * g.per;
+    g.blocks = (int)b;
+    g.own = g.blocks > 2 * g.per ? g.blocks - 2 * g.per : 0;
     const int lines = p.n / 2 + 1, nkb = g.blocks << (p.lk - p.lkc);
     g.slices = (8 * 148 + lines - 1) / lines;  // about eight blocks per SM
     if (g.slices > nkb) g.slices = nkb;
@@ -415,7 +424,9 @@ Geometry geometry(const FftPlan &p, int K) {
 
 size_t qfft_work_bytes(int lat_n, int K) {
     const size_t n = (size_t)lat_n;
-    return (n + geometry(make_plan(lat_n, K), K).slices * n * (n / 2 + 1)) * sizeof(double2);
+    const FftPlan p = make_plan(lat_n, K);
+    const Geometry g = geometry(p, K);
+    return (n + g.slices * n * (n / 2 + 1) + (n * n * g.own << p.lk)) * sizeof(double2);
 }
 
 cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st) {
@@ -424,11 +435,12 @@ cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st) {
 }
 
 int launch_qfft(const double *A, const double *B, int lat_n, int K, const double *m,
-                const double *z, double scale, void *work, double *const scratch[3], double *out,
+                const double *z, double scale, void *work, double *const scratch[2], double *out,
                 cudaStream_t st) {
     const FftPlan p = make_plan(lat_n, K);
     const Geometry g = geometry(p, K);
     double2 *tw = static_cast<double2 *>(work), *part = tw + lat_n;
+    const long half = (long)lat_n * (lat_n / 2 + 1);
     const int rows_t = threads_for(p.n << p.lk), cols_t = threads_for(p.n << (p.lkc + 1));
     const int kc = 1 << p.lk, all = (K + kc - 1) / kc;
     ASD_CUDA_TRY(cudaFuncSetAttribute(qfft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -438,7 +450,8 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
     int launches = 0;
     for (int b0 = 0; b0 < all; b0 += g.blocks) {
         Chunk X;
-        for (int q = 0; q < 3; ++q) X.buf[q] = reinterpret_cast<double2 *>(scratch[q]);
+        for (int q = 0; q < 2; ++q) X.buf[q] = reinterpret_cast<double2 *>(scratch[q]);
+        X.buf[2] = part + g.slices * half;
         X.blocks = all - b0 < g.blocks ? all - b0 : g.blocks;
         X.per = g.per;
         ASD_CUDA_TRY(launch_pdl(qfft_rows_kernel, dim3((unsigned)X.blocks, (unsigned)lat_n), rows_t,
@@ -449,7 +462,6 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
                                 cols_smem(p), st, p, X, tw, b0 > 0, part));
         launches += 2;
     }
-    const long half = (long)lat_n * (lat_n / 2 + 1);
     ASD_CUDA_TRY(launch_pdl(qfft_sum_kernel, (unsigned)((half + 15) / 16), 128, 0, st, part, lat_n,
                             g.slices, scale, reinterpret_cast<double2 *>(out)));
     return launches + 1;

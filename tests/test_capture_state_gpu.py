@@ -1,0 +1,48 @@
+"""Calls captured into a CUDA graph and replayed between uncaptured calls, on
+lattices whose steps run as the one-launch step, which writes the new spins to a
+second buffer."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import asd_b200 as asd
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+KW = dict(J1=-1.0, alpha=0.1, dt=0.01)
+
+
+def make(N, nfile, kernel, stream):
+    ctx = asd.Context(asd.Params.make(N, nfile, **KW), modes=["fp64"])
+    ctx.set_stream(stream.cuda_stream)
+    ctx.set_llg_kernel(kernel)
+    ctx.set_spins(asd.random_spins(N, nfile, seed=N), as_origin=True)
+    return ctx
+
+
+@pytest.mark.parametrize("N,nfile,kernel", [(12, 3, "fused"), (33, 20, "fused"), (128, 256, "auto")])
+def test_replayed_grid_leaves_the_spins(N, nfile, kernel):
+    """The q grid's work space is none of the two buffers that a step alternates
+    between: a replay after an odd number of steps leaves the spins as they are."""
+    stream = torch.cuda.Stream()
+    grid = torch.zeros(2 * N * N, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with make(N, nfile, kernel, stream) as ctx, make(N, nfile, kernel, stream) as other:
+        ctx.step(1)
+        assert asd.load().asd_ctx_last_launches(ctx.handle) == 1
+        other.step(1)
+        ctx.sqt_grid("fp64")  # takes its work space
+        ctx.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.sqt_grid_async("fp64", grid.data_ptr())
+        for _ in range(2):
+            for c in (ctx, other):
+                c.step(1)
+            ctx.synchronize()
+            with torch.cuda.stream(stream):
+                graph.replay()
+            assert np.array_equal(ctx.get_spins(), other.get_spins())
+        del graph
