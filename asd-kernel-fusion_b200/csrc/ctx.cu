@@ -81,6 +81,9 @@ struct asd_ctx {
     // were formed from
     double2 *phase_ws = nullptr, *phase_G = nullptr;
     long g_version = -1;
+    // an origin was set while the stream was captured: replays may change it
+    // unseen by the versions here, so the sums are formed on every call
+    bool origin_captured = false;
     double *d_out = nullptr;
     double *h_out = nullptr;  // pinned
     unsigned *status = nullptr;
@@ -342,6 +345,7 @@ int refresh_origin(asd_ctx *c) {
     c->origin_version = c->state_version;
     for (int k = 1; k <= 3; ++k) c->b_version[k] = -1;
     c->g_version = -1;
+    if (stream_capturing(c->stream)) c->origin_captured = true;
     return ASD_OK;
 }
 
@@ -436,8 +440,9 @@ DmmaSqtArgs dmma_args(const asd_ctx *c) {
 PhaseWork phase_ws(const asd_ctx *c) { return phase_work(c->phase_ws, c->M, c->K); }
 
 // The work space of the phase sums, and the origin's column sums up to date
-// (formed once per origin and q; a captured call forms them itself, as its
-// replays may follow other origins, and leaves the version of the sums alone).
+// (formed once per origin and q; on every call where an origin was set under
+// capture; and a captured call forms them itself, as its replays may follow other
+// origins, and leaves the version of the sums alone).
 int ensure_phase_work(asd_ctx *c) {
     int rc;
     if (!c->phase_ws) {
@@ -459,7 +464,7 @@ int ensure_phase_origin(asd_ctx *c) {
     const int rc = ensure_phase_work(c);
     if (rc != ASD_OK) return rc;
     const bool capturing = stream_capturing(c->stream);
-    if (!capturing && c->g_version == c->origin_version) return ASD_OK;
+    if (!capturing && !c->origin_captured && c->g_version == c->origin_version) return ASD_OK;
     ASD_CUDA_TRY(launch_phase_origin(c->origin, c->M, c->K, c->p.nfile, c->wphase, phase_ws(c),
                                      c->phase_G, c->phase_G + c->K, c->stream));
     if (!capturing) c->g_version = c->origin_version;

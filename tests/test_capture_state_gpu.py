@@ -46,3 +46,31 @@ def test_replayed_grid_leaves_the_spins(N, nfile, kernel):
                 graph.replay()
             assert np.array_equal(ctx.get_spins(), other.get_spins())
         del graph
+
+
+@pytest.mark.parametrize("N,nfile", [(12, 3), (20, 40), (51, 17)])
+def test_replayed_origin_is_the_one_sqt_uses(N, nfile):
+    """A captured set_spins_device(as_origin) gives its replays' origins to the
+    uncaptured S(q,t) and loss that follow them."""
+    stream = torch.cuda.Stream()
+    first, origin, other_spins = (asd.random_spins(N, nfile, seed=k) for k in (1, 2, 3))
+    buf = torch.from_numpy(first.reshape(-1)).cuda()
+    target = np.array([0.2 + 0.1j, 0.1 - 0.1j])
+    torch.cuda.synchronize()
+    with make(N, nfile, "auto", stream) as ctx, make(N, nfile, "auto", stream) as plain:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.set_spins_device(buf.data_ptr(), as_origin=True)
+        for values in (first, origin):
+            buf.copy_(torch.from_numpy(values.reshape(-1)))
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                graph.replay()
+            plain.set_spins(values, as_origin=True)
+            for c in (ctx, plain):
+                c.set_spins(other_spins, as_origin=False)
+                c.step(2)
+            assert ctx.sqt("fp64") == plain.sqt("fp64")
+            a, b = ctx.loss_grad(4, 2, 2, target), plain.loss_grad(4, 2, 2, target)
+            assert a[0] == b[0] and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2])
+        del graph
