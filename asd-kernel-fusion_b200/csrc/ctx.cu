@@ -666,8 +666,9 @@ int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
         c->adj_small_cap = 0;
         c->adj_states = need;
     }
-    // S(q,t) and the loss gradient's factors per evaluation: grown on demand
-    const size_t small = (size_t)(2 * E + 8) * sizeof(double2);
+    // S(q,t) and the loss gradient's factors per evaluation, and the tape's copy of
+    // the origin's sums: grown on demand
+    const size_t small = (size_t)(2 * E + 8 + K + 3) * sizeof(double2);
     double *&buf = c->adj_bufs[c->adj_states + 1];
     if (small > c->adj_small_cap) {
         c->tape_valid = false;
@@ -695,6 +696,7 @@ struct AdjBufs {
     double **stg;  // with a kept segment: stg[4 (j - 1) + q] = s2, s3, s4, acc of step j
     double *bacc, *dgrad;
     double2 *Sv, *coef;  // [E] each
+    double2 *G, *Z;      // the sums of the tape's origin, [K] and [3]
     int nb;
 };
 
@@ -711,6 +713,8 @@ AdjBufs adj_bufs(asd_ctx *c, int nck, int ckpt, int E, bool resident) {
     b.dgrad = b.bacc + (size_t)b.nb * 6;
     b.Sv = reinterpret_cast<double2 *>(B[c->adj_states + 1]);
     b.coef = b.Sv + E + 4;
+    b.G = b.coef + E + 4;
+    b.Z = b.G + c->K;
     return b;
 }
 
@@ -734,6 +738,10 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
     c->last_launches = 0;
     c->tape_valid = false;
     if ((rc = ensure_phase_origin(c)) != ASD_OK) return rc;
+    // the backward pass's own copy: a replayed S(q,t) may form those of another
+    // origin before it
+    ASD_CUDA_TRY(cudaMemcpyAsync(b.G, c->phase_G, ((size_t)K + 3) * sizeof(double2),
+                                 cudaMemcpyDeviceToDevice, st));
     const double sqt_scale = 1.0 / ((double)M * c->p.nfile);
     // forward: checkpoints and S(q,t) at every stride-th step
     ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[0], c->origin, sb, cudaMemcpyDeviceToDevice, st));
@@ -765,8 +773,7 @@ int loss_forward(asd_ctx *c, int nsteps, int stride, int ckpt, const double *tar
         if (n % ckpt == 0 && n / ckpt < nck)
             ASD_CUDA_TRY(cudaMemcpyAsync(b.ck[n / ckpt], cur, sb, cudaMemcpyDeviceToDevice, st));
         if (n % stride == 0 && n / stride <= E) {
-            ASD_CUDA_TRY(launch_phase_sum(cur, M, K, c->uphase, phase_ws(c), c->phase_G,
-                                          c->phase_G + K, sqt_scale,
+            ASD_CUDA_TRY(launch_phase_sum(cur, M, K, c->uphase, phase_ws(c), b.G, b.Z, sqt_scale,
                                           reinterpret_cast<double *>(b.Sv + (n / stride - 1)), st));
             c->last_launches += 2;
         }
@@ -838,7 +845,7 @@ int loss_backward(asd_ctx *c, const double *target, double *grad, double *dtarge
         adjoint_resident_bytes(c->a, ckpt, &work_bytes);
         AdjSegment q{};
         q.stride = stride, q.E = E, q.coef = b.coef;
-        q.u = c->uphase, q.G = c->phase_G, q.Z = c->phase_G + K;
+        q.u = c->uphase, q.G = b.G, q.Z = b.Z;
         q.work = c->adj_res;
         q.states = c->adj_res + work_bytes / sizeof(double);
         q.bacc = b.bacc;
@@ -866,8 +873,7 @@ int loss_backward(asd_ctx *c, const double *target, double *grad, double *dtarge
             const int j = n - base;
             if (n % stride == 0 && n / stride <= E) {
                 const double2 cf = coef[n / stride - 1];
-                ASD_CUDA_TRY(launch_loss_grad(b.lam, M, K, c->uphase, c->phase_G,
-                                              c->phase_G + K, cf.x, cf.y, st));
+                ASD_CUDA_TRY(launch_loss_grad(b.lam, M, K, c->uphase, b.G, b.Z, cf.x, cf.y, st));
                 c->last_launches += 1;
             }
             // y_{n-1} = seg[j-1]: its stage states (kept from the segment's

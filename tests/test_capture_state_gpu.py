@@ -74,3 +74,30 @@ def test_replayed_origin_is_the_one_sqt_uses(N, nfile):
             a, b = ctx.loss_grad(4, 2, 2, target), plain.loss_grad(4, 2, 2, target)
             assert a[0] == b[0] and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2])
         del graph
+
+
+@pytest.mark.parametrize("N,nfile", [(12, 3), (20, 40)])
+def test_backward_keeps_the_origin_of_its_forward(N, nfile):
+    """A replay of {new origin, S(q,t)} between the loss's two passes does not
+    reach the gradient, which belongs to the forward pass's origin."""
+    stream = torch.cuda.Stream()
+    first, second = (asd.random_spins(N, nfile, seed=k) for k in (1, 2))
+    buf = torch.from_numpy(first.reshape(-1)).cuda()
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    target = np.array([0.2 + 0.1j, 0.1 - 0.1j])
+    torch.cuda.synchronize()
+    with make(N, nfile, "auto", stream) as ctx, make(N, nfile, "auto", stream) as plain:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.set_spins_device(buf.data_ptr(), as_origin=True)
+            ctx.sqt_async("fp64", out.data_ptr())
+        for c in (ctx, plain):
+            c.set_spins(first, as_origin=True)
+            c.loss_forward(4, 2, 2, target)
+        buf.copy_(torch.from_numpy(second.reshape(-1)))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        a, b = ctx.loss_backward(target), plain.loss_backward(target)
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+        del graph
