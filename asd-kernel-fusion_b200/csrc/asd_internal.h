@@ -100,8 +100,6 @@ cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout,
 bool llg_resident_wins(const LLGArgs &a, int nsteps);
 // True if the streamed one-launch step is faster than the stage kernels here.
 bool llg_fused_wins(const LLGArgs &a);
-// ... and it gives every resident CTA at least 8 rows.
-bool llg_fused_fills(const LLGArgs &a);
 
 // Counts the x[i] for which the constant divisions by 3 and 6 of the LLG
 // kernels differ from __ddiv_rn in any bit (diagnostic).

@@ -17,6 +17,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "asd_internal.h"
@@ -84,6 +85,9 @@ struct asd_ctx {
     // an origin was set while the stream was captured: replays may change it
     // unseen by the versions here, so the sums are formed on every call
     bool origin_captured = false;
+    // some call was captured: its graph holds the address of y, so from then on
+    // every call leaves the spins there (settle)
+    bool captured = false;
     double *d_out = nullptr;
     double *h_out = nullptr;  // pinned
     unsigned *status = nullptr;
@@ -244,13 +248,6 @@ int chunk_for(const asd_ctx *c, int kind) {
     return c->chunk_k >= 0 ? c->chunk_k : (kind == 1 ? 512 : 1024);
 }
 
-// Prologue of every entry point that may enqueue work: select the device and
-// forget the early y_free point (the caller may touch the LLG buffers next).
-cudaError_t enter(asd_ctx *c) {
-    c->y_free_armed = false;
-    return cudaSetDevice(c->device);
-}
-
 bool stream_capturing(cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
@@ -258,6 +255,14 @@ bool stream_capturing(cudaStream_t s) {
         return true;  // unknown: take the fully ordered path
     }
     return cs != cudaStreamCaptureStatusNone;
+}
+
+// Prologue of every entry point that may enqueue work: select the device and
+// forget the early y_free point (the caller may touch the LLG buffers next).
+cudaError_t enter(asd_ctx *c) {
+    c->y_free_armed = false;
+    if (!c->captured && stream_capturing(c->stream)) c->captured = true;
+    return cudaSetDevice(c->device);
 }
 
 int ensure_llg_stream(asd_ctx *c) {
@@ -377,6 +382,22 @@ bool use_fused(const asd_ctx *c, const LLGArgs &a) {
            (c->llg_kernel == ASD_LLG_AUTO && llg_fused_wins(a));
 }
 
+// After steps that went from y to ys_a and back: the new spins become y.  The
+// buffers swap roles, except where a graph holds their addresses; there an odd
+// number of steps is copied back (128x128x500: 63 us beside a step's 364), so that
+// the replays and the calls between them go on from one another.
+int settle(asd_ctx *c, double *ynew) {
+    if (ynew == c->y) return ASD_OK;
+    if (c->captured) {
+        ASD_CUDA_TRY(cudaMemcpyAsync(c->y, ynew, (size_t)c->M * c->K * sizeof(double),
+                                     cudaMemcpyDeviceToDevice, c->stream));
+    } else {
+        c->ys_a = c->y;
+        c->y = ynew;
+    }
+    return ASD_OK;
+}
+
 int run_steps(asd_ctx *c, int nsteps) {
     if (nsteps > 0 && c->llg_kernel == ASD_LLG_AUTO && llg_resident_wins(c->a, nsteps)) {
         cudaEvent_t t0 = time_begin(c, c->stream);
@@ -386,22 +407,21 @@ int run_steps(asd_ctx *c, int nsteps) {
         c->state_version += nsteps;
         return ASD_OK;
     }
-    // A captured odd number of one-launch steps would leave its replays reading
-    // the same buffer again, so while the stream is captured the default takes
-    // them only on lattices that fill the GPU with rows.
-    if (use_fused(c, c->a) && (c->llg_kernel != ASD_LLG_AUTO || llg_fused_fills(c->a) ||
-                               !stream_capturing(c->stream))) {
+    if (use_fused(c, c->a)) {
+        double *cur = c->y, *nxt = c->ys_a;
         for (int s = 0; s < nsteps; ++s) {
             cudaEvent_t t0 = time_begin(c, c->stream);
-            ASD_CUDA_TRY(launch_llg_step_fused(c->a, c->y, c->ys_a, c->stream));
+            const cudaError_t e = launch_llg_step_fused(c->a, cur, nxt, c->stream);
+            if (e != cudaSuccess) {  // y is the state of the steps that were enqueued
+                settle(c, cur);
+                return cuda_fail(e, "launch_llg_step_fused");
+            }
             time_end(c, 0, 1, c->stream, t0);
-            double *t = c->y;  // ping-pong: the new state becomes y
-            c->y = c->ys_a;
-            c->ys_a = t;
+            std::swap(cur, nxt);
             c->last_launches += 1;
             c->state_version++;
         }
-        return ASD_OK;
+        return settle(c, cur);
     }
     for (int s = 0; s < nsteps; ++s) {
         cudaEvent_t t0 = time_begin(c, c->stream);
@@ -1104,7 +1124,7 @@ int step_host_chunked(asd_ctx *c, const double *spin_in, double *spin_out, int m
     LLGArgs a = c->a;
     long nparts = 0;
     // The one-launch step is out of place: each chunk's new state goes to
-    // ys_a (its replicas only), and y and ys_a swap after the last chunk.
+    // ys_a (its replicas only), which becomes y after the last chunk.
     LLGArgs ac = c->a;  // a whole chunk decides the kernel for every chunk
     ac.nc = cr < nf ? cr : nf;
     const bool fused = use_fused(c, ac);
@@ -1159,10 +1179,7 @@ int step_host_chunked(asd_ctx *c, const double *spin_in, double *spin_out, int m
         nparts += grid;
         c->last_launches += 1;
     }
-    if (fused) {  // ys_a holds the new state of every replica
-        c->ys_a = c->y;
-        c->y = ynew;
-    }
+    if ((rc = settle(c, ynew)) != ASD_OK) return rc;
     c->state_version += 2;  // as set_spins + step
     c->has_state = true;
     if (kind) {
@@ -1262,10 +1279,7 @@ int step_host_async(asd_ctx *c, const double *spin_in, double *spin_out, int mod
         ASD_CUDA_TRY(cudaEventRecord(c->ast_out_done[r], down));
         c->last_launches += fused ? 3 : 6;
     }
-    if (fused) {  // ys_a holds the new state of every replica
-        c->ys_a = c->y;
-        c->y = ynew;
-    }
+    if ((rc = settle(c, ynew)) != ASD_OK) return rc;
     c->state_version += 2;  // as set_spins + step
     c->has_state = true;
     if ((rc = sqt_async(c, mode, c->d_out)) != ASD_OK) return rc;

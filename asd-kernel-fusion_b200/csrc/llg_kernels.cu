@@ -898,12 +898,6 @@ static double fused_cost(const LLGArgs &a) {
     return (run + 9.0) * iter * (a.use_j2 ? 1.29 : 1.0);
 }
 
-// At least 8 rows of work for each of the one-launch step's two CTAs an SM.
-bool llg_fused_fills(const LLGArgs &a) {
-    const StreamGeom g = stream_geom(a);
-    return (long)g.nb * g.ng * a.N >= 8 * 2 * 148;
-}
-
 bool llg_fused_wins(const LLGArgs &a) { return fused_cost(a) < 0.95 * stages_cost(a); }
 
 bool llg_resident_wins(const LLGArgs &a, int nsteps) {

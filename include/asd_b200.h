@@ -125,7 +125,12 @@ int asd_ctx_get_spins(asd_ctx *ctx, double *spin_aos);
 int asd_ctx_get_spins_device(asd_ctx *ctx, double *d_spin_aos);
 
 /* nsteps RK4 steps with renormalisation (llg_sqt_baseline.c:296-309),
- * asynchronous on the context's stream. */
+ * asynchronous on the context's stream.  Asynchronous calls of a context may be
+ * captured into a CUDA graph once they have taken their work space (asd_ctx_step
+ * and, up to N = 39, FP64 S(q,t) at one q take none); replays and uncaptured
+ * calls then go on from one another's spins and origin.  (The split modes form
+ * their operands in the calls that find them out of date, which a replay does not
+ * look up.) */
 int asd_ctx_step(asd_ctx *ctx, int nsteps);
 
 /* S(q,t) between the current state and the origin at q = 2*pi*(vx,vy)/N,

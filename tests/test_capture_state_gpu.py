@@ -101,3 +101,56 @@ def test_backward_keeps_the_origin_of_its_forward(N, nfile):
         a, b = ctx.loss_backward(target), plain.loss_backward(target)
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
         del graph
+
+
+@pytest.mark.parametrize("N,nfile,kernel", [(12, 3, "fused"), (33, 20, "fused"), (96, 300, "auto"),
+                                            (20, 24, "auto"), (20, 24, "stages")])
+@pytest.mark.parametrize("nsteps", [1, 2, 3])
+def test_replays_and_calls_go_on_from_one_another(N, nfile, kernel, nsteps):
+    """Replayed steps start from the spins that the last replay or uncaptured call
+    left, S(q,t) and the q grid see them, and an uncaptured call sees the replay's."""
+    stream = torch.cuda.Stream()
+    sq = torch.zeros(2, dtype=torch.float64, device="cuda")
+    grid = torch.zeros(2 * N * N, dtype=torch.float64, device="cuda")
+    spins = torch.zeros(nfile * N * N * 3, dtype=torch.float64, device="cuda")
+    host = torch.zeros(nfile * N * N * 3, dtype=torch.float64).pin_memory()
+    torch.cuda.synchronize()
+    with make(N, nfile, kernel, stream) as ctx, make(N, nfile, kernel, stream) as plain:
+        if N == 96:  # the default takes the one-launch step here
+            ctx.step(2), plain.step(2)
+            assert asd.load().asd_ctx_last_launches(ctx.handle) == 2
+        for c in (ctx, plain):
+            c.step(1)
+            c.sqt("fp64"), c.sqt_grid("fp64")  # take their work space
+            c.step_host(host.data_ptr(), host.data_ptr(), "fp64")
+            c.set_spins(asd.random_spins(N, nfile, seed=7), as_origin=True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.step(nsteps)
+            ctx.sqt_async("fp64", sq.data_ptr())
+            ctx.sqt_grid_async("fp64", grid.data_ptr())
+            ctx.get_spins_device(spins.data_ptr())
+
+        def replay():
+            with torch.cuda.stream(stream):
+                graph.replay()
+            stream.synchronize()
+            plain.step(nsteps)
+            assert complex(*sq.tolist()) == plain.sqt("fp64")
+            assert np.array_equal(grid.cpu().numpy().view(complex).reshape(N, N),
+                                  plain.sqt_grid("fp64"))
+            y = plain.get_spins()
+            assert np.array_equal(spins.cpu().numpy(), y.reshape(-1))
+            assert np.array_equal(ctx.get_spins(), y)
+
+        for _ in range(3):
+            replay()
+        for between in (lambda c: c.step(1), lambda c: c.step(2),
+                        lambda c: c.step_host(host.data_ptr(), host.data_ptr(), "fp64")):
+            for c in (ctx, plain):
+                host.copy_(torch.from_numpy(plain.get_spins().reshape(-1)))
+                between(c)
+                torch.cuda.synchronize()
+            replay()
+            replay()
+        del graph
