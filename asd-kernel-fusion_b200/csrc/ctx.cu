@@ -257,6 +257,22 @@ bool stream_capturing(cudaStream_t s) {
     return cs != cudaStreamCaptureStatusNone;
 }
 
+// fill(stream), which gives a new work space its fixed contents, so that they are
+// there before any use: on the ctx stream, or, while that is being captured (in
+// relaxed mode a first call may allocate there), done at once on another stream,
+// since calls may come before the graph's first replay.
+template <class F>
+cudaError_t fill_work(asd_ctx *c, F fill) {
+    if (!stream_capturing(c->stream)) return fill(c->stream);
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+    e = fill(s);
+    const cudaError_t es = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    return e != cudaSuccess ? e : es;
+}
+
 // Prologue of every entry point that may enqueue work: select the device and
 // forget the early y_free point (the caller may touch the LLG buffers next).
 cudaError_t enter(asd_ctx *c) {
@@ -468,7 +484,9 @@ int ensure_phase_work(asd_ctx *c) {
     if (!c->phase_ws) {
         const size_t n = phase_work_bytes(c->M, c->K);
         if ((rc = dalloc(&c->phase_ws, n)) != ASD_OK) return rc;
-        const cudaError_t e = cudaMemsetAsync(phase_ws(c).count, 0, sizeof(double2), c->stream);
+        const cudaError_t e = fill_work(c, [&](cudaStream_t s) {
+            return cudaMemsetAsync(phase_ws(c).count, 0, sizeof(double2), s);
+        });
         if (e != cudaSuccess) {  // unusable without its zero count
             cudaFree(c->phase_ws);
             c->phase_ws = nullptr;
@@ -974,7 +992,8 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
             return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 mode");
         if (!c->grid_fft) {
             if ((rc = dalloc(&c->grid_fft, qfft_work_bytes(N, c->K))) != ASD_OK) return rc;
-            const cudaError_t e = launch_qfft_twiddles(N, c->grid_fft, c->stream);
+            const cudaError_t e = fill_work(
+                c, [&](cudaStream_t s) { return launch_qfft_twiddles(N, c->grid_fft, s); });
             if (e != cudaSuccess) {  // unusable without its twiddles
                 cudaFree(c->grid_fft);
                 c->grid_fft = nullptr;
@@ -1000,7 +1019,8 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
     if (!c->grid_g && (rc = dalloc(&c->grid_g, (size_t)M * sizeof(double))) != ASD_OK) return rc;
     if (!c->grid_t) {
         if ((rc = dalloc(&c->grid_t, (size_t)(M + N) * sizeof(double2))) != ASD_OK) return rc;
-        const cudaError_t e = launch_qfft_twiddles(N, c->grid_t + M, c->stream);
+        const cudaError_t e = fill_work(
+            c, [&](cudaStream_t s) { return launch_qfft_twiddles(N, c->grid_t + M, s); });
         if (e != cudaSuccess) {  // unusable without its twiddles
             cudaFree(c->grid_t);
             c->grid_t = nullptr;

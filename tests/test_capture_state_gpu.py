@@ -154,3 +154,38 @@ def test_replays_and_calls_go_on_from_one_another(N, nfile, kernel, nsteps):
             replay()
             replay()
         del graph
+
+
+@pytest.mark.parametrize("call", ["sqt", "grid", "split_grid"])
+def test_first_call_captured_and_never_replayed(call):
+    """In relaxed mode a first call may be captured: it takes its work space there.
+    Uncaptured calls that follow find the fixed contents of that work space (a zero
+    count, the twiddles) although the graph has not run."""
+    N, nfile = 51, 9
+    mode = "fp16x3" if call == "split_grid" else "fp64"
+    stream = torch.cuda.Stream()
+    out = torch.zeros(2 * N * N, dtype=torch.float64, device="cuda")
+    params = asd.Params.make(N, nfile, **KW)
+    with asd.Context(params, modes=[mode]) as ctx, asd.Context(params, modes=[mode]) as plain:
+        for c in (ctx, plain):
+            c.set_stream(stream.cuda_stream)
+            c.set_spins(asd.random_spins(N, nfile, seed=1), as_origin=True)
+        held = [torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda")
+                for n in [4 << 10] * 64 + [1 << 20] * 32]
+        torch.cuda.synchronize()
+        del held
+        torch.cuda.empty_cache()  # what the first call is given is not zero by chance
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            if call == "sqt":
+                ctx.sqt_async(mode, out.data_ptr())
+            else:
+                ctx.sqt_grid_async(mode, out.data_ptr())
+        for c in (ctx, plain):
+            c.set_spins(asd.random_spins(N, nfile, seed=2), as_origin=True)
+        if call == "sqt":
+            assert ctx.sqt(mode) == plain.sqt(mode)
+        else:
+            assert np.array_equal(ctx.sqt_grid(mode), plain.sqt_grid(mode))
+        ctx.check_device_status()
+        del graph
