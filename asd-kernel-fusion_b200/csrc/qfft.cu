@@ -59,6 +59,12 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// The caller's buffer holds doubles, on any boundary of eight bytes: two stores
+// of eight bytes, never one of sixteen.
+__device__ __forceinline__ void put(double *out, long i, double2 v) {
+    out[2 * i] = v.x;
+    out[2 * i + 1] = v.y;
+}
 __device__ __forceinline__ double2 mul_mi(double2 a) { return make_double2(a.y, -a.x); }  // -i a
 
 // Forward transforms of length R in registers.
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
 // 16 frequencies a block, eight threads each: thread s adds slices s, s + 8, ...
 __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict__ part, int n,
                                                        int slices, double scale,
-                                                       double2 *__restrict__ out) {
+                                                       double *__restrict__ out) {
     pdl_begin();
     __shared__ double2 red[8][16];
     const int tl = threadIdx.x & 15, sl = threadIdx.x >> 4;
@@ -317,10 +323,10 @@ __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict
     const int b = (int)(t / n), a = (int)(t - (long)b * n);
     s.x *= scale;
     s.y *= scale;
-    out[(long)a * n + b] = s;
+    put(out, (long)a * n + b, s);
     if (b > 0 && 2 * b != n) {  // -q: the displacement sums are real
         const int ma = (a == 0) ? 0 : n - a;
-        out[(long)ma * n + (n - b)] = make_double2(s.x, -s.y);
+        put(out, (long)ma * n + (n - b), make_double2(s.x, -s.y));
     }
 }
 
@@ -334,7 +340,7 @@ __global__ void __launch_bounds__(MAX_THREADS) bins_dft_kernel(FftPlan p,
                                                                const double2 *__restrict__ T,
                                                                const double2 *__restrict__ tw,
                                                                double scale,
-                                                               double2 *__restrict__ out) {
+                                                               double *__restrict__ out) {
     pdl_begin();
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lk;
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(MAX_THREADS) bins_dft_kernel(FftPlan p,
     for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x) {
         const int line = l0 + (idx & (kc - 1));
         if (line < n)
-            out[(long)(idx >> p.lk) * n + line] = make_double2(f[idx].x * scale, f[idx].y * scale);
+            put(out, (long)(idx >> p.lk) * n + line, make_double2(f[idx].x * scale, f[idx].y * scale));
     }
 }
 
@@ -463,7 +469,7 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
         launches += 2;
     }
     ASD_CUDA_TRY(launch_pdl(qfft_sum_kernel, (unsigned)((half + 15) / 16), 128, 0, st, part, lat_n,
-                            g.slices, scale, reinterpret_cast<double2 *>(out)));
+                            g.slices, scale, out));
     return launches + 1;
 }
 
@@ -481,10 +487,9 @@ cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const doub
             cudaSuccess)
         return e;
     if ((e = launch_pdl(bins_dft_kernel<true>, blocks, threads, smem, st, p, G, nullptr, tw, 1.0,
-                        T)) != cudaSuccess)
+                        reinterpret_cast<double *>(T))) != cudaSuccess)
         return e;
-    return launch_pdl(bins_dft_kernel<false>, blocks, threads, smem, st, p, nullptr, T, tw, scale,
-                      reinterpret_cast<double2 *>(out));
+    return launch_pdl(bins_dft_kernel<false>, blocks, threads, smem, st, p, nullptr, T, tw, scale, out);
 }
 
 }  // namespace asd
