@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <type_traits>
 #include <chrono>
+#include <mutex>
 #include <vector>
 
 #include "asd_internal.h"
@@ -573,6 +574,8 @@ struct asd_batch {
     size_t cl_smem = 0;
     CCta *d_ctas = nullptr;
     CSeg *d_segs = nullptr;
+    // set_spins and get_spins stage in ysa: one at a time, from any thread
+    std::mutex stage_mu;
 };
 
 namespace {
@@ -921,6 +924,7 @@ int asd_batch_set_spins(asd_batch *b, int lattice, const float *spin_aos) {
     ASD_CUDA_TRY(cudaSetDevice(b->device));
     const BatchLattice &L = b->lat[lattice];
     const long M = (long)L.N * L.N;
+    std::lock_guard<std::mutex> lk(b->stage_mu);
     // staged in ysa (stage states only within a run)
     ASD_CUDA_TRY(cudaMemcpyAsync(b->ysa, spin_aos, (size_t)3 * M * sizeof(float),
                                  cudaMemcpyHostToDevice, b->stream));
@@ -937,6 +941,7 @@ int asd_batch_get_spins(asd_batch *b, int lattice, float *spin_aos) {
     ASD_CUDA_TRY(cudaSetDevice(b->device));
     const BatchLattice &L = b->lat[lattice];
     const long M = (long)L.N * L.N;
+    std::lock_guard<std::mutex> lk(b->stage_mu);
     layout_kernel<false><<<(unsigned)((3 * M + 255) / 256), 256, 0, b->stream>>>(b->y + L.off, M,
                                                                                  b->ysa);
     ASD_CUDA_TRY(cudaGetLastError());
