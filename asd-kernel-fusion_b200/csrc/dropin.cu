@@ -152,6 +152,16 @@ cudaError_t stage_share(const Stage &s, int device, size_t t, const std::vector<
     return ok() ? es : e;
 }
 
+// Host arrays that share bytes: written one after the other, in the order given.
+bool overlap(const std::vector<Piece> &p) {
+    for (size_t i = 0; i < p.size(); ++i)
+        for (size_t j = 0; j < i; ++j) {
+            const uintptr_t a = (uintptr_t)p[i].host, b = (uintptr_t)p[j].host;
+            if (a < b + p[j].bytes && b < a + p[i].bytes) return true;
+        }
+    return false;
+}
+
 // Copies whole arrays, complete on return and ordered after the work enqueued on
 // the default stream.
 cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
@@ -159,7 +169,7 @@ cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
     if (e != cudaSuccess) return e;
     size_t total = 0;
     for (const Piece &p : pieces) total += p.bytes;
-    if (total < kStageMin || !ensure_stage(g_buf.stage)) {
+    if (total < kStageMin || (!up && overlap(pieces)) || !ensure_stage(g_buf.stage)) {
         for (const Piece &p : pieces) {
             e = up ? cudaMemcpy(p.dev, p.host, p.bytes, cudaMemcpyHostToDevice)
                    : cudaMemcpy(const_cast<void *>(p.host), p.dev, p.bytes, cudaMemcpyDeviceToHost);
