@@ -162,6 +162,23 @@ bool overlap(const std::vector<Piece> &p) {
     return false;
 }
 
+// Pageable host memory: what the staging threads read and write, and what it is
+// faster for.  The driver copies page-locked arrays directly (runge_kutta on
+// 32x32x800 2.3 ms, staged 4.3), reaches managed ones wherever they are, and
+// refuses device and null addresses.
+bool pageable(const std::vector<Piece> &pieces) {
+    for (const Piece &p : pieces) {
+        cudaPointerAttributes at{};
+        if (!p.host) return false;
+        if (cudaPointerGetAttributes(&at, p.host) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
+
 // Copies whole arrays, complete on return and ordered after the work enqueued on
 // the default stream.
 cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
@@ -169,7 +186,8 @@ cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
     if (e != cudaSuccess) return e;
     size_t total = 0;
     for (const Piece &p : pieces) total += p.bytes;
-    if (total < kStageMin || (!up && overlap(pieces)) || !ensure_stage(g_buf.stage)) {
+    if (total < kStageMin || !pageable(pieces) || (!up && overlap(pieces)) ||
+        !ensure_stage(g_buf.stage)) {
         for (const Piece &p : pieces) {
             e = up ? cudaMemcpy(p.dev, p.host, p.bytes, cudaMemcpyHostToDevice)
                    : cudaMemcpy(const_cast<void *>(p.host), p.dev, p.bytes, cudaMemcpyDeviceToHost);

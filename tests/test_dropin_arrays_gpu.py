@@ -39,3 +39,42 @@ def test_outputs_that_overlap_are_written_in_order(separate):
             want[s:s + n] = o
         rk(spin, [buf[s:s + n] for s in starts])
         assert np.array_equal(buf, want), starts
+
+
+def test_page_locked_and_managed_arrays(separate):
+    from cuda.bindings import runtime as rt
+
+    spin, outs = separate
+    locked = [torch.zeros(spin.size, dtype=torch.float64).pin_memory().numpy() for _ in range(6)]
+    locked[0][:] = spin
+    rk(locked[0], locked[1:])
+    for got, want in zip(locked[1:], outs):
+        assert np.array_equal(got, want)
+    ptrs = []
+    try:
+        for _ in range(6):
+            err, p = rt.cudaMallocManaged(spin.nbytes, rt.cudaMemAttachGlobal)
+            assert int(err) == 0
+            ptrs.append(int(p))
+        managed = [np.frombuffer((C.c_char * spin.nbytes).from_address(p)) for p in ptrs]
+        managed[0][:] = spin
+        rk(ptrs[0], ptrs[1:])
+        for got, want in zip(managed[1:], outs):
+            assert np.array_equal(got, want)
+    finally:
+        for p in ptrs:
+            rt.cudaFree(p)
+
+
+def test_null_arrays_are_refused_as_before(separate):
+    """A null input or output: reported, nothing read or written through it."""
+    spin, outs = separate
+    new = [np.zeros_like(spin) for _ in range(5)]
+    rk(0, new)
+    assert "invalid" in asd.last_error()
+    assert all((x == 0.0).all() for x in new)
+    rk(spin, [new[0], 0, *new[2:]])
+    assert "invalid" in asd.last_error()
+    rk(spin, new)
+    for got, want in zip(new, outs):
+        assert np.array_equal(got, want)
