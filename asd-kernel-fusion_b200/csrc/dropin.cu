@@ -13,10 +13,10 @@
 // and leaves the outputs unchanged.
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <thread>
 #include <utility>
-#include <vector>
 
 #include "asd_internal.h"
 #include "fp64_gemm.h"
@@ -122,22 +122,36 @@ struct Piece {
     const void *host;  // written by downloads
     size_t bytes;
 };
+using Pieces = std::initializer_list<Piece>;
+
+// Chunk i of the arrays in their order (bytes = 0 past the last one).
+Piece chunk(const Pieces &pieces, size_t i) {
+    for (const Piece &p : pieces) {
+        const size_t n = (p.bytes + kStageChunk - 1) / kStageChunk;
+        if (i < n) {
+            const size_t at = i * kStageChunk;
+            return {static_cast<char *>(p.dev) + at, static_cast<const char *>(p.host) + at,
+                    p.bytes - at < kStageChunk ? p.bytes - at : kStageChunk};
+        }
+        i -= n;
+    }
+    return {nullptr, nullptr, 0};
+}
 
 // One thread's share of a staged copy: chunks t, t + kStageThreads, ...
-cudaError_t stage_share(const Stage &s, int device, size_t t, const std::vector<Piece> &chunks,
-                        bool up) {
+cudaError_t stage_share(const Stage &s, int device, size_t t, const Pieces &pieces, bool up) {
     cudaError_t e = cudaSetDevice(device);
     auto ok = [&] { return e == cudaSuccess; };
-    auto fetch = [&](size_t i, int b) {
-        e = cudaMemcpyAsync(s.pinned[t][b], chunks[i].dev, chunks[i].bytes, cudaMemcpyDeviceToHost,
-                            s.stream[t]);
+    auto fetch = [&](const Piece &c, int b) {
+        e = cudaMemcpyAsync(s.pinned[t][b], c.dev, c.bytes, cudaMemcpyDeviceToHost, s.stream[t]);
         if (ok()) e = cudaEventRecord(s.done[t][b], s.stream[t]);
     };
     int b = 0;
-    if (!up && t < chunks.size() && ok()) fetch(t, 0);
-    for (size_t i = t; i < chunks.size() && ok(); i += kStageThreads, b ^= 1) {
-        const Piece &c = chunks[i];
-        if (!up && i + kStageThreads < chunks.size()) fetch(i + kStageThreads, b ^ 1);
+    Piece c = chunk(pieces, t);
+    if (!up && c.bytes && ok()) fetch(c, 0);
+    for (size_t i = t; c.bytes && ok(); i += kStageThreads, b ^= 1) {
+        const Piece next = chunk(pieces, i + kStageThreads);
+        if (!up && next.bytes) fetch(next, b ^ 1);
         if (ok()) e = cudaEventSynchronize(s.done[t][b]);  // buffer b: its last copy is done
         if (!ok()) break;
         if (up) {
@@ -147,17 +161,18 @@ cudaError_t stage_share(const Stage &s, int device, size_t t, const std::vector<
         } else {
             std::memcpy(const_cast<void *>(c.host), s.pinned[t][b], c.bytes);
         }
+        c = next;
     }
     const cudaError_t es = cudaStreamSynchronize(s.stream[t]);  // on the error paths too
     return ok() ? es : e;
 }
 
 // Host arrays that share bytes: written one after the other, in the order given.
-bool overlap(const std::vector<Piece> &p) {
-    for (size_t i = 0; i < p.size(); ++i)
-        for (size_t j = 0; j < i; ++j) {
-            const uintptr_t a = (uintptr_t)p[i].host, b = (uintptr_t)p[j].host;
-            if (a < b + p[j].bytes && b < a + p[i].bytes) return true;
+bool overlap(const Pieces &pieces) {
+    for (const Piece &p : pieces)
+        for (const Piece &q : pieces) {
+            const uintptr_t a = (uintptr_t)p.host, b = (uintptr_t)q.host;
+            if (&p < &q && a < b + q.bytes && b < a + p.bytes) return true;
         }
     return false;
 }
@@ -166,7 +181,7 @@ bool overlap(const std::vector<Piece> &p) {
 // faster for.  The driver copies page-locked arrays directly (runge_kutta on
 // 32x32x800 2.3 ms, staged 4.3), reaches managed ones wherever they are, and
 // refuses device and null addresses.
-bool pageable(const std::vector<Piece> &pieces) {
+bool pageable(const Pieces &pieces) {
     for (const Piece &p : pieces) {
         cudaPointerAttributes at{};
         if (!p.host) return false;
@@ -180,8 +195,8 @@ bool pageable(const std::vector<Piece> &pieces) {
 }
 
 // Copies whole arrays, complete on return and ordered after the work enqueued on
-// the default stream.
-cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
+// the default stream.  Nothing here throws but what starts a thread.
+cudaError_t copy(const Pieces &pieces, bool up) {
     cudaError_t e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) return e;
     size_t total = 0;
@@ -195,29 +210,24 @@ cudaError_t copy(const std::vector<Piece> &pieces, bool up) {
         }
         return cudaSuccess;
     }
-    std::vector<Piece> chunks;
-    for (const Piece &p : pieces)
-        for (size_t at = 0; at < p.bytes; at += kStageChunk)
-            chunks.push_back({static_cast<char *>(p.dev) + at, static_cast<const char *>(p.host) + at,
-                              p.bytes - at < kStageChunk ? p.bytes - at : kStageChunk});
     cudaError_t err[kStageThreads] = {};
-    auto share = [&](size_t t) { err[t] = stage_share(g_buf.stage, g_buf.device, t, chunks, up); };
-    std::vector<std::thread> threads;
+    auto share = [&](size_t t) { err[t] = stage_share(g_buf.stage, g_buf.device, t, pieces, up); };
+    std::thread threads[kStageThreads];
     size_t t = 1;
     try {
-        threads.reserve(kStageThreads);
-        for (; t < kStageThreads; ++t) threads.emplace_back(share, t);
+        for (; t < kStageThreads; ++t) threads[t] = std::thread(share, t);
     } catch (...) {  // no more threads: this one takes their shares
     }
     share(0);
     for (; t < kStageThreads; ++t) share(t);
-    for (std::thread &th : threads) th.join();
+    for (std::thread &th : threads)
+        if (th.joinable()) th.join();
     for (cudaError_t r : err)
         if (r != cudaSuccess) return r;
     return cudaSuccess;
 }
-cudaError_t upload(const std::vector<Piece> &p) { return copy(p, true); }
-cudaError_t download(const std::vector<Piece> &p) { return copy(p, false); }
+cudaError_t upload(const Pieces &p) { return copy(p, true); }
+cudaError_t download(const Pieces &p) { return copy(p, false); }
 
 // The cached buffers belong to one device.  A call on another device frees
 // them there (with that device current, as cudaFree wants) and starts over.

@@ -78,3 +78,54 @@ def test_null_arrays_are_refused_as_before(separate):
     rk(spin, new)
     for got, want in zip(new, outs):
         assert np.array_equal(got, want)
+
+
+PRELOAD = r"""
+#include <cstdlib>
+#include <new>
+static thread_local int armed = 0;
+extern "C" void fail_new(int on) { armed = on; }
+void *operator new(std::size_t n) {
+    void *p = armed ? nullptr : std::malloc(n ? n : 1);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, std::size_t) noexcept { std::free(p); }
+"""
+
+CHILD = r"""
+import ctypes as C, sys
+import numpy as np
+import asd_b200 as asd
+N, NFILE = 32, 120
+spin = asd.random_spins(N, NFILE, seed=5).reshape(-1)
+asd.set_params(N, NFILE, 1.0, 0.02)
+runs = []
+for failing in (0, 1):
+    outs = [np.zeros_like(spin) for _ in range(5)]
+    p = [C.c_void_p(x.ctypes.data) for x in (spin, *outs)]
+    C.CDLL(None).fail_new(failing)
+    asd.load().runge_kutta(*p)
+    C.CDLL(None).fail_new(0)
+    runs.append(outs)
+assert all(np.array_equal(x, y) and x.any() for x, y in zip(*runs))
+print("same")
+"""
+
+
+def test_no_exception_leaves_the_c_entry(tmp_path):
+    """With every C++ allocation of the calling thread failing, runge_kutta still
+    gives its results: the staging starts no threads and throws nothing."""
+    import os
+    import subprocess
+    import sys
+
+    src, lib = tmp_path / "fail_new.cpp", tmp_path / "fail_new.so"
+    src.write_text(PRELOAD)
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    env = dict(os.environ, LD_PRELOAD=str(lib),
+               PYTHONPATH=os.pathsep.join([p for p in sys.path if p]))
+    r = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]
