@@ -9,8 +9,9 @@
 // They take host pointers and return when the results are back in host
 // memory, like the originals.  Device buffers are cached between calls on the
 // current device and grow on demand.  The functions return void, as in the
-// reference; a failure is reported on stderr and through asd_last_error(),
-// and leaves the outputs unchanged.
+// reference; a failure is reported on stderr and through asd_last_error().  One
+// before the results are copied back (arguments, memory, upload, kernels) leaves the
+// outputs unchanged; one during that copy leaves them partly written.
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
