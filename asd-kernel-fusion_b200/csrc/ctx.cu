@@ -645,68 +645,40 @@ bool use_resident_adjoint(const asd_ctx *c) {
     return blocks > 0;
 }
 
-// Work space of the adjoint: state-sized buffers (stage states, adjoint
-// variables, checkpoints, one recomputed segment) and small reduction buffers.
-// Where the RK4 step runs as four stage kernels and half of the free device
-// memory holds them, also the stage states (s2, s3, s4, acc) of every step of
-// a segment, so that the backward pass reads them instead of recomputing
-// each step's stages a second time (c->adj_keep).
-int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
-    const long M = c->M;
-    const int K = c->K, E = nsteps / stride;
-    const size_t sb = (size_t)M * K * sizeof(double);
-    const int nck = (nsteps + ckpt - 1) / ckpt;  // checkpoints at 0, ckpt, 2 ckpt, ...
-    const int seglen = std::min(ckpt, nsteps);
-    bool resident = use_resident_adjoint(c);
-    size_t work_bytes = 0;
-    const size_t resident_bytes =
-        resident ? adjoint_resident_bytes(c->a, seglen, &work_bytes) : 0;
-    if (resident && resident_bytes > c->adj_res_cap) {  // its padded states may need more memory
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-            resident = (double)resident_bytes <= 0.5 * ((double)free_b + (double)c->adj_res_cap);
-        } else {
-            cudaGetLastError();
-            resident = false;
-        }
-    }
-    c->adj_resident = resident;
-    // resident: the segment's states are in its own work space
-    long need = 10 + nck + (resident ? 2 : ckpt + 1);
-    const long need_keep = need + 4L * ckpt;
-    bool keep = false;
-    if (!use_fused(c, c->a) && !resident) {
-        size_t free_b = 0, total_b = 0;
-        if (c->adj_states >= need_keep) {
-            keep = true;
-        } else if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-            // the buffers held now are freed before the new set is allocated
-            const double avail = (double)free_b + (double)c->adj_states * (double)sb;
-            keep = (double)need_keep * (double)sb <= 0.5 * avail;
-        } else {
-            cudaGetLastError();
-        }
-    }
-    if (keep) need = need_keep;
-    c->adj_keep = keep;
+// Frees the adjoint's state-sized and small buffers.
+void free_adjoint_states(asd_ctx *c) {
+    for (double *q : c->adj_bufs)
+        if (q) cudaFree(q);
+    c->adj_bufs.clear();
+    c->adj_states = 0;
+    c->adj_small_cap = 0;
+    c->tape_valid = false;
+}
+
+void free_adjoint_resident(asd_ctx *c) {
+    if (c->adj_res) cudaFree(c->adj_res);
+    c->adj_res = nullptr;
+    c->adj_res_cap = 0;
+    c->tape_valid = false;
+}
+
+// At least `need` state-sized buffers and the small ones.
+int reserve_adjoint_states(asd_ctx *c, long need, int E) {
+    const size_t sb = (size_t)c->M * c->K * sizeof(double);
     int rc;
     if (c->adj_states < need) {
-        c->tape_valid = false;
-        for (double *q : c->adj_bufs)
-            if (q) cudaFree(q);
+        free_adjoint_states(c);
         c->adj_bufs.assign(need + 2, nullptr);
-        c->adj_states = 0;
         for (long i = 0; i < need; ++i)
             if ((rc = dalloc(&c->adj_bufs[i], sb)) != ASD_OK) return rc;
         const int nb = std::max(adjoint_blocks(c->a), adjoint_resident_blocks(c->a));
         const size_t small = (size_t)(nb + 1) * 6 * sizeof(double);
         if ((rc = dalloc(&c->adj_bufs[need], small)) != ASD_OK) return rc;
-        c->adj_small_cap = 0;
         c->adj_states = need;
     }
     // S(q,t) and the loss gradient's factors per evaluation, and the tape's copy of
     // the origin's sums: grown on demand
-    const size_t small = (size_t)(2 * E + 8 + K + 3) * sizeof(double2);
+    const size_t small = (size_t)(2 * E + 8 + c->K + 3) * sizeof(double2);
     double *&buf = c->adj_bufs[c->adj_states + 1];
     if (small > c->adj_small_cap) {
         c->tape_valid = false;
@@ -716,15 +688,68 @@ int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
         if ((rc = dalloc(&buf, small)) != ASD_OK) return rc;
         c->adj_small_cap = small;
     }
-    if (resident && resident_bytes > c->adj_res_cap) {
-        c->tape_valid = false;
-        if (c->adj_res) cudaFree(c->adj_res);
-        c->adj_res = nullptr;
-        c->adj_res_cap = 0;
-        if ((rc = dalloc(&c->adj_res, resident_bytes)) != ASD_OK) return rc;
-        c->adj_res_cap = resident_bytes;
-    }
     return ASD_OK;
+}
+
+// At least `bytes` of the resident adjoint's work space.
+int reserve_adjoint_resident(asd_ctx *c, size_t bytes) {
+    if (bytes <= c->adj_res_cap) return ASD_OK;
+    free_adjoint_resident(c);
+    const int rc = dalloc(&c->adj_res, bytes);
+    if (rc == ASD_OK) c->adj_res_cap = bytes;
+    return rc;
+}
+
+// Work space of the adjoint: state-sized buffers (stage states, adjoint
+// variables, checkpoints, one recomputed segment) and small reduction buffers; for
+// the resident backward pass its own work space in place of the segment.  That
+// pass is taken where all of it fits in half of the memory that is free or held
+// here already, and given up where its allocation fails all the same, so that a
+// call asks for no more than the kernel-by-kernel form where memory is short.
+// That form also takes, where the RK4 step runs as four stage kernels and the same
+// half holds them, the stage states (s2, s3, s4, acc) of every step of a segment,
+// so that the backward pass reads them instead of recomputing each step's stages a
+// second time (c->adj_keep).
+int ensure_adjoint(asd_ctx *c, int nsteps, int stride, int ckpt) {
+    const int E = nsteps / stride;
+    const double sb = (double)c->M * c->K * sizeof(double);
+    const int nck = (nsteps + ckpt - 1) / ckpt;  // checkpoints at 0, ckpt, 2 ckpt, ...
+    size_t work_bytes = 0;
+    const size_t resident_bytes =
+        use_resident_adjoint(c) ? adjoint_resident_bytes(c->a, std::min(ckpt, nsteps), &work_bytes)
+                                : 0;
+    const long need_resident = 10L + nck + 2, need_plain = 10L + nck + ckpt + 1;
+    const long need_keep = need_plain + 4L * ckpt;
+    // true if `states` buffers and `extra` bytes are held, or fit in half of what is
+    // free and held
+    auto fits = [&](long states, size_t extra) {
+        if (c->adj_states >= states && c->adj_res_cap >= extra) return true;
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        const double held = (double)c->adj_states * sb + (double)c->adj_res_cap;
+        return (double)states * sb + (double)extra <= 0.5 * ((double)free_b + held);
+    };
+    int rc;
+    c->adj_keep = false;
+    c->adj_resident = resident_bytes > 0 && fits(need_resident, resident_bytes);
+    if (c->adj_resident) {
+        if ((rc = reserve_adjoint_states(c, need_resident, E)) != ASD_OK) return rc;
+        if (reserve_adjoint_resident(c, resident_bytes) == ASD_OK) return ASD_OK;
+        // what is held may lie in its way: without it, then without this form
+        free_adjoint_states(c);
+        if (reserve_adjoint_resident(c, resident_bytes) == ASD_OK &&
+            reserve_adjoint_states(c, need_resident, E) == ASD_OK)
+            return ASD_OK;
+        free_adjoint_states(c);
+        c->adj_resident = false;
+    }
+    c->adj_keep = !use_fused(c, c->a) && fits(need_keep, 0);
+    const long need = c->adj_keep ? need_keep : need_plain;
+    if (c->adj_states < need) free_adjoint_resident(c);  // its memory may be needed
+    return reserve_adjoint_states(c, need, E);
 }
 
 // The adjoint's buffers by role.
