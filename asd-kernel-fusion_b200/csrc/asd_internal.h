@@ -127,9 +127,12 @@ cudaError_t launch_rk_pass(int pass, long n, double dt, const double *spin, doub
 
 // --------------------------------------------------------- S(q,t) kernels
 // Per-site replica mean (FP64) plus the FP32 epilogue vectors
-// vec4[i] = (mx, my, mz, phase.re), vec1[i] = phase.im for i < M.
+// vec4[i] = (mx, my, mz, phase.re), vec1[i] = phase.im for i < M.  With top, *top
+// becomes the larger of itself and the high word of the largest magnitude among
+// the state's components (without the sign).
 cudaError_t launch_site_mean(const double *state, long M, int nfile, const double2 *phase,
-                             double *mean, float4 *vec4, float *vec1, cudaStream_t st);
+                             double *mean, float4 *vec4, float *vec1, unsigned *top,
+                             cudaStream_t st);
 
 // Per-site sums over the context's replicas ([M][3]), and the S(q,t) of a
 // replica-sharded ensemble from its all-reduced partial and site sums.
@@ -177,14 +180,15 @@ cudaError_t launch_phase_sum(const double *A, long M, int K, const double2 *upha
 
 // ------------------------------------- FP64 S(q,t) on the q grid (qfft.cu)
 // out[2 (a N + b)] = scale * sum_k A~_k conj(B~_k) at q = 2 pi (a, b) / N, the
-// transforms of A - m and B - z (m, z [M][3]); work: qfft_work_bytes, its first
+// transforms of A - m and B - z (m, z [M][3]); top: the magnitudes of A and B that
+// launch_site_mean gives, and a copy of the first, which the last kernel zeroes; work: qfft_work_bytes, its first
 // N complex values written once by launch_qfft_twiddles; scratch: two buffers
 // of M K doubles.  Returns the number of launches or a negative error.
 size_t qfft_work_bytes(int lat_n, int K);
 cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st);
 int launch_qfft(const double *A, const double *B, int lat_n, int K, const double *m,
-                const double *z, double scale, void *work, double *const scratch[2], double *out,
-                cudaStream_t st);
+                const double *z, unsigned *top, double scale, void *work,
+                double *const scratch[2], double *out, cudaStream_t st);
 
 // ------------------------------------------------- FP64 tensor-core GEMM
 // (dmma_sqt.cu) C = alpha A B^T over site-major [M][K] FP64 operands.  Per

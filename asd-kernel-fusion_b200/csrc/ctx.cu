@@ -91,6 +91,9 @@ struct asd_ctx {
     double *d_out = nullptr;
     double *h_out = nullptr;  // pinned
     unsigned *status = nullptr;
+    // beside it: the magnitudes of the state (zero between q grids), the origin and
+    // a copy of the first (launch_site_mean, launch_qfft)
+    unsigned *top = nullptr;
     long state_version = 0, origin_version = -1;
     bool has_state = false, has_origin = false;
     int last_launches = 0;
@@ -360,8 +363,9 @@ void time_end(asd_ctx *c, int which, int launches, cudaStream_t s, cudaEvent_t b
 
 int refresh_origin(asd_ctx *c) {
     // origin mean and the column epilogue vectors
+    ASD_CUDA_TRY(cudaMemsetAsync(c->top + 1, 0, sizeof(unsigned), c->stream));
     ASD_CUDA_TRY(launch_site_mean(c->origin, c->M, c->p.nfile, c->wphase, c->mean_0, c->col4,
-                                  c->col1, c->stream));
+                                  c->col1, c->top + 1, c->stream));
     c->last_launches += 1;
     c->origin_version = c->state_version;
     for (int k = 1; k <= 3; ++k) c->b_version[k] = -1;
@@ -612,7 +616,7 @@ int sqt_async(asd_ctx *c, int mode, double *d_out, bool shard = false) {
     if (!(c->modes & (1u << mode))) return fail(ASD_ERR_STATE, "mode %d not enabled at create", mode);
     if (mode == ASD_SQT_FP64) return sqt_plain(c, d_out, shard);
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
-                                  c->stream));
+                                  nullptr, c->stream));
     c->rows_ready = true;
     c->last_launches += 1;
     switch (mode) {
@@ -1027,13 +1031,13 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
             c->last_launches += 1;
         }
         ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4,
-                                      c->row1, c->stream));
+                                      c->row1, c->top, c->stream));
         c->rows_ready = true;
         c->last_launches += 1;
         // RK4 state only within a step; not ys_a, which the one-launch step swaps
         // with y: where this call is captured, a replay may find the spins there
         double *const scratch[2] = {c->ys_b, c->acc};
-        rc = launch_qfft(c->y, c->origin, N, c->K, c->mean_t, c->mean_0,
+        rc = launch_qfft(c->y, c->origin, N, c->K, c->mean_t, c->mean_0, c->top,
                          1.0 / ((double)M * c->p.nfile), c->grid_fft, scratch, d_out, c->stream);
         if (rc < 0) return rc;
         c->last_launches += rc;
@@ -1054,7 +1058,7 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
         c->last_launches += 1;
     }
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
-                                  c->stream));
+                                  nullptr, c->stream));
     c->rows_ready = true;
     c->last_launches += 1;
     const int kind = mode_kind(mode);
@@ -1159,7 +1163,7 @@ int step_host_chunked(asd_ctx *c, const double *spin_in, double *spin_out, int m
         if ((rc = ensure_split_origin(c, kind)) != ASD_OK) return rc;
         if (!c->rows_ready) {  // the early chunks' epilogues read the phase u_i
             ASD_CUDA_TRY(launch_site_mean(c->y, M, nf, c->uphase, c->mean_t, c->row4, c->row1,
-                                          c->stream));
+                                          nullptr, c->stream));
             c->rows_ready = true;
             c->last_launches += 1;
         }
@@ -1211,7 +1215,7 @@ int step_host_chunked(asd_ctx *c, const double *spin_in, double *spin_out, int m
         c->last_launches += 1;
         if (last) {
             ASD_CUDA_TRY(launch_site_mean(ynew, M, nf, c->uphase, c->mean_t, c->row4, c->row1,
-                                          comp));
+                                          nullptr, comp));
             c->last_launches += 1;
         }
         UmmaSqtArgs u = split_args(c, kind, 1.0 / (double)nf);
@@ -1470,7 +1474,8 @@ int asd_ctx_create(const asd_params *p, unsigned mode_mask, asd_ctx **out) {
     ASD_ALLOC(c->row1, (size_t)c->Mp * sizeof(float));
     ASD_ALLOC(c->col1, (size_t)c->Mp * sizeof(float));
     ASD_ALLOC(c->d_out, 2 * sizeof(double));
-    ASD_ALLOC(c->status, sizeof(unsigned));
+    ASD_ALLOC(c->status, 4 * sizeof(unsigned));
+    c->top = c->status + 1;
     for (int mode = ASD_SQT_TF32X3; mode <= ASD_SQT_FP16X3; ++mode) {
         const int kind = mode_kind(mode);
         if (!(c->modes & (1u << mode))) continue;
@@ -1491,7 +1496,7 @@ int asd_ctx_create(const asd_params *p, unsigned mode_mask, asd_ctx **out) {
     ASD_CUDA_TRY(cudaMemset(c->col4, 0, (size_t)c->Mp * sizeof(float4)));
     ASD_CUDA_TRY(cudaMemset(c->row1, 0, (size_t)c->Mp * sizeof(float)));
     ASD_CUDA_TRY(cudaMemset(c->col1, 0, (size_t)c->Mp * sizeof(float)));
-    ASD_CUDA_TRY(cudaMemset(c->status, 0, sizeof(unsigned)));
+    ASD_CUDA_TRY(cudaMemset(c->status, 0, 4 * sizeof(unsigned)));
     e = cudaMallocHost((void **)&c->h_out, 2 * sizeof(double));
     if (e != cudaSuccess) {
         destroy(c);
@@ -1684,7 +1689,7 @@ int asd_ctx_sqt_magnitude(asd_ctx *c, double *out) {
     ASD_CUDA_TRY(enter(c));
     c->last_launches = 0;
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
-                                  c->stream));
+                                  nullptr, c->stream));
     c->rows_ready = true;
     const long tiles = dmma_sqt_tiles(c->M);
     if (tiles > 0x7fffffffL) return fail(ASD_ERR_UNSUPPORTED, "lattice too large for the FP64 GEMM");

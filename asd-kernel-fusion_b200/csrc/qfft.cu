@@ -6,10 +6,14 @@
 //   S(q) = (1/(M nfile)) sum_k A~_k(q) conj(B~_k(q)),
 // A~, B~ the 2-D transforms (kernel e^{-i q.r}) of column k of A - m and B - z,
 // m and z the replica means at t and at the origin: sum_f (B - z) = 0, so
-// subtracting m changes nothing but the rounding (both are fluctuations of the
-// same size).  One complex transform serves both: with Z the transform of
-// (A - m) + i (B - z), W = Z(-q),
-//   A~ conj(B~) = (Z.x W.y + Z.y W.x) / 2 + (i/4) (|Z|^2 - |W|^2).
+// subtracting m changes nothing but the rounding.  One complex transform serves
+// both: with Z the transform of (A - m) + i (B - z), W = Z(-q),
+//   A~ conj(B~) = (Z.x W.y + Z.y W.x) / 2 + (i/4) (|Z|^2 - |W|^2),
+// whose rounding is that of the larger of |A~|^2 and |B~|^2.  So each operand is
+// brought to the same size first, by a power of two from its largest component
+// (read beside the means); the product is multiplied back at the end.  Spins of
+// length 1 and 1e8 then have the relative error of equal ones (2e-9 without), and
+// none overflow that the product does not.
 // About 5 M log2(M) operations per column instead of 2 M^2.
 //
 // Columns go in chunks whose transform (16 M bytes a column) stays in L2, held
@@ -193,6 +197,19 @@ __device__ __forceinline__ double2 *transform(double2 *a, double2 *b, const doub
     return a;
 }
 
+// 2^(1023 - e) for the exponent field e of the largest magnitude (high word top),
+// which brings it to [1, 2), and the inverse; 1 where it is subnormal or not finite.
+// The inverse of a zero operand is 0: its product is, but for the rounding of the other.
+__device__ __forceinline__ double to_unit(unsigned top) {
+    const int e = (int)(top >> 20);
+    return e == 0 || e == 0x7ff ? 1.0 : __hiloint2double((2046 - min(e, 2045)) << 20, 0);
+}
+__device__ __forceinline__ double from_unit(unsigned top) {
+    const int e = (int)(top >> 20);
+    if (top == 0) return 0.0;
+    return e == 0 || e == 0x7ff ? 1.0 : __hiloint2double(min(e, 2045) << 20, 0);
+}
+
 __global__ void qfft_twiddle_kernel(int n, double2 *__restrict__ tw) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
@@ -219,7 +236,8 @@ struct Chunk {
 // beyond are zero.
 __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
     FftPlan p, const double *__restrict__ A, const double *__restrict__ B, int K, int k0, Chunk X,
-    const double *__restrict__ m, const double *__restrict__ z, const double2 *__restrict__ tw) {
+    const double *__restrict__ m, const double *__restrict__ z, const unsigned *__restrict__ top,
+    const double2 *__restrict__ tw) {
     pdl_begin();
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lk;
@@ -227,13 +245,14 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
     for (int j = threadIdx.x; j < n; j += blockDim.x) stw[j] = tw[j];
     const long r = blockIdx.y;
     const int kl = blockIdx.x * kc;  // within the chunk
+    const double fa = to_unit(top[0]), fb = to_unit(top[1]);
     for (int idx = threadIdx.x; idx < (n << p.lk); idx += blockDim.x) {
         const int c = idx >> p.lk, k = k0 + kl + (idx & (kc - 1));
         double2 v = make_double2(0.0, 0.0);
         if (k < K) {
             const long site = r * n + c;
-            v.x = A[site * K + k] - m[site * 3 + k % 3];
-            v.y = B[site * K + k] - z[site * 3 + k % 3];
+            v.x = (A[site * K + k] - m[site * 3 + k % 3]) * fa;
+            v.y = (B[site * K + k] - z[site * 3 + k % 3]) * fb;
         }
         b0[idx] = v;
     }
@@ -249,8 +268,10 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_rows_kernel(
 // Block (b, slice): frequencies (a, b) for every a, b <= n / 2; the slice's
 // k blocks of this chunk.  add: onto the sums of the earlier chunks.
 __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
-    FftPlan p, Chunk X, const double2 *__restrict__ tw, int add, double2 *__restrict__ part) {
+    FftPlan p, Chunk X, const double2 *__restrict__ tw, int add, unsigned *top,
+    double2 *__restrict__ part) {
     pdl_begin();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) top[2] = top[0];
     extern __shared__ __align__(16) double2 fsm[];
     const int n = p.n, kc = 1 << p.lkc, lt = p.lkc + 1, len = n << p.lkc;
     double2 *b0 = fsm, *b1 = b0 + (n << lt), *sum = b1 + (n << lt), *stw = sum + n;
@@ -302,10 +323,13 @@ __global__ void __launch_bounds__(MAX_THREADS) qfft_cols_kernel(
 }
 
 // 16 frequencies a block, eight threads each: thread s adds slices s, s + 8, ...
+// The state's magnitude, of which it reads the copy, is zero again for the next call.
 __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict__ part, int n,
                                                        int slices, double scale,
+                                                       unsigned *top,
                                                        double *__restrict__ out) {
     pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) top[0] = 0;
     __shared__ double2 red[8][16];
     const int tl = threadIdx.x & 15, sl = threadIdx.x >> 4;
     const long t = (long)blockIdx.x * 16 + tl;
@@ -321,8 +345,9 @@ __global__ void __launch_bounds__(128) qfft_sum_kernel(const double2 *__restrict
 #pragma unroll
     for (int q = 1; q < 8; ++q) s = cadd(s, red[q][tl]);
     const int b = (int)(t / n), a = (int)(t - (long)b * n);
-    s.x *= scale;
-    s.y *= scale;
+    const double fa = from_unit(top[2]), fb = from_unit(top[1]);
+    s.x = s.x * scale * fa * fb;
+    s.y = s.y * scale * fa * fb;
     put(out, (long)a * n + b, s);
     if (b > 0 && 2 * b != n) {  // -q: the displacement sums are real
         const int ma = (a == 0) ? 0 : n - a;
@@ -441,8 +466,8 @@ cudaError_t launch_qfft_twiddles(int lat_n, void *work, cudaStream_t st) {
 }
 
 int launch_qfft(const double *A, const double *B, int lat_n, int K, const double *m,
-                const double *z, double scale, void *work, double *const scratch[2], double *out,
-                cudaStream_t st) {
+                const double *z, unsigned *top, double scale, void *work,
+                double *const scratch[2], double *out, cudaStream_t st) {
     const FftPlan p = make_plan(lat_n, K);
     const Geometry g = geometry(p, K);
     double2 *tw = static_cast<double2 *>(work), *part = tw + lat_n;
@@ -461,15 +486,15 @@ int launch_qfft(const double *A, const double *B, int lat_n, int K, const double
         X.blocks = all - b0 < g.blocks ? all - b0 : g.blocks;
         X.per = g.per;
         ASD_CUDA_TRY(launch_pdl(qfft_rows_kernel, dim3((unsigned)X.blocks, (unsigned)lat_n), rows_t,
-                                rows_smem(p), st, p, A, B, K, b0 * kc, X, m, z, tw));
+                                rows_smem(p), st, p, A, B, K, b0 * kc, X, m, z, top, tw));
         // a last, shorter chunk still visits every slice (with no block it adds zero)
         ASD_CUDA_TRY(launch_pdl(qfft_cols_kernel,
                                 dim3((unsigned)(lat_n / 2 + 1), (unsigned)g.slices), cols_t,
-                                cols_smem(p), st, p, X, tw, b0 > 0, part));
+                                cols_smem(p), st, p, X, tw, b0 > 0, top, part));
         launches += 2;
     }
     ASD_CUDA_TRY(launch_pdl(qfft_sum_kernel, (unsigned)((half + 15) / 16), 128, 0, st, part, lat_n,
-                            g.slices, scale, out));
+                            g.slices, scale, top, out));
     return launches + 1;
 }
 

@@ -23,29 +23,39 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// One warp per site: mean over replicas of the 3 components.
+// One warp per site: mean over replicas of the 3 components.  With top, the high
+// word of the largest magnitude among all components goes there as a maximum (an
+// integer one: the same in any order); few warps find it below their own.
+template <bool TOP>
 __global__ void __launch_bounds__(256) site_mean_kernel(const double *__restrict__ state, long M,
                                                         int nfile,
                                                         const double2 *__restrict__ phase,
                                                         double *__restrict__ mean,
                                                         float4 *__restrict__ vec4,
-                                                        float *__restrict__ vec1) {
+                                                        float *__restrict__ vec1,
+                                                        unsigned *top) {
     pdl_begin();
     const long site = (long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
     if (site >= M) return;
     const double *p = state + site * 3L * nfile;
     double sx = 0.0, sy = 0.0, sz = 0.0;
+    unsigned big = 0;
+    auto magnitude = [](double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; };
 #pragma unroll 4
     for (int f = lane; f < nfile; f += 32) {
-        sx += p[3 * f];
-        sy += p[3 * f + 1];
-        sz += p[3 * f + 2];
+        const double x = p[3 * f], y = p[3 * f + 1], z = p[3 * f + 2];
+        sx += x;
+        sy += y;
+        sz += z;
+        if (TOP) big = max(big, max(magnitude(x), max(magnitude(y), magnitude(z))));
     }
     sx = warp_sum(sx);
     sy = warp_sum(sy);
     sz = warp_sum(sz);
+    if (TOP) big = __reduce_max_sync(0xffffffffu, big);
     if (lane == 0) {
+        if (TOP && big > __ldcg(top)) atomicMax(top, big);
         const double mx = sx / nfile, my = sy / nfile, mz = sz / nfile;
         mean[site * 3] = mx;
         mean[site * 3 + 1] = my;
@@ -234,9 +244,11 @@ __global__ void __launch_bounds__(256) finalize_kernel(const double2 *__restrict
 }  // namespace
 
 cudaError_t launch_site_mean(const double *state, long M, int nfile, const double2 *phase,
-                             double *mean, float4 *vec4, float *vec1, cudaStream_t st) {
+                             double *mean, float4 *vec4, float *vec1, unsigned *top,
+                             cudaStream_t st) {
     const unsigned blocks = (unsigned)((M + 7) / 8);
-    return launch_pdl(site_mean_kernel, blocks, 256, 0, st, state, M, nfile, phase, mean, vec4, vec1);
+    return launch_pdl(top ? site_mean_kernel<true> : site_mean_kernel<false>, blocks, 256, 0, st,
+                      state, M, nfile, phase, mean, vec4, vec1, top);
 }
 
 cudaError_t launch_site_sum(const double *state, long M, int nfile, double *sums,
