@@ -216,13 +216,30 @@ cudaError_t launch_transpose_f64(const double *in, long rows, long cols, double 
 // C[i + j ldc] *= beta for i < m, j < n (beta == 0: set to +0).
 cudaError_t launch_scale_f64(double *c, long m, long n, long ldc, double beta, cudaStream_t st);
 
-// q grid (qgrid.cu): from per-tile diagonal partials (pairs hi + lo) tdiag[mb][nb][bm+bn-1][2]
+// q grid (qgrid.cu): from per-tile diagonal partials tdiag[mb][nb][bm+bn-1][2]
 // of num_m x num_n tiles of bm x bn sites (bn a multiple of bm) to the N*N
 // displacement bins G, in a fixed order; ds holds qgrid_keys() * (bm+bn-1) * 2
-// doubles of work space.
+// doubles of work space; top: the magnitudes the tiles were formed with, of which the
+// state's is zeroed.
 long qgrid_keys(int num_m, int num_n, int bm, int bn);
 cudaError_t launch_qgrid_bins(const float2 *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
-                              double *ds, double *G, cudaStream_t st);
+                              unsigned *top, double *ds, double *G, cudaStream_t st);
+#ifdef __CUDACC__
+// The power of two that the q grid's values are divided by, from the magnitudes of
+// the state and the origin (launch_site_mean): with |A| < 2^a and |B| < 2^b a value
+// C_ij - m_i . z_j is below 6 x 2^(a + b), a tile's diagonal sum below 2^(a + b + 10),
+// kept to 2^126.
+__device__ __forceinline__ int grid_shift(const unsigned *top) {
+    const int n = (int)(top[0] >> 20) - 1022 + (int)(top[1] >> 20) - 1022 - 116;
+    return n < 0 ? 0 : (n > 32 ? 32 : n);
+}
+// A partial: a float and the rest in units of 2^-54 of its leading bit.
+__device__ __forceinline__ double grid_value(float2 v) {
+    const int e = (__float_as_int(v.x) >> 23) & 0xff;
+    const double unit = e == 0xff ? 0.0 : __hiloint2double((e + (1023 - 127 - 54)) << 20, 0);
+    return (double)v.x + (double)__float_as_int(v.y) * unit;
+}
+#endif
 // out[2*(a*N+b)+{0,1}] = scale * sum_d G[d] e^{-2 pi i (a dr + b dc)/N} (qfft.cu); tw: N twiddles
 // (launch_qfft_twiddles), T: N*N of work space.
 cudaError_t launch_bins_dft(const double *G, int lat_n, double scale, const double2 *tw, double2 *T,
@@ -282,8 +299,9 @@ struct UmmaSqtArgs {
     int chunk_k = 0;          // K elements per TMEM accumulation chunk (0: all)
     float *dbg_c = nullptr;   // diagnostic: store the accumulator instead
     long dbg_ldc = 0;
-    float2 *tdiag = nullptr;  // q grid: per-tile diagonal partials, each a pair
-                              // hi + lo, [Mp/BM][Mp/BN][BM+BN-1][2] (qgrid.cu)
+    float2 *tdiag = nullptr;  // q grid: per-tile diagonal partials (grid_value),
+                              // [Mp/BM][Mp/BN][BM+BN-1][2] (qgrid.cu)
+    const unsigned *top = nullptr;  // and the magnitudes of the two operands
     int lat_n = 0;            // lattice side (q grid)
     // K sub-range [k_begin, k_end) in elements (multiples of the k block;
     // k_end = 0: to Kp).  The epilogue applies the connected-part term only

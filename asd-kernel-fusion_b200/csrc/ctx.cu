@@ -1058,7 +1058,7 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
         c->last_launches += 1;
     }
     ASD_CUDA_TRY(launch_site_mean(c->y, c->M, c->p.nfile, c->uphase, c->mean_t, c->row4, c->row1,
-                                  nullptr, c->stream));
+                                  c->top, c->stream));
     c->rows_ready = true;
     c->last_launches += 1;
     const int kind = mode_kind(mode);
@@ -1070,11 +1070,12 @@ int sqt_grid_async(asd_ctx *c, int mode, double *d_out) {
     if (rc != ASD_OK) return rc;
     UmmaSqtArgs u = split_args(c, kind, 1.0 / (double)c->p.nfile);
     u.tdiag = c->grid_tdiag;
+    u.top = c->top;
     u.lat_n = N;
     const int grid = launch_umma_sqt(u, c->stream);
     if (grid < 0) return grid;
-    ASD_CUDA_TRY(launch_qgrid_bins(c->grid_tdiag, num_m, num_n, bm, bn, N, c->grid_ds, c->grid_g,
-                                   c->stream));
+    ASD_CUDA_TRY(launch_qgrid_bins(c->grid_tdiag, num_m, num_n, bm, bn, N, c->top, c->grid_ds,
+                                   c->grid_g, c->stream));
     c->last_launches += 3;
     ASD_CUDA_TRY(launch_bins_dft(c->grid_g, N, 1.0 / (double)M, c->grid_t + M, c->grid_t, d_out,
                                  c->stream));

@@ -36,10 +36,11 @@ __device__ __forceinline__ long floordiv(long a, long b) {  // b > 0
 constexpr int KEY_X = 64, KEY_SLICES = 4;
 __global__ void __launch_bounds__(KEY_X *KEY_SLICES)
     qgrid_keys_kernel(const float2 *__restrict__ tdiag, int num_m, int num_n, int bm, int bn,
-                      double *__restrict__ ds) {
+                      const unsigned *__restrict__ top, double *__restrict__ ds) {
     pdl_begin();
     __shared__ double red[KEY_SLICES][KEY_X];
     const int x = threadIdx.x % KEY_X, slice = threadIdx.x / KEY_X;
+    const double up = (double)(1L << grid_shift(top));
     const int R = bn / bm, nd = bm + bn - 1;
     const long nkeys = num_m + (long)R * (num_n - 1);
     const long n = nkeys * nd * 2, want = (long)blockIdx.x * KEY_X + x;
@@ -56,21 +57,20 @@ __global__ void __launch_bounds__(KEY_X *KEY_SLICES)
     double s = 0.0;
     t += slice * step;
 #pragma unroll 4
-    for (long mb = mb0 + slice * R; mb < end; mb += R * KEY_SLICES, t += step * KEY_SLICES) {
-        const float2 v = *t;
-        s += (double)v.x + (double)v.y;
-    }
+    for (long mb = mb0 + slice * R; mb < end; mb += R * KEY_SLICES, t += step * KEY_SLICES)
+        s += grid_value(*t);
     red[slice][x] = s;
     __syncthreads();
     if (slice || want >= n) return;
 #pragma unroll
     for (int k = 1; k < KEY_SLICES; ++k) s += red[k][x];
-    ds[idx] = s;
+    ds[idx] = s * up;
 }
 
 __global__ void qgrid_bins_kernel(const double *__restrict__ ds, int num_m, int num_n, int bm,
-                                  int bn, int N, double *__restrict__ G) {
+                                  int bn, int N, unsigned *top, double *__restrict__ G) {
     pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) top[0] = 0;  // read by the kernels before
     const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= (long)N * N) return;
     const int R = bn / bm, nd = bm + bn - 1;
@@ -101,15 +101,15 @@ long qgrid_keys(int num_m, int num_n, int bm, int bn) {
 }
 
 cudaError_t launch_qgrid_bins(const float2 *tdiag, int num_m, int num_n, int bm, int bn, int lat_n,
-                              double *ds, double *G, cudaStream_t st) {
+                              unsigned *top, double *ds, double *G, cudaStream_t st) {
     if (bn % bm != 0) return cudaErrorInvalidValue;
     const long n1 = qgrid_keys(num_m, num_n, bm, bn) * (bm + bn - 1) * 2;
     const cudaError_t e = launch_pdl(qgrid_keys_kernel, (unsigned)((n1 + KEY_X - 1) / KEY_X),
-                                     KEY_X * KEY_SLICES, 0, st, tdiag, num_m, num_n, bm, bn, ds);
+                                     KEY_X * KEY_SLICES, 0, st, tdiag, num_m, num_n, bm, bn, top, ds);
     if (e != cudaSuccess) return e;
     const long n2 = (long)lat_n * lat_n;
     return launch_pdl(qgrid_bins_kernel, (unsigned)((n2 + 255) / 256), 256, 0, st, ds, num_m, num_n,
-                      bm, bn, lat_n, G);
+                      bm, bn, lat_n, top, G);
 }
 
 }  // namespace asd

@@ -46,7 +46,7 @@ constexpr uint32_t WAIT_LIMIT = 1u << 24;
 constexpr int GROUP_M = 16;
 // q grid: per warp, a transposition buffer for half a block (32 rows x 16
 // columns FP32, row stride 17) while a tile is binned, then the warp's
-// tile-diagonal partials (5 x 32 x 2 pairs) when it is combined; the two uses
+// tile-diagonal partials (5 x 32 x 2 pairs of floats) when it is combined; the two uses
 // alternate, so they share one region.
 constexpr int GRID_DIAG_M = 5;  // diagonals per lane and warp: 32 m + lane, 5 values of m
 constexpr int GRID_XPOSE = 32 * 17;
@@ -141,23 +141,40 @@ __device__ __forceinline__ uint32_t grid_below_mask(int x0, int thr, int N) {
     return m;
 }
 
-// A sum of floats as an unevaluated pair: each add's rounding error (Knuth's
-// two-sum) goes to lo, so hi + lo carries about 48 bits.  Overflow is that of
-// FP32, as in the block sums that go in; an infinite sum leaves lo NaN, which
-// the reader has to drop (value()).  The q grid's sums over blocks, K chunks and
-// warps are kept so: with FP64 registers in their place the FP16x3 grid took
-// 496 us at 100 x 100 x 240 and 1880 at 128 x 128 x 500, with pairs 388 and 1710
-// (the one-q epilogue: 329 and 1740).  Against the FP64 grid the error is the
-// same to nine digits, from 12 x 12 to 128 x 128 sites in the three modes.
-struct Pair32 {
-    float hi, lo;
-    __device__ __forceinline__ void add(float x) {
-        const float s = hi + x, b = s - hi;
-        lo += (hi - (s - b)) + (x - b);
-        hi = s;
+// x + y = s + e exactly, s the rounded sum (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float x, float y, float &e) {
+    const float s = x + y, b = s - x;
+    e = (x - (s - b)) + (y - b);
+    return s;
+}
+
+// The q grid's sums over blocks, K chunks and warps: three floats whose unevaluated
+// sum carries about 72 bits, more than FP64's 53.  FP64 registers in their place are
+// slow beside the tensor cores: 45 such instructions a thread and tile took 4.2 us a
+// tile (100x100x240 in FP16x3 380 -> 472 us, 128x128x500 1682 -> 1861).  Their range is
+// FP32's; grid_shift keeps the sums inside it.
+struct Sum3 {
+    float h, m, l;
+    __device__ __forceinline__ void add(float x, float e) {  // x + e, |e| far below |x|
+        float r, t, u;
+        h = two_sum(h, x, r);
+        m = two_sum(m, r, t);
+        m = two_sum(m, e, u);
+        l += t + u;
     }
-    __device__ __forceinline__ float2 value() const {
-        return make_float2(hi, fabsf(hi) <= 3.402823466e38f ? lo : 0.f);
+    // As a float and a fixed-point remainder of 2^-54 of the float's leading bit: 55
+    // bits, in the eight bytes of a double (grid_value reads it).
+    __device__ __forceinline__ float2 pack() const {
+        float a, b, c = l;
+        float x = two_sum(h, m, a);
+        a = two_sum(a, c, b);
+        x = two_sum(x, a, c);
+        a = two_sum(c, b, c);
+        const int e = (__float_as_int(x) >> 23) & 0xff;
+        // 2^(127 - e); for the largest e a subnormal
+        const float up = __int_as_float(e < 254 ? (254 - e) << 23 : 0x00400000);
+        const int rest = __float2int_rn(a * up * 0x1p54f) + __float2int_rn(c * up * 0x1p54f);
+        return e == 0xff ? make_float2(h, 0.f) : make_float2(x, __int_as_float(rest));
     }
 };
 
@@ -248,10 +265,12 @@ __device__ __forceinline__ void grid_half(const uint32_t (&v)[16], int lane, con
 //              warp's 32 rows and 128 columns: a 32 x 32 block of the
 //              accumulator goes through shared memory transposed along its
 //              diagonals, each lane sums its two diagonals of the block in a
-//              fixed order (FP32, at most 32 terms) into pairs of floats, and
-//              the eight warps' pairs are combined per tile in warp order.
-//              No atomics: the bins repeat bit for bit.
-constexpr int EPI_PHASE = 0, EPI_STORE = 1, EPI_GRID = 2;
+//              fixed order (FP32, at most 32 terms), these are added over the
+//              chunks as Sum3, and the eight warps' sums are combined per tile
+//              in warp order.  No atomics: the bins repeat bit for bit.
+//   EPI_GRID1  the same where one chunk takes all of K: at most two block
+//              sums a diagonal and warp, an exact pair of floats.
+constexpr int EPI_PHASE = 0, EPI_STORE = 1, EPI_GRID = 2, EPI_GRID1 = 3;
 template <int KIND, int EPI>
 __global__ void __launch_bounds__(CTA_THREADS, 1)
     umma_sqt_kernel(const __grid_constant__ CUtensorMap tm_ah,
@@ -262,9 +281,11 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                     const float *__restrict__ row1, const float4 *__restrict__ col4,
                     const float *__restrict__ col1, float alpha, double2 *__restrict__ part,
                     unsigned *__restrict__ status, float *__restrict__ dbg_c, long dbg_ldc,
-                    int lat_n, float2 *__restrict__ tdiag, int group_m) {
+                    int lat_n, const unsigned *__restrict__ top, float2 *__restrict__ tdiag,
+                    int group_m) {
     using G = Geo;
     constexpr bool STORE = (EPI == EPI_STORE);
+    constexpr bool GRID = (EPI == EPI_GRID || EPI == EPI_GRID1);
     constexpr int NHALF = EW / 4;              // warps per TMEM lane quarter
     constexpr int GPH = BN / 32 / NHALF;       // 32-column groups per warp
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -470,7 +491,10 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
         // q grid: the first tile's table here, each later one's before the
         // barrier that ends the tile before it
         bool go = true;
-        if (EPI == EPI_GRID && (long)blockIdx.x < num_tiles) {
+        // q grid: every value times a power of two (1 but for spins near 1e17)
+        const float down = GRID ? exp2f(-(float)grid_shift(top)) : 1.f;
+        const float galpha = alpha * down;
+        if (GRID && (long)blockIdx.x < num_tiles) {
             load_table(blockIdx.x, 0);
             go = sync();
         }
@@ -486,7 +510,8 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                 load_table(tile, tb);
                 if (!sync()) break;
             }
-            const float4 r4 = STORE ? make_float4(0.f, 0.f, 0.f, 0.f) : row4[i];
+            float4 r4 = STORE ? make_float4(0.f, 0.f, 0.f, 0.f) : row4[i];
+            if (GRID) r4.x *= down, r4.y *= down, r4.z *= down;
             const float ui = STORE ? 0.f : row1[i];
             double s_re = 0.0, s_im = 0.0;
             bool ok = true;
@@ -494,12 +519,12 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
             // + lane of the tile, both classes; the lattice column of the warp's
             // first row; a = (i - j) mod N of its first block's lambda = L, and the
             // step of a from block to block.
-            Pair32 gd[GRID_DIAG_M][2];
+            Sum3 gd[GRID_DIAG_M][2];  // one chunk: a pair in h, m
             int x_first = 0, a_first = 0, n32 = 0;
-            if (EPI == EPI_GRID) {
+            if (GRID) {
 #pragma unroll
                 for (int mm = 0; mm < GRID_DIAG_M; ++mm)
-                    gd[mm][0] = gd[mm][1] = Pair32{0.f, 0.f};
+                    gd[mm][0] = gd[mm][1] = Sum3{0.f, 0.f, 0.f};
                 x_first = (int)((mb * (long)BM + quarter * 32) % lat_n);
                 // diagonal d = 32 quarter + lane - 32 c_first: i - j = i0 - j0 + d
                 long dl = (long)mb * BM - (long)nb * BN + quarter * 32 + lane - 32 * c_first;
@@ -521,7 +546,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                 // Per 32-column group, in FP32: a = sum_j w_j acc_ij and, in the
                 // last chunk only, o = sum_j w_j (m_i . z_j); the row sum
                 // s_i = alpha * a - o is carried in FP64.
-                if (EPI == EPI_GRID) {
+                if (GRID) {
                     // half blocks in order, the next one's TMEM load in flight
                     const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                         (uint32_t)(abuf * BN + c_first * 32);
@@ -529,6 +554,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                     ptx::tmem_ld_32x32b_x16(t0, v[0]);
                     int a = a_first;  // (i - j) mod N of the block's lambda = L
                     uint32_t below = grid_below_mask(x_first, a, lat_n);
+                    float prev[2] = {0.f, 0.f};  // lambda = L - 32 of the block before
 #pragma unroll
                     for (int cc = 0; cc < GPH; ++cc) {
                         a -= n32;
@@ -540,20 +566,30 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                         float p[4] = {0.f, 0.f, 0.f, 0.f};
                         ptx::tmem_ld_wait();
                         ptx::tmem_ld_32x32b_x16(t0 + cc * 32 + 16, v[1]);
-                        grid_half<0>(v[0], lane, r4, zq, alpha, last, m, xpose, p);
+                        grid_half<0>(v[0], lane, r4, zq, galpha, last, m, xpose, p);
                         ptx::tmem_ld_wait();
                         if (cc + 1 < GPH) ptx::tmem_ld_32x32b_x16(t0 + cc * 32 + 32, v[0]);
-                        grid_half<1>(v[1], lane, r4, zq, alpha, last, m, xpose, p);
-                        // lambda = L: local diagonal GPH - cc; lambda = L - 32 (zero in
-                        // lane 0, which has none): GPH - 1 - cc
-                        gd[GPH - cc][0].add(p[0]);
-                        gd[GPH - cc][1].add(p[1]);
-                        gd[GPH - 1 - cc][0].add(p[2]);
-                        gd[GPH - 1 - cc][1].add(p[3]);
+                        grid_half<1>(v[1], lane, r4, zq, galpha, last, m, xpose, p);
+                        // local diagonal GPH - cc: this block's lambda = L and the
+                        // lambda = L - 32 of the one before (zero in lane 0)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            Sum3 &g = gd[GPH - cc][k];
+                            float e;
+                            const float x = two_sum(prev[k], p[k], e);
+                            if (EPI == EPI_GRID1) g.h = x, g.m = e;
+                            else g.add(x, e);
+                            prev[k] = p[2 + k];
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        if (EPI == EPI_GRID1) gd[0][k].h = prev[k];
+                        else gd[0][k].add(prev[k], 0.f);
                     }
                 }
 #pragma unroll 1
-                for (int cc = 0; cc < (EPI == EPI_GRID ? 0 : GPH); ++cc) {
+                for (int cc = 0; cc < (GRID ? 0 : GPH); ++cc) {
                     const int c = c_first + cc;
                     uint32_t v[32];
                     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
@@ -606,30 +642,58 @@ __global__ void __launch_bounds__(CTA_THREADS, 1)
                 }
             }
             if (!ok) break;
-            if (EPI == EPI_GRID) {
-                // the warps' diagonals -> tdiag[tile], in warp order; each warp
-                // leaves them where its transposition buffer was
+            if (GRID) {
+                // the warps' diagonals -> tdiag[tile], in warp order; each warp leaves
+                // them where its transposition buffer was, the third floats after
+                // the first two have been read.  Diagonals 32 m + lane, m = -8 .. 3:
+                // m and m + 8 to a warp, both classes to a lane.
+                const float4 *const wd = reinterpret_cast<const float4 *>(wdiag) + lane;
+                Sum3 sum[2][2];
+                auto gather = [&](auto third) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const int m = warp - 2 - 8 + EW * j;
+                        if (m >= BM / 32) break;
+#pragma unroll
+                        for (int w = 0; w < EW; ++w) {
+                            // warp 2 + w: quarter (2 + w) % 4, column half w / 4
+                            const int mm = m - ((2 + w) & 3) + (w / 4) * GPH + GPH;
+                            if (mm < 0 || mm >= GRID_DIAG_M) continue;
+                            const float4 t = wd[(w * GRID_DIAG_M + mm) * 32];
+                            if (decltype(third)::value) {
+                                sum[j][0].l += t.x;
+                                sum[j][1].l += t.y;
+                            } else {
+                                sum[j][0].add(t.x, t.y);
+                                sum[j][1].add(t.z, t.w);
+                            }
+                        }
+                    }
+                };
+#pragma unroll
+                for (int j = 0; j < 2; ++j) sum[j][0] = sum[j][1] = Sum3{0.f, 0.f, 0.f};
 #pragma unroll
                 for (int mm = 0; mm < GRID_DIAG_M; ++mm)
                     reinterpret_cast<float4 *>(wq)[mm * 32 + lane] =
-                        make_float4(gd[mm][0].hi, gd[mm][0].lo, gd[mm][1].hi, gd[mm][1].lo);
+                        make_float4(gd[mm][0].h, gd[mm][0].m, gd[mm][1].h, gd[mm][1].m);
                 if (!sync()) break;
-                float2 *td = tdiag + ((long)mb * num_n + nb) * GRID_ND * 2;
-                for (int idx = etid; idx < GRID_ND * 2; idx += 32 * EW) {
-                    const int d = idx / 2 - (BN - 1), cls = idx & 1;
-                    const int L = (d + 256) & 31, m = (d - L) / 32;
-                    Pair32 sum{0.f, 0.f};
+                gather(std::false_type{});
+                if (EPI == EPI_GRID) {
+                    if (!sync()) break;
 #pragma unroll
-                    for (int w = 0; w < EW; ++w) {
-                        // warp 2 + w: quarter (2 + w) % 4, column half w / 4
-                        const int mm = m - ((2 + w) & 3) + (w / 4) * GPH + GPH;
-                        if (mm >= 0 && mm < GRID_DIAG_M) {
-                            const float2 t = wdiag[((w * GRID_DIAG_M + mm) * 32 + L) * 2 + cls];
-                            sum.add(t.x);
-                            sum.lo += t.y;
-                        }
-                    }
-                    td[idx] = sum.value();
+                    for (int mm = 0; mm < GRID_DIAG_M; ++mm)
+                        reinterpret_cast<float2 *>(wq)[2 * (mm * 32 + lane)] =
+                            make_float2(gd[mm][0].l, gd[mm][1].l);
+                    if (!sync()) break;
+                    gather(std::true_type{});
+                }
+                float4 *const td = reinterpret_cast<float4 *>(tdiag + ((long)mb * num_n + nb) * GRID_ND * 2);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int d = 32 * (warp - 2 - 8 + EW * j) + lane;
+                    if (d <= -BN || d >= BM) continue;
+                    const float2 c0 = sum[j][0].pack(), c1 = sum[j][1].pack();
+                    td[d + BN - 1] = make_float4(c0.x, c0.y, c1.x, c1.y);
                 }
                 if (tile + gridDim.x < num_tiles) load_table(tile + gridDim.x, tb ^ 1);
                 if (!sync()) break;
@@ -746,11 +810,15 @@ int launch_umma_sqt(const UmmaSqtArgs &a, cudaStream_t st) {
     int grid = tiles < a.num_sms ? (int)tiles : a.num_sms;
     if (a.max_grid > 0 && grid > a.max_grid) grid = a.max_grid;
     if (grid < 1) return fail(ASD_ERR_INVALID, "no tiles to launch");
-    const int epi = a.dbg_c ? EPI_STORE : (a.tdiag ? EPI_GRID : EPI_PHASE);
-    if (epi == EPI_GRID && (a.lat_n < 1 || (long)a.lat_n * a.lat_n != a.M || a.k_begin != 0 ||
+    const bool grid_epi = !a.dbg_c && a.tdiag;
+    const int epi = a.dbg_c ? EPI_STORE
+                    : !a.tdiag ? EPI_PHASE
+                    : kpc >= num_kb ? EPI_GRID1
+                                    : EPI_GRID;
+    if (grid_epi && (a.lat_n < 1 || (long)a.lat_n * a.lat_n != a.M || a.k_begin != 0 ||
                             (a.k_end != 0 && a.k_end != a.Kp)))
         return fail(ASD_ERR_INVALID, "q grid: M must be N*N and K whole");
-    const int smem = smem_bytes() + ((epi == EPI_GRID) ? GRID_SCRATCH_BYTES : 0);
+    const int smem = smem_bytes() + (grid_epi ? GRID_SCRATCH_BYTES : 0);
     auto go = [&](auto kern) {
         cudaError_t r =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -758,22 +826,21 @@ int launch_umma_sqt(const UmmaSqtArgs &a, cudaStream_t st) {
         kern<<<grid, CTA_THREADS, smem, st>>>(tah, tal, tbh, tbl, num_m, num_n, kb_begin, kb_end,
                                               kpc, a.outer, a.row4, a.row1, a.col4, a.col1,
                                               a.alpha, a.part, a.status, a.dbg_c, a.dbg_ldc,
-                                              a.lat_n, a.tdiag, GROUP_M);
+                                              a.lat_n, a.top, a.tdiag, GROUP_M);
         return cudaGetLastError();
     };
-    cudaError_t e;
-    if (a.kind == 3)
-        e = epi == EPI_STORE  ? go(umma_sqt_kernel<3, EPI_STORE>)
-            : epi == EPI_GRID ? go(umma_sqt_kernel<3, EPI_GRID>)
-                              : go(umma_sqt_kernel<3, EPI_PHASE>);
-    else if (a.kind == 2)
-        e = epi == EPI_STORE  ? go(umma_sqt_kernel<2, EPI_STORE>)
-            : epi == EPI_GRID ? go(umma_sqt_kernel<2, EPI_GRID>)
-                              : go(umma_sqt_kernel<2, EPI_PHASE>);
-    else
-        e = epi == EPI_STORE  ? go(umma_sqt_kernel<1, EPI_STORE>)
-            : epi == EPI_GRID ? go(umma_sqt_kernel<1, EPI_GRID>)
-                              : go(umma_sqt_kernel<1, EPI_PHASE>);
+    auto pick = [&](auto kind) {
+        constexpr int KIND = decltype(kind)::value;
+        switch (epi) {
+            case EPI_STORE: return go(umma_sqt_kernel<KIND, EPI_STORE>);
+            case EPI_GRID: return go(umma_sqt_kernel<KIND, EPI_GRID>);
+            case EPI_GRID1: return go(umma_sqt_kernel<KIND, EPI_GRID1>);
+            default: return go(umma_sqt_kernel<KIND, EPI_PHASE>);
+        }
+    };
+    const cudaError_t e = a.kind == 3   ? pick(std::integral_constant<int, 3>{})
+                          : a.kind == 2 ? pick(std::integral_constant<int, 2>{})
+                                        : pick(std::integral_constant<int, 1>{});
     if (e != cudaSuccess) return cuda_fail(e, "umma_sqt launch");
     return grid;
 }
