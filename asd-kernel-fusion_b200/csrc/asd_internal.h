@@ -25,6 +25,7 @@ struct LLGArgs {
     // ensemble (0, nfile) unless a caller pipelines the step by replica chunk
     // (replicas never interact, so a chunk's step needs no other replica).
     int f0, nc;
+    int sms = 148;  // of the device: the rules that choose a kernel by size
 };
 
 LLGArgs make_llg_args(const asd_params &p);

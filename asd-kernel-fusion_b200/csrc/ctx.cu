@@ -1446,7 +1446,7 @@ int asd_ctx_create(const asd_params *p, unsigned mode_mask, asd_ctx **out) {
     c->p = *p;
     c->a = make_llg_args(*p);
     c->device = g_device;
-    c->num_sms = prop.multiProcessorCount;
+    c->a.sms = c->num_sms = prop.multiProcessorCount;
     c->M = (long)p->N * p->N;
     c->Mp = umma_row_pad(c->M);
     c->K = 3 * p->nfile;
@@ -1653,6 +1653,7 @@ int asd_ctx_set_params(asd_ctx *c, const asd_params *p) {
     c->p = *p;
     c->params_version++;
     c->a = make_llg_args(*p);
+    c->a.sms = c->num_sms;
     if (q_changed) {
         const double qx = 2.0 * M_PI * p->vx / (double)p->N, qy = 2.0 * M_PI * p->vy / (double)p->N;
         std::vector<double2> u((size_t)c->M), w((size_t)c->M);

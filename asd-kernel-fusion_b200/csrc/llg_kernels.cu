@@ -877,14 +877,17 @@ cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout,
 //   one-launch      rows per CTA + 9 iterations, for 72 columns 3.1 with two CTAs
 //                   an SM and 1.8 with one (1.29 times that with J2)
 //   resident        2.8 a launch, and per round of resident CTAs, q to an SM:
-//                   2.3 + 3.7e-3 q n a step (4.7 with J2; clusters 6.3 + 3.9e-3 n),
-//                   and 0.8 + 2.6e-3 q n once to load and store the lattice
-// Measured, stage kernels / one-launch / resident 1 step / resident 10 steps:
+//                   2.3 + 3.7e-3 q n a step (clusters 6.3 + 3.9e-3 n; 1.35 times
+//                   the part in n with J2), and 0.8 + 3.1e-3 q n once to load and
+//                   store the lattice (1.9e-3 up to 32 columns)
+// for 148 SMs, the same work a CTA on others (LLGArgs::sms).  Measured, stage kernels / one-launch / resident 1 step / resident 10 steps:
 //   32x32x50    11.2 /  36 / 12.2 /  6.9     64x64x8     9.7 / 45 / 31.4 / 18.5
 //   32x32x200   22   /  37 / 16.3 / 10.2     64x64x100  35.8 / 45 / 35.3 / 18.6
 //   32x32x1000  70   /  67 / 51.9 / 31.5     12x12x1000 18   / 49 / 18.9 / 10.1
-//   64x64x400   115  /  98 / 103  / 55.6     128x128x500 548 / 368 / 604 / 335
+//   64x64x400   114  /  97 / 101  / 55.3     128x128x500 531 / 364 / 604 / 341
 //   51x51x70    22   /  48 / 21.3 / 13.5     90x90x60   36.5 / 60
+// and with J2, resident 1 / 4 steps a launch: 64x64x1000 298 / 268 / 278 / 189,
+//   64x64x700   214  / 190 / 197  / 134      128x128x150 193 / 170 / -   / 151
 static double stages_cost(const LLGArgs &a) {
     return 9.0 + (a.use_j2 ? 0.073e-3 : 0.065e-3) * (double)a.M * a.nc;
 }
@@ -892,8 +895,8 @@ static double stages_cost(const LLGArgs &a) {
 static double fused_cost(const LLGArgs &a) {
     const StreamGeom g = stream_geom(a);
     const long total = (long)g.nb * g.ng * a.N;
-    const double run = std::max<double>(stream::MIN_RUN, total / (2.0 * 148));
-    const double two = std::min(1.0, std::max(0.0, total / run / 148.0 - 1.0));  // SMs with two
+    const double run = std::max<double>(stream::MIN_RUN, total / (2.0 * a.sms));
+    const double two = std::min(1.0, std::max(0.0, total / run / a.sms - 1.0));  // SMs with two
     const double iter = std::max(1.45 + 0.45 * two, (1.8 + 1.3 * two) * (g.wt + 24) / 96.0);
     return (run + 9.0) * iter * (a.use_j2 ? 1.29 : 1.0);
 }
@@ -907,10 +910,11 @@ bool llg_resident_wins(const LLGArgs &a, int nsteps) {
     if (!resident_geom(a.N, g, w, smem)) return false;
     const double n = (double)g.rows * a.N;
     const bool cl = g.s > 1;
-    const double base = cl ? 6.3 : 2.3, site = (cl ? 3.9e-3 : 3.7e-3) * (a.use_j2 ? 1.27 : 1.0);
-    auto round = [&](double q) { return nsteps * (base + site * q * n) + 0.8 + 2.6e-3 * q * n; };
-    // CTAs an SM takes in all (clusters of 4 fill about 140 of the 148), and q at once
-    const double per_sm = (double)a.nc * g.s / (cl ? 140.0 : 148.0);
+    const double base = cl ? 6.3 : 2.3, site = (cl ? 3.9e-3 : 3.7e-3) * (a.use_j2 ? 1.35 : 1.0);
+    const double move = w <= 32 ? 1.9e-3 : 3.1e-3;
+    auto round = [&](double q) { return nsteps * (base + site * q * n) + 0.8 + move * q * n; };
+    // CTAs an SM takes in all (clusters of 4 fill about 140 of 148), and q at once
+    const double per_sm = (double)a.nc * g.s / (cl ? a.sms * 140.0 / 148.0 : (double)a.sms);
     const int at_once = resident::ctas_per_sm(w);
     double res = 2.8;
     if (per_sm > 3.0 * at_once) {  // rounds blur into one another
