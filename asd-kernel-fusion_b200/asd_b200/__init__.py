@@ -55,7 +55,7 @@ EXPORTED_SYMBOLS = (
     "asd_ctx_last_launches", "asd_ctx_time_kernels", "asd_ctx_kernel_time",
     "asd_ctx_check_device_status", "asd_debug_fail_alloc", "asd_ctx_debug_poison",
     "asd_check_bounded_wait", "asd_check_const_division", "asd_check_const_division_f32", "asd_umma_gemm_f32", "asd_sqt_split_noalloc",
-    "asd_measure_fp64_peak", "asd_check_dmma_layout",
+    "asd_measure_fp64_peak", "asd_check_dmma_layout", "asd_check_adjoint_ctas",
     "asd_spins_save", "asd_spins_load", "asd_batch_create", "asd_batch_destroy",
     "asd_batch_set_stream", "asd_batch_set_spins", "asd_batch_get_spins", "asd_batch_run",
     "asd_batch_configure", "asd_batch_configure_cluster", "asd_batch_autotune",
@@ -155,6 +155,7 @@ def load() -> C.CDLL:
         "asd_ctx_kernel_time": ([vp, C.c_int, dp, C.POINTER(C.c_int)], C.c_int),
         "asd_measure_fp64_peak": ([C.c_int, dp, dp, vp], C.c_int),
         "asd_check_dmma_layout": ([vp, vp, vp, vp], C.c_int),
+        "asd_check_adjoint_ctas": ([C.c_int, C.c_int, C.c_int], C.c_int),
         "asd_ctx_check_device_status": ([vp], C.c_int),
         "asd_debug_fail_alloc": ([C.c_long], C.c_int),
         "asd_ctx_debug_poison": ([vp], C.c_int),

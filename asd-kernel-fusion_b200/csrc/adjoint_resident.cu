@@ -326,7 +326,8 @@ bool geometry(const LLGArgs &a, int &S, int &rows, int &groups, int &rp) {
     for (int s = 1; s <= 4; s *= 2) {
         const int rw = (N + s - 1) / s, r = (rw + groups - 1) / groups;
         if (r > RP || smem_bytes(rw) > 227 * 1024) continue;
-        const long slots = s == 4 ? a.sms * 132L / 148 : a.sms, rounds = ((long)a.nfile * s + slots - 1) / slots;
+        const long slots = std::max(1L, s == 4 ? a.sms * 132L / 148 : (long)a.sms);
+        const long rounds = ((long)a.nfile * s + slots - 1) / slots;
         const double cost = rounds * ((s == 1 ? 6.0 : 9.5) + 0.02 * rw * N);
         if (S == 0 || cost < best) S = s, rows = rw, rp = r, best = cost;
     }

@@ -643,10 +643,10 @@ int step_into(asd_ctx *c, const double *y_in, double *s2, double *s3, double *s4
 // 2.4 times the speed of the kernel-by-kernel adjoint from 16 replicas on (figures
 // in adjoint_resident.cu).  Fewer replicas keep the latter, which spreads a
 // lattice over all SMs.
+constexpr int kResidentAdjointReplicas = 16;
 bool use_resident_adjoint(const asd_ctx *c) {
-    if (c->llg_kernel != ASD_LLG_AUTO || c->p.nfile < 16) return false;
-    const int blocks = adjoint_resident_blocks(c->a);
-    return blocks > 0;
+    return c->llg_kernel == ASD_LLG_AUTO && c->p.nfile >= kResidentAdjointReplicas &&
+           adjoint_resident_blocks(c->a) > 0;
 }
 
 // Frees the adjoint's state-sized and small buffers.
@@ -1641,6 +1641,16 @@ int asd_ctx_loss_backward(asd_ctx *c, const double *target, double *grad, double
     if (!c) return fail(ASD_ERR_INVALID, "ctx is NULL");
     ASD_CUDA_TRY(enter(c));
     return loss_backward(c, target, grad, dtarget);
+}
+
+int asd_check_adjoint_ctas(int N, int nfile, int num_sms) {
+    asd_params p;
+    if (asd_params_default(&p, N, nfile) != ASD_OK || check_params(&p) != ASD_OK || num_sms < 1 ||
+        nfile < kResidentAdjointReplicas)
+        return 0;
+    LLGArgs a = make_llg_args(p);
+    a.sms = num_sms;
+    return adjoint_resident_blocks(a) / nfile;
 }
 
 int asd_ctx_set_params(asd_ctx *c, const asd_params *p) {

@@ -202,6 +202,11 @@ int asd_ctx_loss_forward(asd_ctx *ctx, int nsteps, int stride, int checkpoint, c
                          double *loss, double *sqt_out);
 int asd_ctx_loss_backward(asd_ctx *ctx, const double *target, double *grad, double *dtarget);
 
+/* Diagnostic (host only, no GPU): the CTAs per replica (1, 2 or 4) that the default
+ * backward pass takes for a lattice of side N and nfile replicas on num_sms SMs, or 0
+ * where it runs kernel by kernel.  No counterpart in the reference; tests use it. */
+int asd_check_adjoint_ctas(int N, int nfile, int num_sms);
+
 /* One full step through host buffers, the reference's own contract: spins
  * (AoS) come from host memory, one RK4 step runs, the new spins go back to
  * spin_out and S(q,t) into sqt_out.  spin_in may equal spin_out.  Above 64
