@@ -1,5 +1,5 @@
 // adjoint_resident.cu -- the adjoint of a segment of RK4 steps in one launch, one
-// replica's lattice held on an SM or a pair of SMs (see adjoint.cu for the
+// replica's lattice held on one, two or four SMs (see adjoint.cu for the
 // formulas and llg_kernels.cu for the resident forward steps it mirrors).
 //
 // A launch takes a segment between two checkpoints: it steps forward from the
@@ -18,9 +18,10 @@
 // pointer.  Eight barriers a step instead of 9 to 13 launches that
 // each read and write whole states.
 //
-// Bound by shared-memory traffic (63 % of its wavefronts) and instruction issue
-// (47 %), with waits for L2 and for the cluster barriers' outstanding stores;
-// FP64 pipe 39 %.  Measured on B200, backward pass alone, us a step, kernel by
+// Bound by latency between shared memory, L2 and the cluster barriers (which wait
+// for outstanding stores) at 16 warps an SM: at 64x64x100, two rounds of two CTAs a
+// replica, shared memory moves 45 % of its wavefronts and the FP64 pipe is 39 % busy.
+// Measured on B200, backward pass alone, us a step, kernel by
 // kernel / resident: 64x64x100 144 / 97 (200 CTAs in two rounds), 64x64x74 112 /
 // 50, 64x64x20 59 / 30, 48x48x300 223 / 161, 32x32x200 94 / 50, 12x12x500 54 / 37.
 // With lam_v, lam_y and loc in registers and the walks unrolled, 1 KB of spills:
@@ -315,8 +316,12 @@ size_t smem_bytes(int rows) {
 }
 
 // 1, 2 or 4 CTAs per replica (a CTA an SM; clusters of 4 find room on 132 of the
-// 148 SMs), whichever is done first: a round of CTAs with n sites each took
-// about 6 + 0.02 n us a step, 9.5 + 0.02 n where a cluster has to synchronise.
+// 148 SMs), whichever is done first: a round of CTAs with n sites each took about
+// 8 + 0.019 n us a step, 13 + 0.017 n where a cluster has to synchronise.  Measured
+// with 1 / 2 / 4 (up to 33 replicas fit one round of 4, 74 one of 2):
+//   16x16x16 10.2 / 14.1 / 13.7   20x20x16 15.4 / 15.6 / 14.6   24x24x37 19.4 / 17.1 / 29.2
+//   32x32x16 24.6 / 19.2 / 16.1   32x32x80 24.8 / 37.3 / 45.9   48x48x33  -   / 32.3 / 23.4
+//   48x48x74  -   / 33.1 / 67.6   64x64x33  -   / 47.8 / 29.6   64x64x90  -   / 95.3 / 86.4
 bool geometry(const LLGArgs &a, int &S, int &rows, int &groups, int &rp) {
     const int N = a.N;
     if (N > W || N < MIN_SIDE) return false;
@@ -328,7 +333,7 @@ bool geometry(const LLGArgs &a, int &S, int &rows, int &groups, int &rp) {
         if (r > RP || smem_bytes(rw) > 227 * 1024) continue;
         const long slots = std::max(1L, s == 4 ? a.sms * 132L / 148 : (long)a.sms);
         const long rounds = ((long)a.nfile * s + slots - 1) / slots;
-        const double cost = rounds * ((s == 1 ? 6.0 : 9.5) + 0.02 * rw * N);
+        const double cost = rounds * (s == 1 ? 8.0 + 0.019 * rw * N : 13.0 + 0.017 * rw * N);
         if (S == 0 || cost < best) S = s, rows = rw, rp = r, best = cost;
     }
     return S > 0;

@@ -93,7 +93,7 @@ cudaError_t launch_llg_stage(int stage, const LLGArgs &a, const double *y, const
 cudaError_t launch_llg_step_fused(const LLGArgs &a, const double *y, double *yout,
                                   cudaStream_t st);
 // nsteps (>= 1) RK4 steps in one launch, each replica's lattice resident on one
-// SM or on a cluster of up to 8: y -> yout (may be the same buffer), replicas
+// SM or on a cluster of 2 or 4: y -> yout (may be the same buffer), replicas
 // [a.f0, a.f0 + a.nc); scratch: nc * 3 * M doubles.  llg_resident_wins:
 // the lattice side allows it and it is the fastest of the three ways to step.
 cudaError_t launch_llg_resident(const LLGArgs &a, const double *y, double *yout, double *scratch,

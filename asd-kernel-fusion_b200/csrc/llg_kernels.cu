@@ -792,13 +792,13 @@ cudaError_t launch_llg_stage(int stage, const LLGArgs &a, const double *y, const
 }
 
 // The geometry of the resident steps for lattice side N: rows of W doubles a
-// component, the fewest CTAs per replica (1, 2, 4, 8) whose threads cover the
+// component, the fewest CTAs per replica (1, 2, 4) whose threads cover the
 // rows and whose two buffers fit shared memory; false if none does.
 static bool resident_geom(int N, ResGeom &g, int &w, size_t &smem) {
     w = N <= 32 ? 32 : N <= 64 ? 64 : 128;
     if (N > w) return false;
     g.groups = resident::threads(w) / N;
-    for (g.s = 1; g.s <= 8 && g.s <= N; g.s *= 2) {
+    for (g.s = 1; g.s <= 4 && g.s <= N; g.s *= 2) {
         g.rows = (N + g.s - 1) / g.s;
         smem = (size_t)2 * 3 * (g.rows + 2) * w * sizeof(double);
         if ((g.rows + g.groups - 1) / g.groups <= resident::rows_per_thread(w) && smem <= 227 * 1024) return true;
