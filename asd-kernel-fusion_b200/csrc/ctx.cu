@@ -129,7 +129,8 @@ struct asd_ctx {
     int llg_kernel = ASD_LLG_AUTO;
     // Pipelining of asd_ctx_step behind asd_ctx_sqt_async: once a split-mode
     // S(q,t) has turned y into its GEMM operands, the GEMM reads none of the
-    // LLG buffers, so the next RK4 step may run beside it on llg_stream.
+    // LLG buffers, so the next RK4 step may run beside it on llg_stream (the stage
+    // kernels; CTAs of the other two start as the GEMM's leave their SMs).
     // y_free is recorded on the ctx stream right after the split; armed says
     // that nothing touching y, ys_a, ys_b or acc has been enqueued since.
     // The split-mode GEMM and its finalize run on gemm_stream, created with

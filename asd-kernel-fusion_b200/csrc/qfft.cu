@@ -40,7 +40,8 @@
 // Bound by shared-memory traffic (each stage reads and writes 16 bytes a point)
 // and, below about 64 x 64, by launch latency.  Measured on B200 against the FP64
 // tensor-core GEMM with diagonal sums that served this before: 256x256x1000 831
-// -> 6.61 ms, 128x128x500 26.9 -> 0.80 ms, 32x32x200 0.145 -> 0.031 ms.
+// -> 6.55 ms, 128x128x500 26.9 -> 0.82 ms, 32x32x200 0.145 -> 0.026 ms; of these
+// the scaling by magnitude 0.01, 0.015 and 0.0007 ms.
 #include "asd_internal.h"
 
 namespace asd {

@@ -149,10 +149,10 @@ __device__ __forceinline__ float two_sum(float x, float y, float &e) {
 }
 
 // The q grid's sums over blocks, K chunks and warps: three floats whose unevaluated
-// sum carries about 72 bits, more than FP64's 53.  FP64 registers in their place are
-// slow beside the tensor cores: 45 such instructions a thread and tile took 4.2 us a
-// tile (100x100x240 in FP16x3 380 -> 472 us, 128x128x500 1682 -> 1861).  Their range is
-// FP32's; grid_shift keeps the sums inside it.
+// sum carries about 72 bits, more than FP64's 53.  FP64 registers in their place cost
+// more beside this GEMM: 45 such instructions a thread and tile took 4.2 us a tile (in
+// FP16x3 472 us against 392 at 100x100x240, 1861 against 1730 at 128x128x500).  Their
+// range is FP32's; grid_shift keeps the sums inside it.
 struct Sum3 {
     float h, m, l;
     __device__ __forceinline__ void add(float x, float e) {  // x + e, |e| far below |x|

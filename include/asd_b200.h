@@ -155,8 +155,8 @@ int asd_ctx_sqt_magnitude(asd_ctx *ctx, double *out);
  * along the diagonals i - j of each tile; the diagonal sums are binned by
  * displacement r_i - r_j (mod N) and a 2-D DFT of the N*N bins gives S at every
  * q.  d_out[2*(vx*N+vy)] equals asd_ctx_sqt's value up to rounding.  Any N
- * (FP64: up to 2435); work space on the first call: a few MB in FP64, 8 * 383 * 2
- * bytes per GEMM tile of 128 x 256 in the split modes (0.8 GB at N = 256).
+ * (FP64: up to 2435); work space on the first call: a few MB in FP64 (up to about
+ * 50 at the largest N), 8 * 383 * 2 bytes per GEMM tile of 128 x 256 in the split modes (0.8 GB at N = 256).
  * Every sum runs in a fixed order, so results repeat bit for bit.
  * No counterpart in the reference (its programs evaluate one q). */
 int asd_ctx_sqt_grid_async(asd_ctx *ctx, asd_sqt_mode mode, double *d_out);
@@ -271,15 +271,16 @@ int asd_ctx_shard_sqt_finish(asd_ctx *ctx, const double *d_part, const double *d
 #define ASD_LLG_FUSED_STEP 1 /* one launch per step, the four stages
                                 streamed down the lattice through shared
                                 memory by column band (48 B of DRAM traffic per
-                                site-step; FP64-bound; 1.35x the stages at
-                                128x128x500, 1.6x at 256x256x1000 on B200)  */
+                                site-step; FP64-bound; 1.46x the stages at
+                                128x128x500, 1.48x at 256x256x1000 with J2 on
+                                B200)                                        */
 #define ASD_LLG_AUTO 2       /* default: the fastest of three for the lattice,
                                 replicas and steps of the call: the stage
                                 kernels, the one-launch step, or the resident
                                 steps (each replica's lattice held on one SM, or
                                 a cluster of SMs, for all steps of an
                                 asd_ctx_step; up to N = 128: 64x64x100
-                                43.6 -> 18.9 us a step on B200)              */
+                                43.6 -> 17.1 us a step on B200, 50 a call)   */
 int asd_ctx_set_llg_kernel(asd_ctx *ctx, int kernel);
 
 /* K elements accumulated per TMEM chunk by the split S(q,t) modes (rounded
