@@ -1506,7 +1506,8 @@ int asd_ctx_create(const asd_params *p, unsigned mode_mask, asd_ctx **out) {
     }
     // Small lattices take the phase sums' work space here (a small part of a
     // state array), so that their first FP64 S(q,t) can be captured into a graph.
-    if (dmma_sqt_tiles(c->M) <= c->num_sms && (rc = ensure_phase_work(c)) != ASD_OK) {
+    if ((c->modes & (1u << ASD_SQT_FP64)) && dmma_sqt_tiles(c->M) <= c->num_sms &&
+        (rc = ensure_phase_work(c)) != ASD_OK) {
         destroy(c);
         return rc;
     }
